@@ -31,6 +31,7 @@ SOURCES = {
     # the FP32 kernels spell out every fused multiply-add (fmaf, paired
     # __ffma2_rn), so all strategies round identically
     "fp32_path.cu": ["--fmad=false"],
+    "fp32_eqstate.cu": ["--fmad=false"],
     "ensemble.cu": [],
     "noalloc.cu": [],
 }

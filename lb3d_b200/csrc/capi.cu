@@ -615,9 +615,15 @@ int lb3dc_time_loop(lb3dc_handle *h, int nsteps) {
   int rc = need_loaded(h);
   if (rc) return rc;
   if (nsteps < 0) return fail(h, LB3DC_EINVAL, "nsteps < 0");
-  if (h->p.precision == LB3DC_FP32_DEV && !h->le) {
-    h->nt += nsteps;
-    rc = fp32_run(h->P, h->s32, h->rock, nsteps, h->stream);
+  if (h->p.precision == LB3DC_FP32_DEV && (!h->le || !h->pending_advection)) {
+    // under Lees-Edwards stage 6 of each step first moves the planes
+    std::vector<LEStep> le;
+    for (int s = 0; h->le && s < nsteps; ++s) {
+      if ((rc = lb3dc_bc_apply(h, 6))) return rc;
+      le.push_back(le_step(h));
+    }
+    if (!h->le) h->nt += nsteps;
+    rc = fp32_run(h->P, h->s32, h->rock, nsteps, h->stream, h->le ? le.data() : nullptr, true);
     if (rc) return fail(h, LB3DC_ECUDA, "FP32 run failed: %s", cudaGetErrorString(cudaGetLastError()));
     return LB3DC_OK;
   }
@@ -649,10 +655,6 @@ int lb3dc_sync(lb3dc_handle *h) {
   cudaSetDevice(h->device);
   CK(h, cudaStreamSynchronize(h->stream));
   CK(h, cudaGetLastError());
-  if (h->p.precision == LB3DC_FP32_DEV) {
-    const int rc = fp32_take_error(h->s32, h->stream);
-    if (rc) return fail(h, rc, "a bounded device-side wait of the FP32 path gave up");
-  }
   return LB3DC_OK;
 }
 

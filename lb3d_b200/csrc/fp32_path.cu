@@ -32,6 +32,8 @@
 #include <cstring>
 #include <vector>
 
+#include "fp32_device.cuh"
+#include "fp32_eqstate.h"
 #include "fp32_path.h"
 #include "reduce.h"
 #include "fp64_path.h"
@@ -39,366 +41,6 @@
 
 namespace lb3d {
 namespace f32 {
-
-constexpr float W1 = 1.0f / 36.0f;
-constexpr float W0 = 1.0f / 3.0f;
-LB3D_HDI constexpr float wq(int q) { return q == 18 ? W0 : W1; }
-
-__device__ __forceinline__ int pmod(int v, int n) {
-  int r = v % n;
-  return r < 0 ? r + n : r;
-}
-// Periodic wrap without a division when v lies within one period of the
-// lattice (-n <= v < 2n), the case of every tile and halo coordinate of a
-// lattice at least as large as the halo; pmod otherwise.
-__device__ __forceinline__ int wrapz(int v, int n) {
-  if (v >= -n && v < 2 * n) return v < 0 ? v + n : (v >= n ? v - n : v);
-  return pmod(v, n);
-}
-
-// Langevin function L(x) = coth x - 1/x, accurate in FP32 for small x.
-__device__ __forceinline__ float langevin(float x) {
-  if (x < 0.3f) {
-    float x2 = x * x;
-    return x * fmaf(x2, fmaf(x2, fmaf(x2, -1.0f / 4725.0f, 2.0f / 945.0f), -1.0f / 45.0f), 1.0f / 3.0f);
-  }
-  float t = tanhf(x);
-  return 1.0f / t - 1.0f / x;
-}
-
-// Equilibrium deviation for one component: deq_i = rho*(E_i(v) - w_i) + drho*w_i
-// with E of bdist = 2 (code/lb3d_bdist.F90:301-370), then the BGK update
-// d_i <- d_i + omega (deq_i - d_i), evaluated as (1 - omega) d_i + omega deq_i
-// with omega folded into the equilibrium's coefficients.  Every multiply-add
-// is written out (fmaf), so bgk_update2 below can repeat the same roundings
-// lane by lane.
-__device__ __forceinline__ void bgk_update(float d[19], float rho, float drho, float vx, float vy,
-                                           float vz, float omega) {
-  const float tx = 3.0f * vx, ty = 3.0f * vy, tz = 3.0f * vz;
-  const float uke = 0.5f * fmaf(tz, vz, fmaf(ty, vy, tx * vx));
-  const float a = -uke;          // even part minus w
-  const float b = 1.0f + a;      // odd linear coefficient
-  const float orw = (omega * rho) * W1;
-  const float obase = (omega * drho) * W1;
-  const float om1 = 1.0f - omega;
-#define LB3D_PAIR32(CD, I, J)                                             \
-  {                                                                       \
-    const float e = (CD);                                                 \
-    const float e2 = e * e;                                               \
-    const float ev = fmaf(orw, fmaf(0.5f, e2, a), obase);                 \
-    const float od = (orw * e) * fmaf(e2, 1.0f / 6.0f, b);                \
-    d[I] = fmaf(om1, d[I], ev + od);                                      \
-    d[J] = fmaf(om1, d[J], ev - od);                                      \
-  }
-  LB3D_PAIR32(tx, 0, 1)
-  LB3D_PAIR32(ty, 2, 3)
-  LB3D_PAIR32(tz, 4, 5)
-  LB3D_PAIR32(tx + ty, 6, 11)
-  LB3D_PAIR32(tx - ty, 7, 10)
-  LB3D_PAIR32(tx + tz, 8, 13)
-  LB3D_PAIR32(tx - tz, 9, 12)
-  LB3D_PAIR32(ty + tz, 14, 17)
-  LB3D_PAIR32(ty - tz, 15, 16)
-#undef LB3D_PAIR32
-  const float oeq0 = fmaf((omega * rho) * W0, a, (omega * drho) * W0);
-  d[18] = fmaf(om1, d[18], oeq0);
-}
-
-// Paired FP32 arithmetic (sm_100 FADD2/FMUL2/FFMA2: two lanes per
-// instruction, each rounded as its scalar counterpart).
-__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
-__device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }
-__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
-
-// bgk_update for two components at once (lane x, lane y), bit for bit the
-// scalar routine on each lane.
-__device__ __forceinline__ void bgk_update2(float2 d[19], float2 rho, float2 drho, float2 vx,
-                                            float2 vy, float2 vz, float2 omega) {
-  const float2 tx = mul2(f2(3.0f), vx), ty = mul2(f2(3.0f), vy), tz = mul2(f2(3.0f), vz);
-  const float2 uke = mul2(f2(0.5f), fma2(tz, vz, fma2(ty, vy, mul2(tx, vx))));
-  const float2 a = neg2(uke);
-  const float2 b = add2(f2(1.0f), a);
-  const float2 orw = mul2(mul2(omega, rho), f2(W1));
-  const float2 obase = mul2(mul2(omega, drho), f2(W1));
-  const float2 om1 = add2(f2(1.0f), neg2(omega));
-#define LB3D_PAIR2(CD, I, J)                                                  \
-  {                                                                           \
-    const float2 e = (CD);                                                    \
-    const float2 e2 = mul2(e, e);                                             \
-    const float2 ev = fma2(orw, fma2(f2(0.5f), e2, a), obase);                \
-    const float2 od = mul2(mul2(orw, e), fma2(e2, f2(1.0f / 6.0f), b));       \
-    d[I] = fma2(om1, d[I], add2(ev, od));                                     \
-    d[J] = fma2(om1, d[J], add2(ev, neg2(od)));                               \
-  }
-  LB3D_PAIR2(tx, 0, 1)
-  LB3D_PAIR2(ty, 2, 3)
-  LB3D_PAIR2(tz, 4, 5)
-  LB3D_PAIR2(add2(tx, ty), 6, 11)
-  LB3D_PAIR2(add2(tx, neg2(ty)), 7, 10)
-  LB3D_PAIR2(add2(tx, tz), 8, 13)
-  LB3D_PAIR2(add2(tx, neg2(tz)), 9, 12)
-  LB3D_PAIR2(add2(ty, tz), 14, 17)
-  LB3D_PAIR2(add2(ty, neg2(tz)), 15, 16)
-#undef LB3D_PAIR2
-  const float2 oeq0 = fma2(mul2(mul2(omega, rho), f2(W0)), a, mul2(mul2(omega, drho), f2(W0)));
-  d[18] = fma2(om1, d[18], oeq0);
-}
-
-// Equilibrium deviations of one component written straight to the output
-// (full relaxation: the BGK update with omega = 1), with bgk_update's
-// arithmetic; out[q * S] receives population q.
-__device__ __forceinline__ void eq_store(float *out, unsigned S, float rho, float drho, float vx, float vy,
-                                         float vz, float omega) {
-  const float tx = 3.0f * vx, ty = 3.0f * vy, tz = 3.0f * vz;
-  const float uke = 0.5f * fmaf(tz, vz, fmaf(ty, vy, tx * vx));
-  const float a = -uke;
-  const float b = 1.0f + a;
-  const float orw = (omega * rho) * W1;
-  const float obase = (omega * drho) * W1;
-#define LB3D_EQ32(CD, I, J)                                               \
-  {                                                                       \
-    const float e = (CD);                                                 \
-    const float e2 = e * e;                                               \
-    const float ev = fmaf(orw, fmaf(0.5f, e2, a), obase);                 \
-    const float od = (orw * e) * fmaf(e2, 1.0f / 6.0f, b);                \
-    __stcs(out + (I) * S, ev + od);                                       \
-    __stcs(out + (J) * S, ev - od);                                       \
-  }
-  LB3D_EQ32(tx, 0, 1)
-  LB3D_EQ32(ty, 2, 3)
-  LB3D_EQ32(tz, 4, 5)
-  LB3D_EQ32(tx + ty, 6, 11)
-  LB3D_EQ32(tx - ty, 7, 10)
-  LB3D_EQ32(tx + tz, 8, 13)
-  LB3D_EQ32(tx - tz, 9, 12)
-  LB3D_EQ32(ty + tz, 14, 17)
-  LB3D_EQ32(ty - tz, 15, 16)
-#undef LB3D_EQ32
-  __stcs(out + 18 * S, fmaf((omega * rho) * W0, a, (omega * drho) * W0));
-}
-// eq_store for two components (lanes x, y) with bgk_update2's paired
-// arithmetic; lane x goes to outA, lane y to outB.
-// With bA (optional) the two components' values also go to bA[q * SB] and
-// bB[q * SB].
-__device__ __forceinline__ void eq_store2(float *outA, float *outB, unsigned S, float2 rho, float2 drho,
-                                          float2 vx, float2 vy, float2 vz, float2 omega,
-                                          float *bA = nullptr, float *bB = nullptr, unsigned SB = 0) {
-  const float2 tx = mul2(f2(3.0f), vx), ty = mul2(f2(3.0f), vy), tz = mul2(f2(3.0f), vz);
-  const float2 uke = mul2(f2(0.5f), fma2(tz, vz, fma2(ty, vy, mul2(tx, vx))));
-  const float2 a = neg2(uke);
-  const float2 b = add2(f2(1.0f), a);
-  const float2 orw = mul2(mul2(omega, rho), f2(W1));
-  const float2 obase = mul2(mul2(omega, drho), f2(W1));
-#define LB3D_EQ2(CD, I, J)                                                    \
-  {                                                                           \
-    const float2 e = (CD);                                                    \
-    const float2 e2 = mul2(e, e);                                             \
-    const float2 ev = fma2(orw, fma2(f2(0.5f), e2, a), obase);                \
-    const float2 od = mul2(mul2(orw, e), fma2(e2, f2(1.0f / 6.0f), b));       \
-    const float2 p = add2(ev, od), m = add2(ev, neg2(od));                    \
-    __stcs(outA + (I) * S, p.x);                                              \
-    __stcs(outB + (I) * S, p.y);                                              \
-    __stcs(outA + (J) * S, m.x);                                              \
-    __stcs(outB + (J) * S, m.y);                                              \
-    if (bA) {                                                                 \
-      bA[(I) * SB] = p.x;                                                     \
-      bB[(I) * SB] = p.y;                                                     \
-      bA[(J) * SB] = m.x;                                                     \
-      bB[(J) * SB] = m.y;                                                     \
-    }                                                                         \
-  }
-  LB3D_EQ2(tx, 0, 1)
-  LB3D_EQ2(ty, 2, 3)
-  LB3D_EQ2(tz, 4, 5)
-  LB3D_EQ2(add2(tx, ty), 6, 11)
-  LB3D_EQ2(add2(tx, neg2(ty)), 7, 10)
-  LB3D_EQ2(add2(tx, tz), 8, 13)
-  LB3D_EQ2(add2(tx, neg2(tz)), 9, 12)
-  LB3D_EQ2(add2(ty, tz), 14, 17)
-  LB3D_EQ2(add2(ty, neg2(tz)), 15, 16)
-#undef LB3D_EQ2
-  const float2 oeq0 = fma2(mul2(mul2(omega, rho), f2(W0)), a, mul2(mul2(omega, drho), f2(W0)));
-  __stcs(outA + 18 * S, oeq0.x);
-  __stcs(outB + 18 * S, oeq0.y);
-  if (bA) {
-    bA[18 * SB] = oeq0.x;
-    bB[18 * SB] = oeq0.y;
-  }
-}
-
-// Own-site moments of one component's post-stream deviations d[q * ST]:
-// drho = sum_q g_q d_q and j = sum_q g_q c_q d_q, in q order, one fused
-// multiply-add per term.
-template <int ST>
-__device__ __forceinline__ void own_moments(const float *d, float &dr, float &j0, float &j1,
-                                            float &j2) {
-  float r = 0.f, a0 = 0.f, a1 = 0.f, a2 = 0.f;
-#pragma unroll
-  for (int q = 0; q < 19; ++q) {
-    const float v = d[q * ST], g = (float)gw(q);
-    r = fmaf(g, v, r);
-    if (cx(q)) a0 = fmaf(g * (float)cx(q), v, a0);
-    if (cy(q)) a1 = fmaf(g * (float)cy(q), v, a1);
-    if (cz(q)) a2 = fmaf(g * (float)cz(q), v, a2);
-  }
-  dr = r;
-  j0 = a0;
-  j1 = a1;
-  j2 = a2;
-}
-// own_moments2 of values already in registers (lane x, lane y).
-__device__ __forceinline__ void own_moments2_reg(const float2 v[19], float2 &dr, float2 &j0,
-                                                 float2 &j1, float2 &j2) {
-  float2 r = f2(0.f), a0 = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
-#pragma unroll
-  for (int q = 0; q < 19; ++q) {
-    const float g = (float)gw(q);
-    r = fma2(f2(g), v[q], r);
-    if (cx(q)) a0 = fma2(f2(g * (float)cx(q)), v[q], a0);
-    if (cy(q)) a1 = fma2(f2(g * (float)cy(q)), v[q], a1);
-    if (cz(q)) a2 = fma2(f2(g * (float)cz(q)), v[q], a2);
-  }
-  dr = r;
-  j0 = a0;
-  j1 = a1;
-  j2 = a2;
-}
-// own_moments of two components (lanes x, y) with paired instructions.
-template <int ST>
-__device__ __forceinline__ void own_moments2(const float *dA, const float *dB, float2 &dr,
-                                             float2 &j0, float2 &j1, float2 &j2) {
-  float2 r = f2(0.f), a0 = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
-#pragma unroll
-  for (int q = 0; q < 19; ++q) {
-    const float2 v = make_float2(dA[q * ST], dB[q * ST]);
-    const float g = (float)gw(q);
-    r = fma2(f2(g), v, r);
-    if (cx(q)) a0 = fma2(f2(g * (float)cx(q)), v, a0);
-    if (cy(q)) a1 = fma2(f2(g * (float)cy(q)), v, a1);
-    if (cz(q)) a2 = fma2(f2(g * (float)cz(q)), v, a2);
-  }
-  dr = r;
-  j0 = a0;
-  j1 = a1;
-  j2 = a2;
-}
-
-// Site offsets (32-bit, relative to the lattice base) of the -1, 0, +1
-// neighbours along each axis, with the periodic wrap applied once.
-struct Nbr {
-  int cx[3], ry[3], rz[3];
-};
-
-__device__ __forceinline__ void make_nbr(Nbr &n, int gx, int gy, int gz, int nx, int ny, int nz) {
-  const int pl = nx * ny;
-  n.cx[0] = gx == 0 ? nx - 1 : gx - 1;
-  n.cx[1] = gx;
-  n.cx[2] = gx == nx - 1 ? 0 : gx + 1;
-  n.ry[0] = (gy == 0 ? ny - 1 : gy - 1) * nx;
-  n.ry[1] = gy * nx;
-  n.ry[2] = (gy == ny - 1 ? 0 : gy + 1) * nx;
-  n.rz[0] = (gz == 0 ? nz - 1 : gz - 1) * pl;
-  n.rz[1] = gz * pl;
-  n.rz[2] = (gz == nz - 1 ? 0 : gz + 1) * pl;
-}
-// site offset of x + s*c_q (s = +1 neighbour, s = -1 upstream)
-template <int Q, int SGN>
-__device__ __forceinline__ int noff(const Nbr &n) {
-  return n.cx[1 + SGN * cx(Q)] + n.ry[1 + SGN * cy(Q)] + n.rz[1 + SGN * cz(Q)];
-}
-
-// Pulls the post-stream deviations of component C of one site (with
-// half-way bounce-back when ROCK): d[q] = delta*(x - c_q, q), or
-// delta*(x, bounce(q)) when x - c_q is rock (code/lb3d_bc_bounce.F90:53-90
-// with code/lb3d_advection.F90:109-151).  F points at component 0 of the
-// lattice; the component stride is 19*S.
-// LAST selects the last-use load hint (the final read of these values by
-// this CTA), which lets L2 drop the lines early.  NARROW forms the component
-// offset c*19*S in 32 bits (lattices with 19*nc*S < 2^32), which keeps the
-// register-capped moments pass free of 64-bit products.
-template <bool ROCK, bool LAST = false, bool NARROW = false>
-__device__ __forceinline__ void pull_comp(const float *__restrict__ F, unsigned S, int c, const Nbr &n,
-                                          int self, const uint8_t *__restrict__ rk, float d[19]) {
-  const float *fc = NARROW ? F + (unsigned)(c * 19) * S : F + (size_t)(c * 19) * S;
-  d[18] = LAST ? __ldlu(fc + 18 * S + self) : __ldg(fc + 18 * S + self);
-#define LB3D_PULL(Q)                                                     \
-  {                                                                      \
-    const int up = noff<Q, -1>(n);                                       \
-    bool uf = true;                                                      \
-    if (ROCK) uf = __ldg(rk + up) == 0;                                  \
-    const float *a_ = fc + (uf ? Q * S + up : bounce(Q) * S + self);     \
-    d[Q] = LAST ? __ldlu(a_) : __ldg(a_);                                \
-  }
-  LB3D_PULL(0) LB3D_PULL(1) LB3D_PULL(2) LB3D_PULL(3) LB3D_PULL(4) LB3D_PULL(5)
-  LB3D_PULL(6) LB3D_PULL(7) LB3D_PULL(8) LB3D_PULL(9) LB3D_PULL(10) LB3D_PULL(11)
-  LB3D_PULL(12) LB3D_PULL(13) LB3D_PULL(14) LB3D_PULL(15) LB3D_PULL(16) LB3D_PULL(17)
-#undef LB3D_PULL
-}
-
-// Lees-Edwards pulls (binary, no rock; code/lb3d_bc_leesedwards.F90:147-1315
-// feeding code/lb3d_advection.F90:109-151): across x = 0 (c_x = +1) and
-// x = nx - 1 (c_x = -1) the upstream site lies in the sheared halo planes
-// Lg.le_h[0] / Lg.le_h[1], [nc][19][nz][ny], at the wrapped (y - c_y, z - c_z).
-struct LeYZ {
-  int y[3], z[3];  // wrap(gy + k - 1) and ny * wrap(gz + k - 1)
-};
-__device__ __forceinline__ void make_leyz(LeYZ &w, int gy, int gz, int ny, int nz) {
-  w.y[0] = gy == 0 ? ny - 1 : gy - 1;
-  w.y[1] = gy;
-  w.y[2] = gy == ny - 1 ? 0 : gy + 1;
-  w.z[0] = ny * (gz == 0 ? nz - 1 : gz - 1);
-  w.z[1] = ny * gz;
-  w.z[2] = ny * (gz == nz - 1 ? 0 : gz + 1);
-}
-// With ROCK (walls) the sheared halo sites are never rock, as the
-// reference's exchange leaves them (code/lb3d_bc_leesedwards.F90:678,866),
-// and a pull from a rock site inside the lattice bounces back.
-template <int Q, bool ROCK = false>
-__device__ __forceinline__ const float *le_src(const float *fc, unsigned S, int c, const Nbr &n, int gx,
-                                               int nx, const LeYZ &w, const LatDesc &Lg, int NP,
-                                               int self = 0, const uint8_t *__restrict__ rk = nullptr) {
-  if (cx(Q) == 1 && gx == 0) return Lg.le_h[0] + (c * 19 + Q) * NP + w.y[1 - cy(Q)] + w.z[1 - cz(Q)];
-  if (cx(Q) == -1 && gx == nx - 1)
-    return Lg.le_h[1] + (c * 19 + Q) * NP + w.y[1 - cy(Q)] + w.z[1 - cz(Q)];
-  const int up = noff<Q, -1>(n);
-  if (ROCK && __ldg(rk + up) != 0) return fc + bounce(Q) * S + self;
-  return fc + Q * S + up;
-}
-template <bool NARROW = false, bool ROCK = false>
-__device__ __forceinline__ void pull_comp_le(const float *__restrict__ F, unsigned S, int c, const Nbr &n,
-                                             int self, int gx, int nx, const LeYZ &w,
-                                             const LatDesc &Lg, int NP, float d[19],
-                                             const uint8_t *__restrict__ rk = nullptr) {
-  const float *fc = NARROW ? F + (unsigned)(c * 19) * S : F + (size_t)(c * 19) * S;
-  d[18] = __ldg(fc + 18 * S + self);
-#define LB3D_PULL_LE(Q) d[Q] = __ldg(le_src<Q, ROCK>(fc, S, c, n, gx, nx, w, Lg, NP, self, rk));
-  LB3D_PULL_LE(0) LB3D_PULL_LE(1) LB3D_PULL_LE(2) LB3D_PULL_LE(3) LB3D_PULL_LE(4) LB3D_PULL_LE(5)
-  LB3D_PULL_LE(6) LB3D_PULL_LE(7) LB3D_PULL_LE(8) LB3D_PULL_LE(9) LB3D_PULL_LE(10) LB3D_PULL_LE(11)
-  LB3D_PULL_LE(12) LB3D_PULL_LE(13) LB3D_PULL_LE(14) LB3D_PULL_LE(15) LB3D_PULL_LE(16) LB3D_PULL_LE(17)
-#undef LB3D_PULL_LE
-}
-
-// Writes one component's 19 deviations of a site on the x boundary of a
-// Lees-Edwards lattice to the compact boundary planes: set 0 (pre-stream,
-// le_b[0] at x = nx - 1, le_b[1] at x = 0) or set 2 (post-stream, le_b[2],
-// le_b[3]); sites elsewhere write nothing.
-__device__ __forceinline__ void le_store_boundary(const LatDesc &Lg, int set, int c, int gx, int gy,
-                                                  int gz, const float d[19]) {
-  const int nx = Lg.nx, NP = Lg.ny * Lg.nz;
-  const int o = (c * 19) * NP + gy + Lg.ny * gz;
-  if (gx == nx - 1) {
-    float *b = Lg.le_b[set] + o;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) b[q * NP] = d[q];
-  }
-  if (gx == 0) {
-    float *b = Lg.le_b[set + 1] + o;
-#pragma unroll
-    for (int q = 0; q < 19; ++q) b[q * NP] = d[q];
-  }
-}
 
 // ---------------------------------------------------------------------------
 // The fused kernel.  Grid: persistent CTAs over a tile list.  Populations
@@ -413,7 +55,6 @@ __device__ __forceinline__ void le_store_boundary(const LatDesc &Lg, int set, in
 //   B  ternary: new dipoles {d_x, d_y, d_z, -} on the tile + 1 halo, 3 planes
 //   D  ternary: previous dipoles on the tile + 3 halo, 3 planes
 // ---------------------------------------------------------------------------
-#include "fp32_stencil.cuh"
 #include "inflow.cuh"
 
 // Stage-8 inflow boundaries of one site on the FP32 path
@@ -783,7 +424,6 @@ __global__ void __launch_bounds__(TX *TY, (MODE == MODE_MOMENTS ? 1024 / (TX * T
 }
 
 #include "fp32_split.cuh"
-#include "fp32_mfield.cuh"
 
 __global__ void k_flip(LatDesc *lats, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -995,7 +635,7 @@ int fp32_fused_ctas_per_sm(int nc, bool rock, bool body, const FusedShape &sh) {
 // count), from the pass's own occupancy, so a pass with a large shared
 // memory stage does not throttle the others.  The dynamic shared memory
 // attribute and the occupancy are set up once per kernel and device.
-static cudaError_t prepare_kernel(const void *fn, int nthreads, size_t smem, int *ctas_total) {
+cudaError_t fp32_prepare_kernel(const void *fn, int nthreads, size_t smem, int *ctas_total) {
   static std::mutex mu;
   static std::map<std::tuple<const void *, size_t, int, int>, int> cache;
   int dev = 0;
@@ -1029,7 +669,7 @@ static cudaError_t launch_mode(int mode, int nc, bool rock, bool body, const Fus
   if (!fn) return cudaErrorInvalidConfiguration;
   size_t smem = fp32_mode_smem(nc, sh, mode);
   int resident = 0;
-  cudaError_t e = prepare_kernel(fn, sh.tx * sh.ty, smem, &resident);
+  cudaError_t e = fp32_prepare_kernel(fn, sh.tx * sh.ty, smem, &resident);
   if (e != cudaSuccess) return e;
   int grid = std::max(1, std::min(ntiles, resident));
   if (max_grid > 0) grid = std::min(grid, max_grid);
@@ -1172,221 +812,99 @@ long long fp32_footprint(const lb3dc_params &p) {
   const long long N = (long long)p.nx * p.ny * p.nz;
   const bool le = p.boundary_cond != 0 && (p.inv_fluid == 5 || p.inv_fluid == 6);
   const long long np = (long long)p.ny * p.nz;
-  // the moment field of strategy 3 when every component relaxes fully
+  // the fields of strategy 3 when every component relaxes fully (with the
+  // neighbour mask of a binary lattice with rock)
   const bool full = p.tau_r == 1.0 && p.tau_b == 1.0 && (p.ncomp == 2 || p.tau_s == 1.0);
-  const long long mf = full ? (long long)(p.nx + 2 * MF_PAD) * (p.ny + 2 * MF_PAD) * p.nz *
-                                             (p.ncomp == 3 ? 48 : 16) + N * 12
-                                   : 0;
+  const long long mf = full ? N * (p.ncomp == 3 ? 44 : 24) : 0;
   return 2LL * p.ncomp * 19 * N * 4 + (p.ncomp == 3 ? 6LL * N * 4 : 0) +
          N * fp32_moment_bytes(p.ncomp) + mf +
          (le ? 2 * np * (p.ncomp * 19 * 4 + 8) + 4 * np * p.ncomp * 19 * 4 : 0) + N * 16 + 4096;
 }
 
 // ---------------------------------------------------------------------------
-// moment-field strategy (split 3): eligibility, field, tensor maps, launches
+// strategy 3: eligibility, fields, tile lists, steps
 // ---------------------------------------------------------------------------
-bool fp32_mf_eligible(const DevParams &P) {
+bool fp32_eq_eligible(const DevParams &P) {
   if ((P.le && P.nc != 2) || P.invk) return false;
   for (int c = 0; c < P.nc; ++c)
     if (P.omega[c] != 1.0) return false;
-  if (P.nx < 2 || P.ny < 2) return false;
-  return (long long)(P.nx + 2 * MF_PAD) * (P.ny + 2 * MF_PAD) * P.nz < (1LL << 31);
+  return P.nx >= 2 && P.ny >= 2;
 }
 
-long long fp32_mf_bytes(const DevParams &P) {
-  return (long long)(P.nx + 2 * MF_PAD) * (P.ny + 2 * MF_PAD) * P.nz * (P.nc == 3 ? 48 : 16) +
-         P.nsites * (P.nc == 3 ? 12 : 8) + 64;
-}
-
-static int ensure_mf(const DevParams &P, Fp32State &s, cudaStream_t st) {
-  if (s.MF1) return LB3DC_OK;
-  const size_t plane = (size_t)(P.nx + 2 * MF_PAD) * (P.ny + 2 * MF_PAD) * P.nz * sizeof(float4);
-  bool ok = cudaMalloc(&s.MF1, plane) == cudaSuccess;
-  if (ok && P.nc == 3) ok = cudaMalloc(&s.MF2, plane) == cudaSuccess;
-  if (ok && P.nc == 3) ok = cudaMalloc(&s.DD, plane) == cudaSuccess;
-  if (ok) ok = cudaMalloc(&s.MFp, (size_t)P.nsites * sizeof(float2)) == cudaSuccess;
-  if (ok && P.nc == 3) ok = cudaMalloc(&s.DS, (size_t)P.nsites * sizeof(float)) == cudaSuccess;
-  if (ok && !s.err) ok = cudaMalloc(&s.err, sizeof(int)) == cudaSuccess;
-  if (!ok) {
-    cudaGetLastError();
-    if (s.MF1) cudaFree(s.MF1);
-    if (s.MF2) cudaFree(s.MF2);
-    if (s.DD) cudaFree(s.DD);
-    if (s.MFp) cudaFree(s.MFp);
-    if (s.DS) cudaFree(s.DS);
-    s.MF1 = s.MF2 = s.DD = nullptr;
-    s.MFp = nullptr;
-    s.DS = nullptr;
-    return LB3DC_ENOMEM;
+// The fields of strategy 3, allocated the first time a lattice is switched to
+// it, and (with rock) the neighbour mask and the rock sites' psi entries.
+static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
+  const size_t N = (size_t)P.nsites;
+  if (!s.o1) {
+    bool ok = cudaMalloc(&s.o1, N * sizeof(float4)) == cudaSuccess;
+    if (ok) ok = cudaMalloc(&s.o2, N * sizeof(float)) == cudaSuccess;
+    if (ok && P.nc == 3)
+      ok = cudaMalloc(&s.o3, N * sizeof(float4)) == cudaSuccess && cudaMalloc(&s.psi, N * sizeof(float2)) == cudaSuccess;
+    if (!ok) {
+      cudaGetLastError();
+      if (s.o1) cudaFree(s.o1);
+      if (s.o2) cudaFree(s.o2);
+      if (s.o3) cudaFree(s.o3);
+      if (s.psi) cudaFree(s.psi);
+      s.o1 = s.o3 = nullptr;
+      s.o2 = nullptr;
+      s.psi = nullptr;
+      return LB3DC_ENOMEM;
+    }
+    s.bytes += (long long)N * (P.nc == 3 ? 44 : 20);
   }
-  // padding entries that no site writes are read only by inactive lanes
-  cudaMemsetAsync(s.MF1, 0, plane, st);
-  if (s.MF2) cudaMemsetAsync(s.MF2, 0, plane, st);
-  if (s.DD) cudaMemsetAsync(s.DD, 0, plane, st);
-  cudaMemsetAsync(s.err, 0, sizeof(int), st);
-  s.bytes += (long long)plane * (P.nc == 3 ? 3 : 1) + P.nsites * (P.nc == 3 ? 12 : 8);
+  if (s.lat.flags & LAT_ROCK) {
+    if (!s.mask) {
+      if (cudaMalloc(&s.mask, N * sizeof(uint32_t)) != cudaSuccess) {
+        s.mask = nullptr;
+        cudaGetLastError();
+        return LB3DC_ENOMEM;
+      }
+      s.bytes += (long long)N * 4;
+    }
+    if (eq_build_mask(P.nx, P.ny, P.nz, P.le != 0, s.rock, s.mask, reinterpret_cast<float2 *>(s.M), s.lat.psi0,
+                      st) != cudaSuccess)
+      return LB3DC_ECUDA;
+  }
   return LB3DC_OK;
 }
 
-// cuTensorMapEncodeTiled through the runtime's driver entry point (no link
-// against libcuda).
-typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *,
-                                  const cuuint64_t *, const cuuint64_t *, const cuuint32_t *,
-                                  const cuuint32_t *, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_tiled() {
-  static EncodeTiledFn fn = nullptr;
-  static std::once_flag once;
-  std::call_once(once, [] {
-    void *p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  });
-  return fn;
+static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool first, int tx, int ty, EqKernel *k) {
+  const bool rock = (s.lat.flags & LAT_ROCK) != 0;
+  int ax = tx, ay = ty;
+  if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.ny, &ax, &ay);
+  return eq_kernel(pass, first, P.nc, rock, s.le_h[0] != nullptr, ax, ay, 19ull * P.nc * s.S < (1ull << 32), k);
 }
 
-// A padded float4 field as a 4-D FP32 tensor {component 0..3, padded x,
-// padded y, z}; one box is the tile plus one halo site in x and y, one plane
-// deep.
-static int encode_mf_map(CUtensorMap *m, float4 *base, const DevParams &P, int tx, int ty) {
-  EncodeTiledFn fn = encode_tiled();
-  if (!fn) return LB3DC_ECUDA;
-  const cuuint64_t XP = (cuuint64_t)P.nx + 2 * MF_PAD, YP = (cuuint64_t)P.ny + 2 * MF_PAD;
-  const cuuint64_t dims[4] = {4, XP, YP, (cuuint64_t)P.nz};
-  const cuuint64_t strides[3] = {16, 16 * XP, 16 * XP * YP};
-  const cuuint32_t box[4] = {4, (cuuint32_t)(tx + 2), (cuuint32_t)(ty + 2), 1};
-  const cuuint32_t es[4] = {1, 1, 1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-                        CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS ? LB3DC_OK : LB3DC_ECUDA;
-}
-
-template <int NC, int TX, int TY, bool ROCK, bool BODY, bool LE>
-static void mf_ptrs(bool narrow, const void **mom, const void **dip, const void **col) {
-  *mom = narrow ? (const void *)k_mf_moments<NC, TX, TY, ROCK, true, LE>
-                : (const void *)k_mf_moments<NC, TX, TY, ROCK, false, LE>;
-  *dip = NC == 3 ? (const void *)k_mf_dipole<TX, TY> : nullptr;
-  *col = (const void *)k_mf_collide<NC, TX, TY, ROCK, BODY, LE>;
-}
-// The kernels of strategy 3 for a lattice kind and tile shape (false if the
-// shape is not compiled); dip is null for binary lattices.  The
-// Lees-Edwards variants exist for binary lattices without walls.
-static bool mf_fns(int nc, bool rock, bool body, int tx, int ty, bool narrow, const void **mom,
-                   const void **dip, const void **col, bool le = false) {
-#define LB3D_MF(NC, R, B, L)                                                                   \
-  if (tx == 32 && ty == 8) return mf_ptrs<NC, 32, 8, R, B, L>(narrow, mom, dip, col), true;   \
-  if (tx == 32 && ty == 4) return mf_ptrs<NC, 32, 4, R, B, L>(narrow, mom, dip, col), true;   \
-  if (tx == 16 && ty == 16) return mf_ptrs<NC, 16, 16, R, B, L>(narrow, mom, dip, col), true; \
-  if (tx == 16 && ty == 8) return mf_ptrs<NC, 16, 8, R, B, L>(narrow, mom, dip, col), true;   \
-  if (tx == 64 && ty == 4) return mf_ptrs<NC, 64, 4, R, B, L>(narrow, mom, dip, col), true;
-  if (le) {
-    if (nc != 2) return false;
-    if (rock) {
-      if (body) { LB3D_MF(2, true, true, true) } else { LB3D_MF(2, true, false, true) }
-    } else {
-      if (body) { LB3D_MF(2, false, true, true) } else { LB3D_MF(2, false, false, true) }
-    }
-    return false;
-  }
-  if (nc == 3) {
-    if (rock) return false;
-    if (body) { LB3D_MF(3, false, true, false) } else { LB3D_MF(3, false, false, false) }
-  } else if (rock) {
-    if (body) { LB3D_MF(2, true, true, false) } else { LB3D_MF(2, true, false, false) }
-  } else {
-    if (body) { LB3D_MF(2, false, true, false) } else { LB3D_MF(2, false, false, false) }
-  }
-#undef LB3D_MF
-  return false;
-}
-// Dynamic shared memory of pass `which` (0 moments, 1 dipole, 2 collide);
-// mirrors MfGeom.
-static size_t mf_smem(int nc, int tx, int ty, int which) {
-  const size_t an = (size_t)(tx + 2) * (ty + 2), field = (16 * an + 127) / 128 * 128;
-  if (which == 0) return nc == 3 ? 4 * an * 16 : 0;
-  if (which == 1) return 8 * ((field + 1023) / 1024 * 1024) + 1024;
-  const size_t slot = ((nc == 3 ? 2 : 1) * field + 1023) / 1024 * 1024;
-  return 8 * slot + 4 * an * 8 + 1024;
-}
-
-// One step of strategy 3: the moments pass, (ternary) the dipole pass and the
-// collide pass, each on its own tile list and resident grid; with le (a
+// One step of strategy 3: the moments pass (ternary: two of them after the
+// first step of a loop), the dipole pass (ternary) and the collide pass, each on its own tile list and resident grid; with le (a
 // binary Lees-Edwards lattice) the stage-6 halo kernel runs before the
-// moments pass and the stage-8 one before the collide pass.
-// One pass of strategy 3, launched with programmatic stream serialization
-// (pdl): its CTAs may start while the previous kernel on the stream
-// finishes, and wait for it before reading its results (pdl_wait_previous).
-// Lattices with rock launch plainly (the overlap measured 0.8 % slower on
-// the porous lattice, 0.9-1 % faster on the periodic and sheared ones).
-static cudaError_t launch_pdl(const void *fn, dim3 grid, dim3 block, void **args, size_t smem,
-                              cudaStream_t st, bool pdl) {
-  if (!pdl) return cudaLaunchKernel(fn, grid, block, args, smem, st);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelExC(&cfg, fn, args);
-}
-
-static cudaError_t launch_mf(const DevParams &P, Fp32State &s, const uint8_t *rockp, cudaStream_t st,
-                             const LEStep *le) {
-  const bool rock = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
-  const unsigned S = (unsigned)s.S;
-  const bool narrow = 19ull * P.nc * s.S < (1ull << 32);
-  const void *fn[3] = {nullptr, nullptr, nullptr};
-  if (!mf_fns(P.nc, rock, body, s.tx, s.ty, narrow, &fn[0], &fn[1], &fn[2], le != nullptr))
-    return cudaErrorInvalidConfiguration;
+// moments pass and the stage-8 one before the collide pass.  Lattices with
+// rock launch plainly: the overlap of programmatic dependent launch measured
+// 0.8 % slower on the porous lattice, 0.9-1 % faster on the others.
+static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rockp, bool first, bool last,
+                           const LEStep *le, cudaStream_t st) {
   if (le && !s.le_h[0]) return cudaErrorInvalidValue;
+  const bool rock = (s.lat.flags & LAT_ROCK) != 0;
   const unsigned leg = (unsigned)((2 * P.ny * P.nz + 63) / 64);  // two threads per (y, z)
-  if (s.mf_tx != s.tx || s.mf_ty != s.ty || !s.mf_tiles) return cudaErrorInvalidConfiguration;
-  const int nt = s.tx * s.ty;
-  const LatDesc *dl = s.d_lat;
-  cudaError_t e = cudaSuccess;
-  for (int pass = 0; pass < 3 && e == cudaSuccess; ++pass) {
-    if (!fn[pass]) continue;
-    if (le && pass == 0) {
-      k_le_pre32<2><<<leg, 64, 0, st>>>(P, *le, dl, s.f[0], s.f[1], S);
-      if ((e = cudaGetLastError()) != cudaSuccess) break;
-    }
-    if (le && pass == 2) {
-      k_le_post32<2><<<leg, 64, 0, st>>>(P, *le, dl, s.f[0], s.f[1], S);
-      if ((e = cudaGetLastError()) != cudaSuccess) break;
-    }
-    const size_t sm = mf_smem(P.nc, s.tx, s.ty, pass);
-    int res = 0;
-    if ((e = prepare_kernel(fn[pass], nt, sm, &res)) != cudaSuccess) break;
-    const Tile *dt = s.mf_tiles + s.mf_off[pass];
-    int ntl = s.mf_ntiles[pass];
-    const dim3 grid(std::max(1, std::min(ntl, res)));
-    if (pass == 0) {
-      const float *f0 = s.f[0], *f1 = s.f[1], *d0 = s.db[0], *d1 = s.db[1];
-      void *args[] = {(void *)&dl, (void *)&dt, (void *)&ntl, (void *)&f0, (void *)&f1, (void *)&d0,
-                      (void *)&d1, (void *)&rockp, (void *)&S, (void *)&s.MF1, (void *)&s.MF2,
-                      (void *)&s.MFp, (void *)&s.DS};
-      e = launch_pdl(fn[pass], grid, dim3(nt), args, sm, st, !rock);
-    } else if (pass == 1) {
-      const float *ds = s.DS;
-      void *args[] = {(void *)&s.tm2, (void *)&dl, (void *)&dt, (void *)&ntl, (void *)&s.db[0],
-                      (void *)&s.db[1], (void *)&ds, (void *)&s.DD, (void *)&s.err};
-      e = launch_pdl(fn[pass], grid, dim3(nt), args, sm, st, !rock);
-    } else {
-      const float2 *mfp = s.MFp;
-      void *args[] = {(void *)&s.tm1, (void *)&s.tmd, (void *)&dl, (void *)&dt, (void *)&ntl,
-                      (void *)&s.f[0], (void *)&s.f[1], (void *)&s.db[0], (void *)&s.db[1], (void *)&rockp,
-                      (void *)&S, (void *)&mfp, (void *)&s.err};
-      e = launch_pdl(fn[pass], grid, dim3(nt), args, sm, st, !rock);
-    }
+  EqArgs a{};
+  a.lats = s.d_lat;
+  a.f0 = s.f[0], a.f1 = s.f[1], a.db0 = s.db[0], a.db1 = s.db[1];
+  a.rock = rockp;
+  a.mask = s.mask;
+  a.X = EqFields{s.M, P.nc == 3 ? s.psi : reinterpret_cast<float2 *>(s.M), s.o1, s.o3, s.o2, (unsigned)s.S};
+  for (int pass = 0; pass < EQ_PASSES; ++pass) {
+    EqKernel k;
+    if (!eq_kernel_of(P, s, pass, first, s.tx, s.ty, &k)) continue;
+    if (le && pass == EQ_MOMENTS) k_le_pre32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+    if (le && pass == EQ_COLLIDE) k_le_post32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    a.tiles = s.eq_tiles + s.eq_off[pass];
+    a.ntiles = s.eq_ntiles[pass];
+    if ((e = eq_launch(k, pass, first, last, a, !rock, st)) != cudaSuccess) return e;
   }
-  return e;
+  return cudaSuccess;
 }
 
 // The z chunking of one pass of strategy 3: nxy column tiles, `resident`
@@ -1395,7 +913,7 @@ static cudaError_t launch_mf(const DevParams &P, Fp32State &s, const uint8_t *ro
 // resident grid (1 to 8 rounds), weighed against the halo planes that
 // shorter chunks reload; the chunks of a column differ in length by at most
 // one plane.
-static int mf_chunks(int nz, int nxy, int resident, int halo) {
+int fp32_z_chunks(int nz, int nxy, int resident, int halo) {
   int best = 1;
   double best_score = -1.0;
   for (int rounds = 1; rounds <= 8; ++rounds) {
@@ -1409,30 +927,27 @@ static int mf_chunks(int nz, int nxy, int resident, int halo) {
   return best;
 }
 
-static int mf_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st) {
-  const void *fn[3];
-  if (!mf_fns(P.nc, (s.lat.flags & LAT_ROCK) != 0, (s.lat.flags & LAT_BODY) != 0, sh.tx, sh.ty,
-              19ull * P.nc * s.S < (1ull << 32), &fn[0], &fn[1], &fn[2], s.le_h[0] != nullptr))
-    return LB3DC_EINVAL;
+static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st) {
   const LatDesc &L = s.lat;
-  const int nxt = (L.nx + sh.tx - 1) / sh.tx, nyt = (L.ny + sh.ty - 1) / sh.ty, nxy = nxt * nyt;
   std::vector<Tile> all;
-  // planes a chunk reads beyond its own: the dipole and collide passes load
-  // one field plane on each side; the moments pass counts one for the
-  // dipole planes its ring loads ahead of its first plane
-  const int halo[3] = {1, 2, 2};
-  for (int pass = 0; pass < 3; ++pass) {
-    s.mf_off[pass] = (int)all.size();
-    s.mf_ntiles[pass] = 0;
-    if (!fn[pass]) continue;
-    int res = 0;
-    if (prepare_kernel(fn[pass], sh.tx * sh.ty, mf_smem(P.nc, sh.tx, sh.ty, pass), &res) != cudaSuccess)
-      return LB3DC_ECUDA;
-    const int k = mf_chunks(L.nz, nxy, res, halo[pass]);
+  // a chunk of any pass works on one plane beyond each of its ends
+  for (int pass = 0; pass < EQ_PASSES; ++pass) {
+    s.eq_off[pass] = (int)all.size();
+    s.eq_ntiles[pass] = 0;
+    EqKernel kn;
+    if (!eq_kernel_of(P, s, pass, false, sh.tx, sh.ty, &kn)) {
+      if (pass == EQ_MOMENTS || pass == EQ_COLLIDE) return LB3DC_EINVAL;
+      continue;
+    }
+    int tx = sh.tx, ty = sh.ty, res = 0;
+    if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.ny, &tx, &ty);
+    if (fp32_prepare_kernel(kn.fn, kn.threads, kn.smem, &res) != cudaSuccess) return LB3DC_ECUDA;
+    const int nxy = ((L.nx + tx - 1) / tx) * ((L.ny + ty - 1) / ty);
+    const int k = fp32_z_chunks(L.nz, nxy, res, 2);
     for (int c = 0; c < k; ++c) {
       const int z0 = (int)((long long)L.nz * c / k), z1 = (int)((long long)L.nz * (c + 1) / k);
-      for (int y0 = 0; y0 < L.ny; y0 += sh.ty)
-        for (int x0 = 0; x0 < L.nx; x0 += sh.tx) {
+      for (int y0 = 0; y0 < L.ny; y0 += ty)
+        for (int x0 = 0; x0 < L.nx; x0 += tx) {
           Tile t;
           t.lat = 0;
           t.x0 = (short)x0;
@@ -1442,26 +957,15 @@ static int mf_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
           all.push_back(t);
         }
     }
-    s.mf_ntiles[pass] = (int)all.size() - s.mf_off[pass];
-    s.mf_grid[pass] = std::min(s.mf_ntiles[pass], res);
+    s.eq_ntiles[pass] = (int)all.size() - s.eq_off[pass];
   }
-  if (s.mf_tiles) cudaFree(s.mf_tiles);
-  s.mf_tiles = nullptr;
-  if (cudaMalloc(&s.mf_tiles, all.size() * sizeof(Tile)) != cudaSuccess) return LB3DC_ENOMEM;
-  if (cudaMemcpyAsync(s.mf_tiles, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice, st) !=
+  if (s.eq_tiles) cudaFree(s.eq_tiles);
+  s.eq_tiles = nullptr;
+  if (cudaMalloc(&s.eq_tiles, all.size() * sizeof(Tile)) != cudaSuccess) return LB3DC_ENOMEM;
+  if (cudaMemcpyAsync(s.eq_tiles, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice, st) !=
       cudaSuccess)
     return LB3DC_ECUDA;
   return cudaStreamSynchronize(st) == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;
-}
-
-int fp32_take_error(Fp32State &s, cudaStream_t st) {
-  if (!s.err) return LB3DC_OK;
-  int v = 0;
-  if (cudaMemcpyAsync(&v, s.err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
-    return LB3DC_ECUDA;
-  if (v) cudaMemsetAsync(s.err, 0, sizeof(int), st);
-  return v;
 }
 
 // Lees-Edwards lattices: the compact pre-stream boundary planes from the
@@ -1511,26 +1015,10 @@ static int rebuild_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh,
     if (rc) return rc;
   }
   if (sh.split == 3) {
-    if (!fp32_mf_eligible(P)) return LB3DC_ENOTSUP;
-    const void *a, *b, *c;
-    if (!mf_fns(P.nc, (s.lat.flags & LAT_ROCK) != 0, (s.lat.flags & LAT_BODY) != 0, sh.tx, sh.ty, true,
-                &a, &b, &c, s.le_h[0] != nullptr))
-      return LB3DC_EINVAL;
-    int rc = ensure_mf(P, s, st);
-    if (rc) return rc;
-    if (s.mf_tx != sh.tx || s.mf_ty != sh.ty) {
-      s.mf_tx = s.mf_ty = 0;
-      if ((rc = encode_mf_map(&s.tm1, s.MF1, P, sh.tx, sh.ty)) != LB3DC_OK) return rc;
-      if (P.nc == 3) {
-        if ((rc = encode_mf_map(&s.tm2, s.MF2, P, sh.tx, sh.ty)) != LB3DC_OK) return rc;
-        if ((rc = encode_mf_map(&s.tmd, s.DD, P, sh.tx, sh.ty)) != LB3DC_OK) return rc;
-      } else {
-        s.tm2 = s.tmd = s.tm1;  // unused by the binary kernels
-      }
-      s.mf_tx = sh.tx;
-      s.mf_ty = sh.ty;
-    }
-    if ((rc = mf_build_tiles(P, s, sh, st)) != LB3DC_OK) return rc;
+    if (!fp32_eq_eligible(P)) return LB3DC_ENOTSUP;
+    int rc = ensure_eq(P, s, st);
+    if (rc == LB3DC_OK) rc = eq_build_tiles(P, s, sh, st);
+    if (rc != LB3DC_OK) return rc;
   }
   std::vector<Tile> tiles;
   fp32_tiles_for(s.lat, 0, sh, tiles);
@@ -1564,7 +1052,7 @@ int fp32_set_shape(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaS
   // Lees-Edwards lattices and lattices with inflow boundaries run the
   // staged split strategy only
   if ((s.le_h[0] && sh.split < 2) || (s.lat.invk && sh.split != 2)) return LB3DC_ENOTSUP;
-  if (sh.split == 3 && !fp32_mf_eligible(P)) return LB3DC_ENOTSUP;
+  if (sh.split == 3 && !fp32_eq_eligible(P)) return LB3DC_ENOTSUP;
   if (sh.split && !s.M) return LB3DC_EINVAL;
   if (sh.split < 0 || sh.split > 3) return LB3DC_EINVAL;
   if (sh.zc < 1) return LB3DC_EINVAL;
@@ -1585,7 +1073,7 @@ std::vector<FusedShape> fp32_candidate_shapes(const DevParams &P) {
   }
   // strategy 3 chunks z per pass from each pass's resident grid: one
   // candidate per tile shape (its zc is not used)
-  if (fp32_mf_eligible(P)) {
+  if (fp32_eq_eligible(P)) {
     for (auto &t : xy) {
       if (t[0] > 2 * P.nx && t[0] > 16) continue;
       out.push_back(FusedShape{t[0], t[1], 16, 3});
@@ -1698,19 +1186,17 @@ void fp32_free(Fp32State &s) {
   if (s.d_tiles) cudaFree(s.d_tiles);
   if (s.M) cudaFree(s.M);
   if (s.J) cudaFree(s.J);
-  if (s.MF1) cudaFree(s.MF1);
-  if (s.MF2) cudaFree(s.MF2);
-  if (s.DD) cudaFree(s.DD);
-  if (s.MFp) cudaFree(s.MFp);
-  if (s.DS) cudaFree(s.DS);
-  if (s.err) cudaFree(s.err);
-  if (s.mf_tiles) cudaFree(s.mf_tiles);
-  s.MF1 = s.MF2 = s.DD = nullptr;
-  s.MFp = nullptr;
-  s.DS = nullptr;
-  s.mf_tiles = nullptr;
-  s.err = nullptr;
-  s.mf_tx = s.mf_ty = 0;
+  if (s.psi) cudaFree(s.psi);
+  if (s.o1) cudaFree(s.o1);
+  if (s.o2) cudaFree(s.o2);
+  if (s.o3) cudaFree(s.o3);
+  if (s.mask) cudaFree(s.mask);
+  if (s.eq_tiles) cudaFree(s.eq_tiles);
+  s.psi = nullptr;
+  s.o1 = s.o3 = nullptr;
+  s.o2 = nullptr;
+  s.mask = nullptr;
+  s.eq_tiles = nullptr;
   if (s.stage) cudaFree(s.stage);
   s.stage = nullptr;
   for (int i = 0; i < 4; ++i) {
@@ -1745,6 +1231,7 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   s.lat = fp32_make_desc(P, rho0, 0, any);
   attach_le(s);
   s.lat.parity = 0;
+  s.rock = rockp;
   // one FP64 plane at a time through two staging planes: the copy of plane
   // cq + 1 (copy stream) overlaps the conversion of plane cq (populations to
   // deviations, dipoles rounded to FP32, into both buffers); xev[b] marks
@@ -1875,25 +1362,29 @@ int fp32_step(const DevParams &P, Fp32State &s, const uint8_t *rock, cudaStream_
 }
 
 int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, cudaStream_t st,
-             const LEStep *le) {
+             const LEStep *le, bool le_per_step) {
   FusedShape sh{s.tx, s.ty, s.zc, s.split};
   const bool rk = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
   if (le && !s.le_h[0]) return LB3DC_ESTATE;
-  // kernels per step: the pass(es), two Lees-Edwards halo kernels, the parity flip
+  // kernels per step: the pass(es) (ternary strategy 3: one more after its
+  // first step), two Lees-Edwards halo kernels, and the parity flip (strategy
+  // 3: one for the whole loop)
   const int passes = sh.split ? (P.nc == 3 ? 3 : 2) : 1;
-  const int per_step = passes + (le ? 2 : 0) + 1;
   for (int i = 0; i < nsteps; ++i) {
+    const LEStep *l = le ? le + (le_per_step ? i : 0) : nullptr;
+    const bool flip = sh.split != 3 || i == nsteps - 1;
     if (s.timer) s.timer->start(st);
     cudaError_t e = sh.split == 3
-                        ? launch_mf(P, s, rock, st, le)
+                        ? eq_step(P, s, rock, i == 0, i == nsteps - 1, l, st)
                         : fp32_launch_fused(P.nc, rk, body, sh, s.d_lat, s.d_tiles, s.ntiles, 0,
                                             s.f[0], s.f[1], s.db[0], s.db[1], rock, s.S, st, s.M,
-                                            s.J, le, &P);
+                                            s.J, l, &P);
     if (s.timer) {
       s.timer->stop(st);
-      s.timer->launches += per_step;
+      s.timer->launches += passes + (sh.split == 3 && P.nc == 3 && i > 0 ? 1 : 0) + (le ? 2 : 0) + (flip ? 1 : 0);
     }
     if (e != cudaSuccess) return LB3DC_ECUDA;
+    if (!flip) continue;
     e = fp32_flip_parity(s.d_lat, 1, st);
     if (e != cudaSuccess) return LB3DC_ECUDA;
     s.lat.parity ^= 1;

@@ -5,8 +5,6 @@
 
 #include <vector>
 
-#include <cuda.h>
-
 #include "common.cuh"
 #include "reduce.h"
 
@@ -76,21 +74,16 @@ struct Fp32State {
   float *le_h[2] = {nullptr, nullptr};  // Lees-Edwards halo planes (see LatDesc)
   float2 *le_p[2] = {nullptr, nullptr};
   float *le_b[4] = {nullptr, nullptr, nullptr, nullptr};
-  // moment-field strategy (split 3): the halo-padded moment fields (and
-  // dipole field, ternary), the plain momentum plane, the tensor maps of their
-  // TMA boxes (encoded for the tile shape mf_tx x mf_ty) and the device flag
-  // of a wait that gave up
-  float4 *MF1 = nullptr, *MF2 = nullptr, *DD = nullptr;
-  float2 *MFp = nullptr;
-  float *DS = nullptr;
-  int *err = nullptr;
-  CUtensorMap tm1{}, tm2{}, tmd{};
-  int mf_tx = 0, mf_ty = 0;
-  // its tile lists, one per pass (moments, dipole, collide), each chunking z
-  // so that the tiles fill the pass's resident grid: mf_ntiles[p] tiles at
-  // mf_tiles + mf_off[p], launched on mf_grid[p] CTAs
-  Tile *mf_tiles = nullptr;
-  int mf_ntiles[3] = {0, 0, 0}, mf_off[3] = {0, 0, 0}, mf_grid[3] = {0, 0, 0};
+  // strategy 3 (fp32_eqstate.h): its fields beside M, the neighbour mask of a
+  // lattice with rock, and its tile lists, one per pass, each chunking z so that the tiles fill the pass's resident grid:
+  // eq_ntiles[p] tiles at eq_tiles + eq_off[p]
+  float2 *psi = nullptr;  // ternary (a binary lattice's M holds psi)
+  float4 *o1 = nullptr, *o3 = nullptr;
+  float *o2 = nullptr;
+  uint32_t *mask = nullptr;
+  const uint8_t *rock = nullptr;  // the handle's rock flags, as of the last upload
+  Tile *eq_tiles = nullptr;
+  int eq_ntiles[4] = {0, 0, 0, 0}, eq_off[4] = {0, 0, 0, 0};
 };
 
 // Launch configuration of the fused kernel.
@@ -98,8 +91,8 @@ struct FusedShape {
   int tx, ty, zc;
   int split = 0;  // 0: one fused pass per step; 1: moments (+ dipole) + collide passes;
                   // 2: as 1 with the asynchronously staged collide pass (no J field);
-                  // 3: moment field + TMA-fed dipole/force/equilibrium pass (full
-                  //    relaxation only, single lattices)
+                  // 3: as 1, carrying the equilibrium's arguments from step to step
+                  //    (full relaxation only)
 };
 
 long long fp32_footprint(const lb3dc_params &p);
@@ -114,10 +107,10 @@ int fp32_download(const DevParams &P, const lb3dc_params &p, Fp32State &s, doubl
 // One step; le gives this step's Lees-Edwards offset (null: periodic).
 int fp32_step(const DevParams &P, Fp32State &s, const uint8_t *rock, cudaStream_t st,
               const LEStep *le = nullptr);
-// nsteps steps; le (null: periodic) is applied unchanged to every step, as the
-// autotuner wants; a Lees-Edwards time loop advances one step at a time.
+// nsteps steps; le (null: periodic) holds one Lees-Edwards offset, applied to
+// every step, or with le_per_step one for each step.
 int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, cudaStream_t st,
-             const LEStep *le = nullptr);
+             const LEStep *le = nullptr, bool le_per_step = false);
 int fp32_dump(const DevParams &P, Fp32State &s, int field, const uint8_t *rock, double *out,
               cudaStream_t st);
 cudaError_t fp32_reduce_conservation(const DevParams &P, Fp32State &s, const uint8_t *rock,
@@ -157,6 +150,9 @@ cudaError_t fp32_planes_to_fp64(const float *src, double *dst, long long S, long
 inline long long fp32_moment_bytes(int nc) { return nc == 3 ? 32 : 8; }
 inline long long fp32_own_bytes(int nc) { return nc == 3 ? 48 : 32; }
 // Flips the parity of every active lattice (one tiny kernel).
+// Raises the dynamic shared memory limit of a kernel and returns how many of its
+// CTAs are resident at once on the current device (kept per kernel and device).
+cudaError_t fp32_prepare_kernel(const void *fn, int nthreads, size_t smem, int *ctas_total);
 cudaError_t fp32_flip_parity(LatDesc *d_lat, int nlat, cudaStream_t st);
 size_t fp32_fused_smem(int nc, const FusedShape &sh);
 int fp32_set_shape(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st);
@@ -165,15 +161,12 @@ std::vector<FusedShape> fp32_candidate_shapes(const DevParams &P);
 int fp32_autotune(const DevParams &P, Fp32State &s, const uint8_t *rock, double *ms_out,
                   int *ntried, cudaStream_t st, const LEStep *le = nullptr);
 int fp32_fused_ctas_per_sm(int nc, bool rock, bool body, const FusedShape &sh);
-// The moment-field strategy applies: every component relaxes fully
-// (omega = 1), periodic or walled lattice without Lees-Edwards planes or
-// inflow boundaries, at least 2 sites across in x and y.
-bool fp32_mf_eligible(const DevParams &P);
-// Bytes of the moment and dipole fields of strategy 3.
-long long fp32_mf_bytes(const DevParams &P);
-// The device error flag of the handle's kernels (0, or LB3DC_ETIMEOUT when a
-// bounded wait gave up), read and cleared; LB3DC_OK when no flag exists.
-int fp32_take_error(Fp32State &s, cudaStream_t st);
+// Strategy 3 applies: every component relaxes fully (omega = 1), no inflow
+// boundaries, Lees-Edwards planes on binary lattices only, at least 2 sites
+// across in x and y.
+bool fp32_eq_eligible(const DevParams &P);
+// z chunks of a pass over a lattice of nxy column tiles (see fp32_path.cu).
+int fp32_z_chunks(int nz, int nxy, int resident, int halo);
 
 }  // namespace lb3d
 #endif

@@ -16,26 +16,6 @@
 // memory while marching in z, so every field is loaded from global memory
 // once per tile plane (halos hit L2).
 
-// Asynchronous copies global -> shared (cp.async, 4/8/16 bytes) in commit
-// groups; a thread waits for its own groups, a barrier then publishes them.
-__device__ __forceinline__ void cp_async4(void *dst, const void *src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
-  const unsigned s = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // Dipole pass: the {rho_b - rho_r, da} entries of M stream through a
 // five-slot ring, refilled with cp.async three planes ahead of the plane
 // being relaxed (one barrier per plane); each thread also prefetches its own
