@@ -28,11 +28,11 @@
 //             127-330), body force, velocities, and the arguments (or, in the
 //             last step of a loop, the populations) of the next state.
 //
-// The arguments live in planes 0..3 of each component of the buffer the
-// loop's first pass has read (dead from then on), the dipoles are updated in
-// place, so a loop needs no memory beyond the pass fields and flips the
-// lattice's parity once.  Lattices of an ensemble share the launches through
-// their descriptors and tile lists, as in the other strategies.
+// The arguments and the dipoles of the steps between lie in X.Q, which a
+// single lattice lays over the buffer the loop's first pass has read (dead
+// from then on), so a loop needs no memory beyond the pass fields, and flips
+// the lattice's parity once.  Lattices of an ensemble share the launches
+// through their descriptors and tile lists, as in the other strategies.
 #include <algorithm>
 #include <type_traits>
 
@@ -231,6 +231,9 @@ __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return mul2(a, b); 
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
 __device__ __forceinline__ float vneg(float a) { return -a; }
+__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
+// one instruction: b scaled by -1 is exact
+__device__ __forceinline__ float2 vsub(float2 a, float2 b) { return fma2(f2(-1.0f), b, a); }
 __device__ __forceinline__ float2 vneg(float2 a) { return neg2(a); }
 
 // The equilibrium of a site from its arguments: eq_store's arithmetic with
@@ -256,10 +259,6 @@ struct EqSite {
   }
 };
 
-#ifndef EQ_TX
-#define EQ_TX 32
-#define EQ_TY 8
-#endif
 template <typename V, int TX, int TY, bool ROCK>
 struct EqGeom {
   static constexpr bool SURF = sizeof(V) == 4;
@@ -267,33 +266,39 @@ struct EqGeom {
   static constexpr int NTH = (AN + 31) / 32 * 32;
   static constexpr int DS = ROCK ? 2 : 1;  // a bounced pull returns the own site's D populations
   static constexpr int PLANES = 4 * DS + 2 * 8 + 2 * 4;
-  static constexpr int DIP = SURF ? 3 * AN * 16 : 0;
-  static constexpr int SMEM = DIP + PLANES * AN * (int)sizeof(V);
-#ifndef MBS
-#define MBS 2
-#endif
-#ifndef MBR
-#define MBR 2
-#endif
-  static constexpr int MINB = SURF ? MBS : MBR;
+  static constexpr int DIP = SURF ? 4 * AN * 16 : 0;
+  // staged own entries, two slots: the arguments (red and blue: two float4),
+  // for the surfactant the other launch's o1 and o2
+  static constexpr int STAGE = SURF ? 2 * (NTH * 16 + NT * 20) : 2 * NTH * 32;
+  static constexpr int SMEM = DIP + STAGE + PLANES * AN * (int)sizeof(V);
+  // 80 registers a thread: two CTAs of 32 x 8 tiles, four of 16 x 8
+  static constexpr int MINB = NTH > 192 ? 2 : 4;
 };
+
+// All threads of the CTA, from the tile's and the halo's loop alike.
+template <int N>
+__device__ __forceinline__ void cta_barrier() {
+  asm volatile("bar.sync 1, %0;\n" ::"n"(N) : "memory");
+}
 
 template <typename V, int TX, int TY, bool ROCK, bool LE>
 __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY, ROCK>::MINB)
-    k_eq_moments(const LatDesc *__restrict__ lats, const Tile *__restrict__ tiles, int ntiles, const float *f0,
-                 const float *f1, const float *db0, const float *db1, const uint32_t *__restrict__ mask,
-                 const __grid_constant__ EqFields X) {
+    k_eq_moments(const LatDesc *__restrict__ lats, const Tile *__restrict__ tiles, int ntiles,
+                 const uint32_t *__restrict__ mask, const __grid_constant__ EqFields X) {
   using G = EqGeom<V, TX, TY, ROCK>;
   constexpr bool SURF = G::SURF;
-  constexpr int NT = G::NT, AW = G::AW, AN = G::AN, DS = G::DS;
+  constexpr int NT = G::NT, AW = G::AW, AN = G::AN, DS = G::DS, NTH = G::NTH;
   static_assert(NT % 32 == 0, "a warp holds tile sites or halo sites");
   extern __shared__ float4 sme[];
   __shared__ LatDesc sLat;
-  float4 *dip = sme;                                 // [3][AN] dipoles
-  V *pD = reinterpret_cast<V *>(sme + G::DIP / 16);  // [DS][4][AN]
+  float4 *dip = sme;                       // [4][AN] dipoles
+  float4 *stA = sme + G::DIP / 16;         // [2][NTH] arguments
+  float4 *stB = stA + 2 * NTH;             // [2][NTH] arguments, or [2][NT] o1
+  float *stC = reinterpret_cast<float *>(stB + 2 * NT);  // surfactant: [2][NT] o2
+  V *pD = reinterpret_cast<V *>(reinterpret_cast<unsigned char *>(stA) + G::STAGE);  // [DS][4][AN]
   V *pZ = pD + 4 * DS * AN;                          // [2][8][AN]
   V *pU = pZ + 16 * AN;                              // [2][4][AN]
-  const unsigned S = X.S;
+  const size_t S = X.S;
   const int tid = threadIdx.x;
   // threads 0 .. NT - 1 own the tile's sites, the others the halo ring: its
   // bottom and top rows with the corners, then its left and right columns
@@ -307,170 +312,191 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
     else
       hx = r - 2 * AW < TY ? 0 : TX + 1, hy = (r - 2 * AW) % TY + 1;
   }
-  const bool part = tid < AN, halo = tid >= NT;
+  const bool part = tid < AN;
   const int s = hx + AW * hy;
-  // a halo site's directions into the tile: lo, its side (left, bottom); three
-  // in the plane, one up, one down
-  const bool row = hy == 0 || hy == TY + 1, lo = row ? hy == 0 : hx == 0;
-  const int hq[5] = {row ? (lo ? 2 : 3) : (lo ? 0 : 1), lo ? 6 : 11, row ? (lo ? 10 : 7) : (lo ? 7 : 10),
-                     row ? (lo ? 14 : 16) : (lo ? 8 : 12), row ? (lo ? 15 : 17) : (lo ? 9 : 13)};
-  int off[5];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    off[k] = s;
-#pragma unroll
-    for (int q = 0; q < 18; ++q)
-      if (q != 4 && q != 5 && hq[k] == q) off[k] = dir_slot(q) * AN + s;
-  }
   pdl_launch_next();
   pdl_wait_previous();
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const Tile T = tiles[t];
     if (tid == 0) sLat = lats[T.lat];
-    __syncthreads();
+    cta_barrier<NTH>();
     const LatDesc &Lg = sLat;
     const int nx = Lg.nx, ny = Lg.ny, nz = Lg.nz, pl = nx * ny;
-    const int par = Lg.parity;
-    const float *Q0 = (par ? f1 : f0) + Lg.base + (SURF ? (size_t)38 * S : 0), *Q1 = Q0 + (size_t)19 * S;
-    const float *DB = SURF ? (par ? db0 : db1) + Lg.base : nullptr;  // this loop's dipoles
     const float rho0 = Lg.rho0;
     const int x0 = T.x0, y0 = T.y0, z0 = T.z0, zc = T.zc;
     const int vx = x0 - 1 + hx, vy = y0 - 1 + hy;
     const int wy = wrapz(vy, ny), xy = wrapz(vx, nx) + nx * wy;
-    const bool act = !halo && vx < nx && vy < ny;
     const int side = !LE || !part ? -1 : vx == -1 ? 0 : vx == nx ? 1 : -1;  // a sheared halo site
-    // the arguments of the plane evaluated next (a sheared halo site: the
-    // populations of the stage-6 halo plane that enter the lattice)
-    V q[4] = {vset(V(), 0.f), vset(V(), 0.f), vset(V(), 0.f), vset(V(), 0.f)};
-    float3 dd = make_float3(0.f, 0.f, 0.f);
+    // the arguments of the plane evaluated next, copied one iteration ahead
+    // (asynchronously into shared memory: held in registers, the 16-byte loads
+    // were moved out of their register quads at once and their latency with
+    // them); the dipoles go straight into their ring
+    const float4 *qa = X.Q[Lg.parity] + (SURF ? 2 * S : 0) + Lg.base + xy, *qb = qa + S;
+    int zl = wrapz(z0 - 1, nz);  // z of the plane copied next
     auto load = [&](int m) {
-      const unsigned i = (unsigned)(xy + pl * wrapz(z0 - 1 + m, nz));
+      const int i = pl * zl;
+      cp_async16(stA + (m & 1) * NTH + tid, qa + i);
+      cp_async16(SURF ? dip + (m & 3) * AN + s : stB + (m & 1) * NTH + tid, qb + i);
+      zl = zl + 1 == nz ? 0 : zl + 1;
+    };
+    auto site = [&](int m) {
+      const float4 la = stA[(m & 1) * NTH + tid];
       if constexpr (SURF) {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = Q0[k * S + i];
-        dd = make_float3(DB[i], DB[S + i], DB[2 * (size_t)S + i]);
+        return EqSite<V>(rho0, la.x, la.y, la.z, la.w);
       } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) q[k] = make_float2(Q0[k * S + i], Q1[k * S + i]);
+        const float4 lb = stB[(m & 1) * NTH + tid];
+        return EqSite<V>(rho0, make_float2(la.x, la.y), make_float2(la.z, la.w), make_float2(lb.x, lb.y),
+                         make_float2(lb.z, lb.w));
       }
     };
-    // waiting: U of the last plane; those along z (4: last two planes, 5: last
-    // plane and, for a bounce, the one before); at rest
+    // the populations of the stage-6 halo plane at a sheared halo site
+    const int NP = ny * nz;
+    auto sheared = [&](int d, int z) {
+      const float *h = Lg.le_h[side] + wy + ny * z;
+      return make_float2(h[d * NP], h[(19 + d) * NP]);
+    };
+    if (part) load(0);
+    cp_async_commit();
+    if (tid >= NT) {
+      // ---- halo: lo, the site's side (left, bottom); its directions into the
+      // tile: three in the plane, one up, one down
+      const bool row = hy == 0 || hy == TY + 1, lo = row ? hy == 0 : hx == 0;
+      const int hq[5] = {row ? (lo ? 2 : 3) : (lo ? 0 : 1), lo ? 6 : 11, row ? (lo ? 10 : 7) : (lo ? 7 : 10),
+                         row ? (lo ? 14 : 16) : (lo ? 8 : 12), row ? (lo ? 15 : 17) : (lo ? 9 : 13)};
+      int off[5];
+#pragma unroll
+      for (int k = 0; k < 5; ++k) {
+        off[k] = s;
+#pragma unroll
+        for (int q = 0; q < 18; ++q)
+          if (q != 4 && q != 5 && hq[k] == q) off[k] = dir_slot(q) * AN + s;
+      }
+      const V sg = vset(V(), lo ? 1.0f : -1.0f), sd = vset(V(), lo != row ? 1.0f : -1.0f);
+      V up = vset(V(), 0.f);
+#pragma unroll 1
+      for (int m = 0; m <= zc + 1; ++m) {
+        if (part) {
+          const int z = zl == 0 ? nz - 1 : zl - 1;  // of plane m
+          V *mD = pD + (m % DS) * 4 * AN, *mZ = pZ + (m & 1) * 8 * AN, *mU = pU + ((m - 1) & 1) * 4 * AN;
+          if (m > 0) mU[off[3]] = up;
+          cp_async_wait<0>();
+          const EqSite<V> E = site(m);
+          if (m <= zc) load(m + 1);
+          cp_async_commit();
+          const V t1 = row ? E.ty : E.tx;
+          V ev, od, z0v, z1v, z2v;
+          E.pair(t1, ev, od);
+          z0v = vfma(sg, od, ev);
+          E.pair(vadd(E.tx, E.ty), ev, od);
+          z1v = vfma(sg, od, ev);
+          E.pair(vsub(E.tx, E.ty), ev, od);
+          z2v = vfma(sd, od, ev);
+          E.pair(vadd(t1, E.tz), ev, od);
+          const V A = vfma(sg, od, ev);
+          E.pair(vsub(t1, E.tz), ev, od);
+          const V B = vfma(sg, od, ev);
+          up = lo ? A : B;
+          V down = lo ? B : A;
+          if constexpr (LE && !SURF)
+            if (side >= 0)
+              z0v = sheared(hq[0], z), z1v = sheared(hq[1], z), z2v = sheared(hq[2], z), up = sheared(hq[3], z),
+              down = sheared(hq[4], z);
+          mZ[off[0]] = z0v;
+          mZ[off[1]] = z1v;
+          mZ[off[2]] = z2v;
+          mD[off[4]] = down;
+        }
+        if (m < 2) continue;
+        cta_barrier<NTH>();
+        cta_barrier<NTH>();
+      }
+      continue;
+    }
+    // ---- tile.  Waiting: U of the last plane; those along z (4: last two
+    // planes, 5: last plane and, for a bounce, the one before); at rest
+    const bool act = vx < nx && vy < ny;
     V ur[4], u4 = vset(V(), 0.f), u4p = u4, d5 = u4, d5p = u4, rest = u4;
     ur[0] = ur[1] = ur[2] = ur[3] = u4;
-    float3 d0 = make_float3(0.f, 0.f, 0.f), d1 = d0, d2 = d0;  // own dipoles of planes m, m - 1, m - 2
-    float4 own = make_float4(0.f, 0.f, 0.f, 0.f), own_next = own;  // SURF: the other launch's o1
-    float opz = 0.f, opz_next = 0.f;
-    uint32_t mk = 0, mk_next = 0;
-    if (part) load(0);
-    for (int m = 0; m <= zc + 1; ++m) {
-      const V rest1 = rest, u4q = u4p;  // plane m - 1, plane m - 2
-      if (part) {
-        const EqSite<V> E(rho0, q[0], q[1], q[2], q[3]);
-        V *mD = pD + (m % DS) * 4 * AN, *mZ = pZ + (m & 1) * 8 * AN, *mU = pU + ((m - 1) & 1) * 4 * AN;
-        V ev, od;
-        if (!halo) {
-          if (m > 0)
+    int zo = z0 == 0 ? nz - 1 : z0 - 1;  // z of the plane before the one summed next
+    const size_t own = (size_t)Lg.base + xy;
+    uint32_t mk = 0, mkn = 0;  // rock mask of the plane summed, summed next
+    auto iterate = [&](auto parity, int m) {
+      constexpr int P = decltype(parity)::value;  // m & 1
+      const V rest1 = rest, u4q = u4p;            // plane m - 1, plane m - 2
+      V *mD = pD + (DS == 2 ? P * 4 * AN : 0) + s, *mZ = pZ + P * 8 * AN + s, *mU = pU + (1 - P) * 4 * AN + s;
+      const float4 *dm = dip + (m & 2) * AN + s, *dx = dip + (2 - (m & 2)) * AN + s;  // dipole slots of this pair, the last
+      if (m > 0)
 #pragma unroll
-            for (int k = 0; k < 4; ++k) mU[k * AN + s] = ur[k];
-          u4p = u4, d5p = d5, rest = E.rest;
-          auto put = [&](int d, V v) {
-            if (d == 4) u4 = v;
-            else if (d == 5) d5 = v;
-            else if (cz(d) == 1) ur[dir_slot(d) % 4] = v;
-            else (cz(d) ? mD : mZ)[dir_slot(d) * AN + s] = v;
-          };
+        for (int k = 0; k < 4; ++k) mU[k * AN] = ur[k];
+      u4p = u4, d5p = d5;
+      {
+        cp_async_wait<0>();
+        const EqSite<V> E = site(m);
+        rest = E.rest;
+        const int z = zl == 0 ? nz - 1 : zl - 1;  // of plane m
+        if (m <= zc) load(m + 1);
+        mk = mkn;
+        if ((ROCK || SURF) && m >= 1 && m <= zc) {
+          // of plane m, summed in the next iteration
+          const int i = pl * z;
+          if (ROCK) mkn = __ldg(mask + own + i);
+          if (SURF && act) {
+            cp_async16(stB + P * NT + tid, X.o1 + own + i);
+            cp_async4(stC + P * NT + tid, X.o2 + own + i);
+          }
+        }
+        cp_async_commit();
+        V ev, od;
+        auto put = [&](int d, V v) {
+          if (d == 4) u4 = v;
+          else if (d == 5) d5 = v;
+          else if (cz(d) == 1) ur[dir_slot(d) % 4] = v;
+          else (cz(d) ? mD : mZ)[dir_slot(d) * AN] = v;
+        };
 #define LB3D_EQP(E_, I, J)  \
   E.pair(E_, ev, od);       \
   put(I, vadd(ev, od));     \
-  put(J, vadd(ev, vneg(od)));
-          LB3D_EQP(E.tx, 0, 1)
-          LB3D_EQP(E.ty, 2, 3)
-          LB3D_EQP(E.tz, 4, 5)
-          LB3D_EQP(vadd(E.tx, E.ty), 6, 11)
-          LB3D_EQP(vadd(E.tx, vneg(E.ty)), 7, 10)
-          LB3D_EQP(vadd(E.tx, E.tz), 8, 13)
-          LB3D_EQP(vadd(E.tx, vneg(E.tz)), 9, 12)
-          LB3D_EQP(vadd(E.ty, E.tz), 14, 17)
-          LB3D_EQP(vadd(E.ty, vneg(E.tz)), 15, 16)
+  put(J, vsub(ev, od));
+        LB3D_EQP(E.tx, 0, 1)
+        LB3D_EQP(E.ty, 2, 3)
+        LB3D_EQP(E.tz, 4, 5)
+        LB3D_EQP(vadd(E.tx, E.ty), 6, 11)
+        LB3D_EQP(vsub(E.tx, E.ty), 7, 10)
+        LB3D_EQP(vadd(E.tx, E.tz), 8, 13)
+        LB3D_EQP(vsub(E.tx, E.tz), 9, 12)
+        LB3D_EQP(vadd(E.ty, E.tz), 14, 17)
+        LB3D_EQP(vsub(E.ty, E.tz), 15, 16)
 #undef LB3D_EQP
-        } else {
-          if (m > 0) mU[off[3]] = ur[0];
-          const V t1 = row ? E.ty : E.tx, sg = vset(V(), lo ? 1.0f : -1.0f), sd = vset(V(), lo != row ? 1.0f : -1.0f);
-          E.pair(t1, ev, od);
-          mZ[off[0]] = vfma(sg, od, ev);
-          E.pair(vadd(E.tx, E.ty), ev, od);
-          mZ[off[1]] = vfma(sg, od, ev);
-          E.pair(vadd(E.tx, vneg(E.ty)), ev, od);
-          mZ[off[2]] = vfma(sd, od, ev);
-          E.pair(vadd(t1, E.tz), ev, od);
-          const V A = vfma(sg, od, ev);
-          E.pair(vadd(t1, vneg(E.tz)), ev, od);
-          const V B = vfma(sg, od, ev);
-          ur[0] = lo ? A : B;
-          mD[off[4]] = lo ? B : A;
-        }
         if constexpr (LE && !SURF) {
-          if (side >= 0) {
-            // across the sheared boundary: x = -1 or x = nx, which may lie
-            // inside the tile's span
-            const int NP = ny * nz;
-            const float *h = Lg.le_h[side] + wy + ny * wrapz(z0 - 1 + m, nz);
-            auto at = [&](int d) { return make_float2(h[d * NP], h[(19 + d) * NP]); };
-            if (halo) {
-#pragma unroll
-              for (int k = 0; k < 3; ++k) mZ[off[k]] = at(hq[k]);
-              ur[0] = at(hq[3]);
-              mD[off[4]] = at(hq[4]);
-            } else {
-              mZ[dir_slot(1) * AN + s] = at(1);
-              mZ[dir_slot(10) * AN + s] = at(10);
-              mZ[dir_slot(11) * AN + s] = at(11);
-              ur[dir_slot(12)] = at(12);
-              mD[dir_slot(13) * AN + s] = at(13);
-            }
-          }
-        }
-        if (SURF) {
-          d2 = d1, d1 = d0, d0 = dd;
-          dip[(m % 3) * AN + s] = make_float4(dd.x, dd.y, dd.z, 0.f);
-        }
-        if (m <= zc) load(m + 1);
-        if ((ROCK || SURF) && act) {
-          mk = mk_next, own = own_next, opz = opz_next;
-          if (m >= 1 && m <= zc) {
-            const size_t i = (size_t)Lg.base + xy + pl * wrapz(z0 + m - 1, nz);
-            if (ROCK) mk_next = __ldg(mask + i);
-            if (SURF) own_next = X.o1[i], opz_next = X.o2[i];
+          if (side >= 0) {  // x = nx lies inside the tile's span
+            put(1, sheared(1, z)), put(10, sheared(10, z)), put(11, sheared(11, z));
+            put(12, sheared(12, z)), put(13, sheared(13, z));
           }
         }
       }
-      if (m < 2) continue;
-      __syncthreads();
+      if (m < 2) return;
+      zo = zo + 1 == nz ? 0 : zo + 1;  // z of plane m - 1
+      cta_barrier<NTH>();
       if (act) {
-        // the pulled populations of plane m - 1
-        const int gz = wrapz(z0 + m - 2, nz);
-        const size_t self = (size_t)Lg.base + xy + pl * gz;
-        const bool fluid = !ROCK || !(mk >> 18 & 1u);
-        // plane class of d in shared memory: U of plane m - 2, Z of plane
+        // the pulled populations of plane m - 1: U of plane m - 2, Z of plane
         // m - 1, D of plane m; the own site's (plane m - 1) for a bounce
+        const size_t self = own + pl * zo;
+        const bool fluid = !ROCK || !(mk >> 18 & 1u);
         auto plane = [&](int d, bool own_site) {
-          if (cz(d) == 0) return pZ + (((m - 1) & 1) * 8 + dir_slot(d)) * AN + s;
-          if (cz(d) == 1) return pU + (((own_site ? m - 1 : m) & 1) * 4 + dir_slot(d)) * AN + s;
-          return pD + (((own_site ? m - 1 : m) % DS) * 4 + dir_slot(d)) * AN + s;
+          if (cz(d) == 0) return pZ + ((1 - P) * 8 + dir_slot(d)) * AN + s;
+          if (cz(d) == 1) return pU + ((own_site ? 1 - P : P) * 4 + dir_slot(d)) * AN + s;
+          return pD + ((DS == 1 ? 0 : own_site ? 1 - P : P) * 4 + dir_slot(d)) * AN + s;
         };
         // a site on the sheared boundary also leaves them for the stage-8 halo
         // kernel (a rock site the populations it keeps)
-        const int NP = ny * nz;
-        float *lb = nullptr;
-        if (LE && (vx == 0 || vx == nx - 1)) lb = Lg.le_b[vx == 0 ? 3 : 2] + vy + ny * gz;
+        float *lbp = nullptr;
+        if (LE && (vx == 0 || vx == nx - 1)) lbp = Lg.le_b[vx == 0 ? 3 : 2] + vy + ny * zo;
         V r = vset(V(), 0.f), j0 = r, j1 = r, j2 = r;
         float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-        const float4 *dm = dip + ((m + 1) % 3) * AN + s, *dc = dip + ((m + 2) % 3) * AN + s, *dp = dip + (m % 3) * AN + s;
 #pragma unroll
         for (int d = 0; d < 19; ++d) {
-          const bool hit = ROCK && d < 18 && (mk >> d & 1u);
           V v;
+          const bool hit = ROCK && d < 18 && (mk >> d & 1u);
           if (d == 18) {
             v = rest1;
           } else if (d == 4) {
@@ -483,9 +509,9 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
             v = *p;
           }
           if constexpr (LE && !SURF) {
-            if (lb) {
-              lb[d * NP] = fluid ? v.x : rock_dev(d, rho0);
-              lb[(19 + d) * NP] = fluid ? v.y : rock_dev(d, rho0);
+            if (lbp) {
+              lbp[d * NP] = fluid ? v.x : rock_dev(d, rho0);
+              lbp[(19 + d) * NP] = fluid ? v.y : rock_dev(d, rho0);
             }
           }
           const float g = (float)gw(d);
@@ -495,13 +521,9 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
           if (cz(d)) j2 = vfma(vset(V(), g * (float)cz(d)), v, j2);
           if constexpr (SURF) {
             // da = sum_q (n_s(x - c_q, q) g_q) db(x - c_q) + n_s(x, rest) db(x)
-            float3 bb;
-            if (cx(d) == 0 && cy(d) == 0) {
-              bb = cz(d) == 0 ? d1 : cz(d) == 1 ? d2 : d0;
-            } else {
-              const float4 b4 = (cz(d) == 0 ? dc : cz(d) == 1 ? dm : dp)[-cx(d) - AW * cy(d)];
-              bb = make_float3(b4.x, b4.y, b4.z);
-            }
+            // planes m - 2, m - 1, m
+            const float4 *p = cz(d) == 1 ? dx + P * AN : cz(d) == 0 ? (P ? dm : dx + AN) : dm + P * AN;
+            const float4 bb = p[-cx(d) - AW * cy(d)];
             const float ng = g * fmaf(wq(d), rho0, v);
             a0 = fmaf(ng, bb.x, a0);
             a1 = fmaf(ng, bb.y, a1);
@@ -510,13 +532,20 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
         }
         if constexpr (SURF) {
           const float am = Lg.amass[2] * Lg.omega[2];
-          X.o3[self] = make_float4(r, fmaf(am, j0, own.z), fmaf(am, j1, own.w), fmaf(am, j2, opz));
-          X.M[self] = make_float4(own.y - own.x, a0, a1, a2);
+          const float4 o1 = stB[(1 - P) * NT + tid];
+          const float o2 = stC[(1 - P) * NT + tid];
+          X.o3[self] = make_float4(r, fmaf(am, j0, o1.z), fmaf(am, j1, o1.w), fmaf(am, j2, o2));
+          X.M[self] = make_float4(o1.y - o1.x, a0, a1, a2);
         } else if (fluid) {
           put_rb(X, self, Lg, r, j0, j1, j2);
         }
       }
-      __syncthreads();  // the next iteration overwrites the planes read here
+      cta_barrier<NTH>();  // the next iteration overwrites the planes read here
+    };
+#pragma unroll 1
+    for (int m = 0; m <= zc + 1; m += 2) {
+      iterate(std::integral_constant<int, 0>(), m);
+      if (m + 1 <= zc + 1) iterate(std::integral_constant<int, 1>(), m + 1);
     }
   }
 }
@@ -529,7 +558,7 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
 template <int TX, int TY>
 __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
     k_eq_dipole(const LatDesc *__restrict__ lats, const Tile *__restrict__ tiles, int ntiles, float *db0,
-                float *db1, const __grid_constant__ EqFields X) {
+                float *db1, const __grid_constant__ EqFields X, int last) {
   constexpr int NT = TX * TY, AW = TX + 2, AN = AW * (TY + 2), RS = 5, RE = (AN + NT - 1) / NT;
   extern __shared__ float4 sme[];  // [RS][AN]
   __shared__ LatDesc sLat;
@@ -543,7 +572,8 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
     __syncthreads();
     const LatDesc &Lg = sLat;
     const int nx = Lg.nx, ny = Lg.ny, nz = Lg.nz, pl = nx * ny;
-    float *__restrict__ DBo = (Lg.parity ? db0 : db1) + Lg.base;
+    float *DBo = (Lg.parity ? db0 : db1) + Lg.base;
+    float4 *Qd = X.Q[Lg.parity] + 3 * (size_t)S + Lg.base;
     const float4 *Mb = X.M + Lg.base;
     float4 *DD = X.M + (size_t)S + Lg.base;
     const float4 *O3 = X.o3 + Lg.base;
@@ -581,9 +611,12 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
         const float3 d = dipole_site<AW>((const float4 *)sme + (k % RS) * AN, (const float4 *)sme + ((k + 1) % RS) * AN,
                                          (const float4 *)sme + ((k + 2) % RS) * AN, as, Lg, Lg.rho0, own);
         const int i = own_xy + pl * wrapz(z0 + k, nz);
-        DBo[i] = d.x;
-        DBo[(size_t)S + i] = d.y;
-        DBo[2 * (size_t)S + i] = d.z;
+        Qd[i] = make_float4(d.x, d.y, d.z, 0.f);
+        if (last) {
+          DBo[i] = d.x;
+          DBo[(size_t)S + i] = d.y;
+          DBo[2 * (size_t)S + i] = d.z;
+        }
         const float pse = -Lg.em0 * expm1f(-own);
         const float ps = Lg.psi0 + pse;
         const float2 a01 = mul2(make_float2(d.x, d.y), f2(ps));
@@ -597,9 +630,12 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
 
 // ---------------------------------------------------------------------------
 // Collide pass: psi deviations and (ternary) {a, dpsi_s} entries stream
-// through five-slot rings as in the dipole pass; the own entries are loaded
-// one plane ahead into registers.  to_pops: write the populations (the last
-// step of a loop) instead of the equilibrium's arguments.
+// through five-slot rings as in the dipole pass, and the own entries with
+// them (prefetched in registers the 16-byte ones exposed their latency: 78
+// against 70 us at ternary 128^3).  to_pops: write the populations (the last
+// step of a loop) instead of the equilibrium's arguments.  Ternary 128^3: 70
+// us at 16 warps per SM and 62 % issue (the pass that wrote populations every
+// step: 154 us); binary 256x128x128: 66 us (172 us).
 // ---------------------------------------------------------------------------
 // force_ternary with the neighbours' a = d (psi0 + dpsi_s) from the dipole
 // pass: the same operations in the same order.
@@ -723,20 +759,23 @@ __device__ __forceinline__ void force_binary_masked(const float2 *Pm, const floa
 template <int NC, int TX, int TY>
 struct EqCollideGeom {
   static constexpr int NT = TX * TY, AW = TX + 2, AN = AW * (TY + 2), RS = 5;
-  static constexpr int SMEM = RS * AN * (NC == 3 ? 24 : 8);
+  // rings of {a, dpsi_s} (ternary) and psi; the own entries: ternary
+  // {drho_s, P}, the dipole and {drho_r, drho_b}, binary o1 and o2
+  static constexpr int SMEM = RS * (AN * (NC == 3 ? 24 : 8) + NT * (NC == 3 ? 40 : 20));
   static constexpr int MINB = NC == 3 ? 512 / NT : 768 / NT;
 };
 
 template <int NC, int TX, int TY, bool ROCK, bool LE>
 __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
     k_eq_collide(const LatDesc *__restrict__ lats, const Tile *__restrict__ tiles, int ntiles, float *f0, float *f1,
-                 const float *db0, const float *db1, const uint32_t *__restrict__ mask,
-                 const __grid_constant__ EqFields X, int to_pops) {
+                 const uint32_t *__restrict__ mask, const __grid_constant__ EqFields X, int to_pops) {
   using G = EqCollideGeom<NC, TX, TY>;
   constexpr int NT = G::NT, AW = G::AW, AN = G::AN, RS = G::RS, RE = (AN + NT - 1) / NT;
   extern __shared__ float4 sme[];
   float4 *ringA = sme;                                                  // [RS][AN] (ternary)
-  float2 *ringP = reinterpret_cast<float2 *>(sme + (NC == 3 ? RS * AN : 0));  // [RS][AN]
+  float4 *own1 = sme + (NC == 3 ? RS * AN : 0), *own2 = own1 + (NC == 3 ? RS * NT : 0);  // [RS][NT] each
+  float2 *ringP = reinterpret_cast<float2 *>(own2 + RS * NT);                           // [RS][AN]
+  float2 *own3 = ringP + RS * AN;                                                       // [RS][NT]
   __shared__ LatDesc sLat;
   const unsigned S = X.S;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
@@ -755,7 +794,7 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
     const float4 *DD = NC == 3 ? X.M + (size_t)S + base : nullptr;
     const float4 *O1 = X.o1 + base, *O3 = X.o3 + base;
     const float *O2 = X.o2 + base;
-    const float *DBn = NC == 3 ? (par ? db0 : db1) + base : nullptr;
+    float4 *Q = X.Q[par] + base;
     const int x0 = T.x0, y0 = T.y0, z0 = T.z0, zc = T.zc;
     const int gx = x0 + tx, gy = y0 + ty;
     const bool act = gx < nx && gy < ny;
@@ -780,59 +819,60 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
         }
         cp_async8(ringP + sl + s, src);
       }
+      if (act) {
+        const int i = own_xy + pl * gz, o = (r % RS) * NT + tid;
+        if (NC == 3) {
+          cp_async16(own1 + o, O3 + i);
+          cp_async16(own2 + o, Q + 3 * (size_t)S + i);
+          cp_async8(own3 + o, O1 + i);
+        } else {
+          cp_async16(own1 + o, O1 + i);
+          cp_async4(reinterpret_cast<float *>(own3) + o, O2 + i);
+        }
+      }
     };
     load_ring(0);
     load_ring(1);
     load_ring(2);
     cp_async_commit();
-    // the own entries of the plane collided next
-    float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);  // drho_s (ternary), P
-    float2 drn = make_float2(0.f, 0.f);
-    float3 dn = make_float3(0.f, 0.f, 0.f);
-    uint32_t mkn = 0;
-    auto load_own = [&](int k) {
-      const int i = own_xy + pl * wrapz(z0 + k, nz);
-      if (ROCK) mkn = __ldg(mask + base + i);
-      if (NC == 3) {
-        drn = *reinterpret_cast<const float2 *>(O1 + i);
-        pn = O3[i];
-        dn = make_float3(DBn[i], DBn[(size_t)S + i], DBn[2 * (size_t)S + i]);
-      } else {
-        const float4 o = O1[i];
-        drn = make_float2(o.x, o.y);
-        pn = make_float4(0.f, o.z, o.w, O2[i]);
-      }
-    };
-    if (act) load_own(0);
+    uint32_t mkn = 0;  // rock mask of the plane collided next
+    if (ROCK && act) mkn = __ldg(mask + base + own_xy + pl * z0);
     for (int k = 0; k < zc; ++k) {
       if (k + 3 <= zc + 1) load_ring(k + 3);
       cp_async_commit();
-      const float4 pp = pn;
-      const float2 drb = drn;
-      const float3 dd = dn;
       const uint32_t mk = mkn;
-      if (act && k + 1 < zc) load_own(k + 1);
+      if (ROCK && act && k + 1 < zc) mkn = __ldg(mask + base + own_xy + pl * wrapz(z0 + k + 1, nz));
       cp_async_wait<1>();  // ring planes up to k + 2 landed (this thread's copies)
       __syncthreads();     // ... and everybody's
       if (!act) continue;
       const int gz = wrapz(z0 + k, nz);
       const int self = own_xy + pl * gz;
-      float *fo = (to_pops ? (par ? f0 : f1) : (par ? f1 : f0)) + base + self;
       if (ROCK && (mk >> 18 & 1u)) {
-        // a rock site's populations stay zero; the arguments of the loop's
-        // earlier steps lie in the buffer this one will be read from
+        // a rock site's populations stay zero, in both buffers: the arguments
+        // of the loop's earlier steps were laid over one of them
         if (to_pops) {
 #pragma unroll
-          for (int q = 0; q < 19; ++q) {
-            fo[q * S] = rock_dev(q, Lg.rho0);
-            fo[(size_t)(19 + q) * S] = rock_dev(q, Lg.rho0);
+          for (int q = 0; q < 38; ++q) {
+            f0[base + (size_t)q * S + self] = rock_dev(q % 19, Lg.rho0);
+            f1[base + (size_t)q * S + self] = rock_dev(q % 19, Lg.rho0);
           }
         }
         continue;
       }
-      const int as = (tx + 1) + AW * (ty + 1);
+      const int as = (tx + 1) + AW * (ty + 1), o = ((k + 1) % RS) * NT + tid;
       float Fx[NC][3];
       const float2 *Pm = ringP + (k % RS) * AN, *P0 = ringP + ((k + 1) % RS) * AN, *Pp = ringP + ((k + 2) % RS) * AN;
+      float4 pp = own1[o];  // drho_s (ternary), P
+      float2 drb;
+      float3 dd = make_float3(0.f, 0.f, 0.f);
+      if (NC == 3) {
+        const float4 d = own2[o];
+        dd = make_float3(d.x, d.y, d.z);
+        drb = own3[o];
+      } else {
+        drb = make_float2(pp.x, pp.y);
+        pp = make_float4(0.f, pp.z, pp.w, reinterpret_cast<const float *>(own3)[o]);
+      }
       if constexpr (NC == 3)
         force_ternary_pre<AW>(Pm, P0, Pp, ringA + (k % RS) * AN, ringA + ((k + 1) % RS) * AN,
                               ringA + ((k + 2) % RS) * AN, as, dd, Lg, psi0, reinterpret_cast<float(*)[3]>(Fx));
@@ -885,18 +925,14 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
         eq_store2(b, b + 19 * NP, (unsigned)NP, rho2, dr2, vx2, vy2, vz2, one);
       }
       if (to_pops) {
+        float *fo = (par ? f0 : f1) + base + self;
         eq_store2(fo, fo + (size_t)19 * S, S, rho2, dr2, vx2, vy2, vz2, one);
         if (NC == 3)
           eq_store(fo + (size_t)38 * S, S, rho[NC - 1], dr[NC - 1], vx[NC - 1], vy[NC - 1], vz[NC - 1], 1.0f);
       } else {
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          float *o = fo + (size_t)(c * 19) * S;
-          o[0] = dr[c];
-          o[S] = vx[c];
-          o[2 * S] = vy[c];
-          o[3 * S] = vz[c];
-        }
+        Q[self] = make_float4(dr2.x, dr2.y, vx2.x, vx2.y);
+        Q[S + self] = make_float4(vy2.x, vy2.y, vz2.x, vz2.y);
+        if (NC == 3) Q[2 * (size_t)S + self] = make_float4(dr[NC - 1], vx[NC - 1], vy[NC - 1], vz[NC - 1]);
       }
     }
     cp_async_wait<0>();
@@ -933,35 +969,41 @@ using namespace f32;
 // ---------------------------------------------------------------------------
 // launches
 // ---------------------------------------------------------------------------
-// Tile of the moments passes: 32 x 8, or 16 x 16 where that pads the
-// lattice's x and y sides less.
-void eq_moments_tile(int nx, int ny, int *tx, int *ty) {
-  (void)nx;
-  (void)ny;
-  *tx = EQ_TX;
-  *ty = EQ_TY;
+// Tile of the moments passes: 32 x 8, or 16 x 8 where that pads the lattice's
+// x side less.  At equal padding the wider tile is 3 % faster (ternary 128^3,
+// a step: 0.213 against 0.220 ms; binary 256x128x128: 0.162 against 0.164):
+// its halo is 0.33 of the tile's sites, the narrower one's 0.41.
+void eq_moments_tile(int nx, int *tx, int *ty) {
+  *tx = 1.03 * ((nx + 15) / 16 * 16) < (double)((nx + 31) / 32 * 32) ? 16 : 32;
+  *ty = 8;
+}
+
+template <int NC, bool ROCK, bool LE, int TX, int TY>
+static bool eq_moments_fn(int pass, bool first, bool narrow, EqKernel *k) {
+  if (first) {
+    if (pass == EQ_SURFACTANT) return false;
+    k->fn = narrow ? (const void *)k_eq_moments0<NC, TX, TY, ROCK, true, LE>
+                   : (const void *)k_eq_moments0<NC, TX, TY, ROCK, false, LE>;
+    k->threads = TX * TY;
+    k->smem = NC == 3 ? 4 * (TX + 2) * (TY + 2) * 16 : 0;
+  } else if (pass == EQ_MOMENTS) {
+    k->fn = (const void *)k_eq_moments<float2, TX, TY, ROCK, LE>;
+    k->threads = EqGeom<float2, TX, TY, ROCK>::NTH;
+    k->smem = EqGeom<float2, TX, TY, ROCK>::SMEM;
+  } else {
+    k->fn = (const void *)k_eq_moments<float, TX, TY, false, false>;
+    k->threads = EqGeom<float, TX, TY, false>::NTH;
+    k->smem = EqGeom<float, TX, TY, false>::SMEM;
+  }
+  return true;
 }
 
 template <int NC, bool ROCK, bool LE>
 static bool eq_fn(int pass, bool first, int tx, int ty, bool narrow, EqKernel *k) {
   if (pass == EQ_MOMENTS || pass == EQ_SURFACTANT) {
-    if (pass == EQ_SURFACTANT && (NC != 3 || first)) return false;
-    const size_t an = (size_t)(tx + 2) * (ty + 2);
-    if (first) {
-      k->fn = narrow ? (const void *)k_eq_moments0<NC, EQ_TX, EQ_TY, ROCK, true, LE>
-                     : (const void *)k_eq_moments0<NC, EQ_TX, EQ_TY, ROCK, false, LE>;
-      k->threads = tx * ty;
-      k->smem = NC == 3 ? 4 * an * 16 : 0;
-    } else if (pass == EQ_MOMENTS) {
-      k->fn = (const void *)k_eq_moments<float2, EQ_TX, EQ_TY, ROCK, LE>;
-      k->threads = EqGeom<float2, EQ_TX, EQ_TY, ROCK>::NTH;
-      k->smem = EqGeom<float2, EQ_TX, EQ_TY, ROCK>::SMEM;
-    } else {
-      k->fn = (const void *)k_eq_moments<float, EQ_TX, EQ_TY, false, false>;
-      k->threads = EqGeom<float, EQ_TX, EQ_TY, false>::NTH;
-      k->smem = EqGeom<float, EQ_TX, EQ_TY, false>::SMEM;
-    }
-    return true;
+    if (ty != 8 || (tx != 16 && tx != 32) || (pass == EQ_SURFACTANT && NC != 3)) return false;
+    return tx == 32 ? eq_moments_fn<NC, ROCK, LE, 32, 8>(pass, first, narrow, k)
+                    : eq_moments_fn<NC, ROCK, LE, 16, 8>(pass, first, narrow, k);
   }
 #define LB3D_EQ_SHAPE(TX, TY)                                            \
   if (tx == TX && ty == TY) {                                            \
@@ -1004,14 +1046,16 @@ cudaError_t eq_launch(const EqKernel &k, int pass, bool first, bool last, const 
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 1 : 0;
-  int to_pops = last ? 1 : 0;
-  void *src = first ? (void *)&a.rock : (void *)&a.mask;
-  void *p0[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.f0, (void *)&a.f1,
-                (void *)&a.db0, (void *)&a.db1, src, (void *)&a.X};
-  void *p1[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.db0, (void *)&a.db1, (void *)&a.X};
+  int l = last ? 1 : 0;
+  void *p00[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.f0, (void *)&a.f1,
+                 (void *)&a.db0, (void *)&a.db1, (void *)&a.rock, (void *)&a.X};
+  void *p0[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.mask, (void *)&a.X};
+  void *p1[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.db0, (void *)&a.db1, (void *)&a.X,
+                (void *)&l};
   void *p2[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.f0, (void *)&a.f1,
-                (void *)&a.db0, (void *)&a.db1, (void *)&a.mask, (void *)&a.X, (void *)&to_pops};
-  return cudaLaunchKernelExC(&cfg, k.fn, pass == EQ_DIPOLE ? p1 : pass == EQ_COLLIDE ? p2 : p0);
+                (void *)&a.mask, (void *)&a.X, (void *)&l};
+  return cudaLaunchKernelExC(&cfg, k.fn,
+                             pass == EQ_DIPOLE ? p1 : pass == EQ_COLLIDE ? p2 : first ? p00 : p0);
 }
 
 cudaError_t eq_build_mask(int nx, int ny, int nz, bool le, const uint8_t *rock, uint32_t *mask, float2 *psi,

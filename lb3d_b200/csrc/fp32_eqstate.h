@@ -13,11 +13,15 @@ namespace lb3d {
 //   psi  {dpsi_r, dpsi_b}
 //   o1   {drho_r, drho_b, P_x, P_y}, o2: P_z, P of red and blue
 //   o3   ternary: {drho_s, P}, P of all components
+// and between the steps of a loop, for lattices of parity 0 and 1,
+//   Q    float4 [4][S]: {drho_r, drho_b, vx_r, vx_b}, {vy_r, vy_b, vz_r, vz_b},
+//        ternary: {drho_s, v_s}, {d}
 struct EqFields {
   float4 *M;
   float2 *psi;
   float4 *o1, *o3;
   float *o2;
+  float4 *Q[2];
   unsigned S;
 };
 
@@ -41,8 +45,8 @@ struct EqArgs {
 // pass exist for ternary lattices, and a first step (from populations) takes
 // all moments in EQ_MOMENTS.
 enum { EQ_MOMENTS, EQ_SURFACTANT, EQ_DIPOLE, EQ_COLLIDE, EQ_PASSES };
-// Tile of the moments passes for a lattice nx sites by ny across.
-void eq_moments_tile(int nx, int ny, int *tx, int *ty);
+// Tile of the moments passes for a lattice nx sites wide.
+void eq_moments_tile(int nx, int *tx, int *ty);
 // The kernel of a pass for a lattice kind and tile; false if there is none.
 // narrow: 19 nc S < 2^32.
 bool eq_kernel(int pass, bool first, int nc, bool rock, bool le, int tx, int ty, bool narrow, EqKernel *k);

@@ -872,7 +872,7 @@ static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
 static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool first, int tx, int ty, EqKernel *k) {
   const bool rock = (s.lat.flags & LAT_ROCK) != 0;
   int ax = tx, ay = ty;
-  if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.ny, &ax, &ay);
+  if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, &ax, &ay);
   return eq_kernel(pass, first, P.nc, rock, s.le_h[0] != nullptr, ax, ay, 19ull * P.nc * s.S < (1ull << 32), k);
 }
 
@@ -892,7 +892,8 @@ static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rock
   a.f0 = s.f[0], a.f1 = s.f[1], a.db0 = s.db[0], a.db1 = s.db[1];
   a.rock = rockp;
   a.mask = s.mask;
-  a.X = EqFields{s.M, P.nc == 3 ? s.psi : reinterpret_cast<float2 *>(s.M), s.o1, s.o3, s.o2, (unsigned)s.S};
+  a.X = EqFields{s.M, P.nc == 3 ? s.psi : reinterpret_cast<float2 *>(s.M), s.o1, s.o3, s.o2,
+                 {reinterpret_cast<float4 *>(s.f[0]), reinterpret_cast<float4 *>(s.f[1])}, (unsigned)s.S};
   for (int pass = 0; pass < EQ_PASSES; ++pass) {
     EqKernel k;
     if (!eq_kernel_of(P, s, pass, first, s.tx, s.ty, &k)) continue;
@@ -940,7 +941,7 @@ static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
       continue;
     }
     int tx = sh.tx, ty = sh.ty, res = 0;
-    if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.ny, &tx, &ty);
+    if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, &tx, &ty);
     if (fp32_prepare_kernel(kn.fn, kn.threads, kn.smem, &res) != cudaSuccess) return LB3DC_ECUDA;
     const int nxy = ((L.nx + tx - 1) / tx) * ((L.ny + ty - 1) / ty);
     const int k = fp32_z_chunks(L.nz, nxy, res, 2);
