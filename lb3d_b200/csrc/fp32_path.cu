@@ -987,9 +987,15 @@ static void attach_le(Fp32State &s) {
   for (int b = 0; b < 4; ++b) s.lat.le_b[b] = s.le_b[b];
 }
 
-// Shape before any autotuning: the split strategy with the staged collide
-// pass, which measured fastest on 128^3 ternary and 256^3 binary lattices.
+// Shape before any autotuning.  Fully relaxing lattices: strategy 3 with 16x8
+// tiles, the fastest or within 3 % of it on every lattice measured (ternary
+// 32^3, 64^3, 75x67x87, 128^3: 0.029, 0.049, 0.070, 0.213 ms a step against
+// 0.058, 0.082, 0.126, 0.383 for strategy 2; binary 256x128x128 0.161 against
+// 0.418, sheared 0.288 against 0.536, porous 192^3 0.268 against 0.911).
+// Others: the split strategy with the staged collide pass, the fastest of 0 to
+// 2.
 static FusedShape default_shape(const DevParams &P) {
+  if (fp32_eq_eligible(P)) return FusedShape{16, 8, 16, 3};
   FusedShape sh{32, 4, P.nc == 3 ? 8 : 16, 2};
   if (P.nx < 32) sh.tx = 16, sh.ty = 8;
   return sh;
@@ -1174,7 +1180,14 @@ int fp32_alloc(const DevParams &P, const lb3dc_params &p, Fp32State &s, cudaStre
   }
   s.lat = fp32_make_desc(P, p.rho0 > 0 ? p.rho0 : 0.7, 0, false);
   attach_le(s);
-  return rebuild_tiles(P, s, default_shape(P), st);
+  FusedShape sh = default_shape(P);
+  int rc = rebuild_tiles(P, s, sh, st);
+  if (rc == LB3DC_ENOMEM && sh.split == 3) {
+    // no room for strategy 3's fields
+    sh = FusedShape{sh.tx, sh.ty, sh.zc, 2};
+    rc = rebuild_tiles(P, s, sh, st);
+  }
+  return rc;
 }
 
 void fp32_free(Fp32State &s) {
