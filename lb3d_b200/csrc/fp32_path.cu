@@ -472,11 +472,39 @@ __global__ void k_plane_from_fp64(const double *__restrict__ src, float *__restr
   d0[i] = x;
   d1[i] = x;
 }
-__global__ void k_plane_to_fp64(const float *__restrict__ src, double *__restrict__ dst, long long N,
-                                double w) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+// One plane of a download, FP64: a population plane (the deviations of one
+// direction plus w; rock sites hold no populations), a density or momentum
+// plane (summed in FP64 over the populations in direction order, the
+// products and sums rounded separately), or a dipole plane.  A density plane
+// reads 76 B a site, so even the four moment planes of a component take less
+// than the link needs for one of them (128^3: 25 us against 365 us).
+struct PlaneJob {
+  int kind;  // 0: population (src one plane), 1: density, 2..4: momentum x, y, z (src 19 planes), 5: as it is
+  const float *src;
+  double rho0;
+};
+__global__ void k_plane_to_fp64(PlaneJob J, long long S, double *__restrict__ dst, long long N, double w,
+                                const uint8_t *__restrict__ rock) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
-  dst[i] = __dadd_rn((double)src[i], w);
+  const bool solid = rock && rock[i] != 0;
+  if (J.kind == 0) {
+    dst[i] = solid ? 0.0 : __dadd_rn((double)J.src[i], w);
+    return;
+  }
+  if (J.kind == 5) {
+    dst[i] = (double)J.src[i];
+    return;
+  }
+  double m = 0.0;
+#pragma unroll
+  for (int q = 0; q < 19; ++q) {
+    const int c = J.kind == 1 ? 1 : J.kind == 2 ? cx(q) : J.kind == 3 ? cy(q) : cz(q);
+    const double wr = __dmul_rn(q == 18 ? 1.0 / 3.0 : 1.0 / 36.0, J.rho0);
+    const double n = solid ? 0.0 : __dadd_rn((double)J.src[(long long)q * S + i], wr);
+    m = __dadd_rn(m, __dmul_rn(__dmul_rn(n, (double)gw(q)), (double)c));
+  }
+  dst[i] = m;
 }
 
 }  // namespace f32
@@ -1292,79 +1320,39 @@ int fp32_download(const DevParams &P, const lb3dc_params &p, Fp32State &s, doubl
   const int nc = P.nc;
   const int cur = s.lat.parity;
   const double rho0 = s.lat.rho0;
-  std::vector<double> tmp;
-  double *nn = n;
-  if (!nn && (rho || mom)) {
-    tmp.resize((size_t)nc * 19 * N);
-    nn = tmp.data();
+  // one FP64 plane at a time through two staging planes: the conversion of a
+  // plane (and the sums of the density and momentum planes) overlaps the copy
+  // of the one before (copy stream); xev[b] marks staging plane b filled,
+  // xev[2 + b] drained
+  const uint8_t *rk = rockp && (s.lat.flags & LAT_ROCK) ? rockp : nullptr;
+  cudaError_t e = cudaEventRecord(s.xev[2], s.xs);
+  if (e == cudaSuccess) e = cudaEventRecord(s.xev[3], s.xs);
+  int planes = 0;
+  auto plane = [&](int kind, const float *src, double w, double *dst) {
+    if (e != cudaSuccess) return;
+    const int b = planes++ & 1;
+    double *stg = s.stage + (size_t)b * N;
+    e = cudaStreamWaitEvent(st, s.xev[2 + b], 0);
+    if (e != cudaSuccess) return;
+    k_plane_to_fp64<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(PlaneJob{kind, src, rho0}, s.S, stg, N, w, rk);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(s.xev[b], st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s.xs, s.xev[b], 0);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(dst, stg, (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, s.xs);
+    if (e == cudaSuccess) e = cudaEventRecord(s.xev[2 + b], s.xs);
+  };
+  for (int c = 0; c < nc; ++c) {
+    const float *f = s.f[cur] + (size_t)c * 19 * s.S;
+    for (int q = 0; n && q < 19; ++q)
+      plane(0, f + (size_t)q * s.S, (q == 18 ? 1.0 / 3.0 : 1.0 / 36.0) * rho0, n + ((size_t)c * 19 + q) * N);
+    if (rho) plane(1, f, 0.0, rho + (size_t)c * N);
+    for (int k = 0; mom && k < 3; ++k) plane(2 + k, f, 0.0, mom + ((size_t)c * 3 + k) * N);
   }
-  if (nn) {
-    // deviations -> FP64 populations, one plane at a time through two
-    // staging planes: the conversion of plane cq + 1 overlaps the copy of
-    // plane cq (copy stream); xev[b] marks staging plane b filled, xev[2 + b]
-    // drained
-    cudaError_t e = cudaEventRecord(s.xev[2], s.xs);
-    if (e == cudaSuccess) e = cudaEventRecord(s.xev[3], s.xs);
-    for (int cq = 0; cq < nc * 19 && e == cudaSuccess; ++cq) {
-      const int b = cq & 1;
-      double *stg = s.stage + (size_t)b * N;
-      const double w = (cq % 19 == 18 ? 1.0 / 3.0 : 1.0 / 36.0) * rho0;
-      e = cudaStreamWaitEvent(st, s.xev[2 + b], 0);
-      if (e != cudaSuccess) break;
-      k_plane_to_fp64<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(s.f[cur] + (size_t)cq * s.S,
-                                                                    stg, N, w);
-      e = cudaGetLastError();
-      if (e == cudaSuccess) e = cudaEventRecord(s.xev[b], st);
-      if (e == cudaSuccess) e = cudaStreamWaitEvent(s.xs, s.xev[b], 0);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(nn + (size_t)cq * N, stg, (size_t)N * sizeof(double),
-                            cudaMemcpyDeviceToHost, s.xs);
-      if (e == cudaSuccess) e = cudaEventRecord(s.xev[2 + b], s.xs);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s.xs);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return LB3DC_ECUDA;
-  }
-  std::vector<uint8_t> rk(N, 0);
-  if (rockp && (s.lat.flags & LAT_ROCK)) {
-    if (cudaMemcpyAsync(rk.data(), rockp, N, cudaMemcpyDeviceToHost, st) != cudaSuccess) return LB3DC_ECUDA;
-    cudaStreamSynchronize(st);
-    // rock sites hold no populations (code/lb3d_ic_rock.F90:163-170)
-    if (nn)
-      for (long long i = 0; i < N; ++i)
-        if (rk[i])
-          for (int cq = 0; cq < nc * 19; ++cq) nn[(size_t)cq * N + i] = 0.0;
-  }
-  if (rho || mom) {
-    for (int c = 0; c < nc; ++c)
-      for (long long i = 0; i < N; ++i) {
-        double r = 0, m0 = 0, m1 = 0, m2 = 0;
-        for (int q = 0; q < 19; ++q) {
-          const double ng = nn[((size_t)c * 19 + q) * N + i] * gw(q);
-          r += ng;
-          m0 += ng * cx(q);
-          m1 += ng * cy(q);
-          m2 += ng * cz(q);
-        }
-        if (rho) rho[(size_t)c * N + i] = r;
-        if (mom) {
-          mom[((size_t)c * 3 + 0) * N + i] = m0;
-          mom[((size_t)c * 3 + 1) * N + i] = m1;
-          mom[((size_t)c * 3 + 2) * N + i] = m2;
-        }
-      }
-  }
-  if (db) {
-    if (nc == 3) {
-      std::vector<float> d(3 * N);
-      if (cudaMemcpyAsync(d.data(), s.db[cur], d.size() * 4, cudaMemcpyDeviceToHost, st) != cudaSuccess)
-        return LB3DC_ECUDA;
-      cudaStreamSynchronize(st);
-      for (long long i = 0; i < 3 * N; ++i) db[i] = d[i];
-    } else {
-      std::memset(db, 0, 3 * N * sizeof(double));
-    }
-  }
+  for (int k = 0; db && nc == 3 && k < 3; ++k) plane(5, s.db[cur] + (size_t)k * s.S, 0.0, db + (size_t)k * N);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s.xs);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return LB3DC_ECUDA;
+  if (db && nc != 3) std::memset(db, 0, 3 * N * sizeof(double));
   if (da) std::memset(da, 0, 3 * N * sizeof(double));
   (void)p;
   return LB3DC_OK;
@@ -1425,14 +1413,7 @@ int fp32_dump(const DevParams &P, Fp32State &s, int field, const uint8_t *rock, 
   k_to_fp64<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(s.f[cur], n, s.S, 0, N, nc, s.lat.rho0);
   cudaError_t e = cudaGetLastError();
   if (e == cudaSuccess) e = fp64_moments(P, n, rho, psi, mom, st);
-  if (e == cudaSuccess && nc == 3) {
-    std::vector<float> h(3 * N);
-    std::vector<double> hd(3 * N);
-    e = cudaMemcpyAsync(h.data(), s.db[cur], 3 * N * 4, cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    for (long long i = 0; i < 3 * N; ++i) hd[i] = h[i];
-    if (e == cudaSuccess) e = cudaMemcpyAsync(db, hd.data(), 3 * N * 8, cudaMemcpyHostToDevice, st);
-  }
+  if (e == cudaSuccess && nc == 3) e = fp32_planes_to_fp64(s.db[cur], db, s.S, 0, N, 3, st);
   if (e == cudaSuccess) e = fp64_dump(P, field, n, rho, psi, db, rock, out, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(n);
