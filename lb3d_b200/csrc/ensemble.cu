@@ -19,6 +19,7 @@
 #include <vector>
 
 #include "../../include/lb3dc.h"
+#include "fp32_eqstate.h"
 #include "fp32_path.h"
 #include "params.h"
 
@@ -51,6 +52,9 @@ struct lb3dc_ensemble {
   std::map<long long, long long> free_ranges;  // base -> length
   FusedShape shape{32, 4, 8, 2};  // fastest measured on the parameter-sweep stream
   float4 *M = nullptr, *J = nullptr;
+  EqFields X{};     // strategy 3's fields (null pointers: no room for them)
+  bool eq = false;  // the active members run strategy 3
+  unsigned char *eq_block = nullptr;
   double *stage = nullptr;  // FP64 staging of one member's populations (admit / retire)
   size_t stage_bytes = 0;
   cudaStream_t copy_stream = nullptr;  // asynchronous retires
@@ -93,6 +97,13 @@ void drop_graph(lb3dc_ensemble *e) {
   e->graph_steps = 0;
 }
 
+void free_eq(lb3dc_ensemble *e) {
+  if (e->eq_block) cudaFree(e->eq_block);
+  e->eq_block = nullptr;
+  e->X = EqFields{};
+  cudaGetLastError();
+}
+
 bool take_range(lb3dc_ensemble *e, long long n, long long *base) {
   for (auto it = e->free_ranges.begin(); it != e->free_ranges.end(); ++it) {
     if (it->second >= n) {
@@ -123,13 +134,52 @@ void give_range(lb3dc_ensemble *e, long long base, long long n) {
   }
 }
 
+// Strategy 3 (fp32_eqstate.cu) advances the active members when all of them
+// relax fully; their tiles serve every pass.
+constexpr int EQ_TX = 16, EQ_TY = 8;
+
+bool runs_eq(const lb3dc_ensemble *e) {
+  if (!e->X.o1 || e->shape.split != 2) return false;
+  for (const Member &m : e->members)
+    if (m.used && m.remaining > 0 && !fp32_eq_eligible(dev_params_from(m.p))) return false;
+  return true;
+}
+
+// z chunk of strategy 3's tiles: the active columns' planes over two rounds of
+// the collide pass's resident CTAs, at least 8 planes (each chunk works on two
+// more) and at most 32.
+int eq_zc(const lb3dc_ensemble *e, int resident) {
+  long long planes = 0;
+  for (const Member &m : e->members)
+    if (m.used && m.remaining > 0)
+      planes += (long long)((m.desc.nx + EQ_TX - 1) / EQ_TX) * ((m.desc.ny + EQ_TY - 1) / EQ_TY) * m.desc.nz;
+  return (int)std::min(32LL, std::max(8LL, planes / (2LL * std::max(1, resident))));
+}
+
+bool eq_kernel_of(const lb3dc_ensemble *e, int pass, bool first, EqKernel *k) {
+  return eq_kernel(pass, first, e->nc, false, false, EQ_TX, EQ_TY, 19ull * e->nc * e->S < (1ull << 32), k);
+}
+
 int rebuild(lb3dc_ensemble *e) {
   std::vector<Tile> tiles;
   e->body = false;
+  e->eq = runs_eq(e);
+  FusedShape sh = e->shape;
+  if (e->eq) {
+    int res = 0;
+    for (int pass = 0; pass < EQ_PASSES; ++pass)
+      for (int first = 0; first < 2; ++first) {
+        EqKernel k;
+        if (eq_kernel_of(e, pass, first != 0, &k) &&
+            fp32_prepare_kernel(k.fn, k.threads, k.smem, &res) != cudaSuccess)
+          return efail(e, LB3DC_ECUDA, "kernel set-up failed");
+      }
+    sh = FusedShape{EQ_TX, EQ_TY, eq_zc(e, res), 3};
+  }
   for (int i = 0; i < (int)e->members.size(); ++i) {
     Member &m = e->members[i];
     if (!m.used || m.remaining <= 0) continue;
-    fp32_tiles_for(m.desc, i, e->shape, tiles);
+    fp32_tiles_for(m.desc, i, sh, tiles);
     if (m.desc.flags & LAT_BODY) e->body = true;
   }
   if ((int)tiles.size() > e->tile_cap) {
@@ -152,13 +202,30 @@ int rebuild(lb3dc_ensemble *e) {
   return LB3DC_OK;
 }
 
-// One step of every active lattice: the fused kernel, then the parity flip.
-cudaError_t launch_step(lb3dc_ensemble *e) {
-  cudaError_t r = fp32_launch_fused(e->nc, false, e->body, e->shape, e->d_lat, e->d_tiles, e->ntiles,
-                                    0, e->f[0], e->f[1], e->db[0], e->db[1], e->rock, e->S,
-                                    e->stream, e->M, e->J);
-  if (r != cudaSuccess) return r;
-  return fp32_flip_parity(e->d_lat, e->max_lat, e->stream);
+// One step of every active lattice: the passes, then the parity flip
+// (strategy 3: after the last of the steps enqueued together).
+cudaError_t launch_step(lb3dc_ensemble *e, bool first, bool last) {
+  if (!e->eq) {
+    cudaError_t r = fp32_launch_fused(e->nc, false, e->body, e->shape, e->d_lat, e->d_tiles, e->ntiles,
+                                      0, e->f[0], e->f[1], e->db[0], e->db[1], e->rock, e->S,
+                                      e->stream, e->M, e->J);
+    if (r != cudaSuccess) return r;
+    return fp32_flip_parity(e->d_lat, e->max_lat, e->stream);
+  }
+  EqArgs a{};
+  a.lats = e->d_lat;
+  a.tiles = e->d_tiles;
+  a.ntiles = e->ntiles;
+  a.f0 = e->f[0], a.f1 = e->f[1], a.db0 = e->db[0], a.db1 = e->db[1];
+  a.rock = e->rock;
+  a.X = e->X;
+  for (int pass = 0; pass < EQ_PASSES; ++pass) {
+    EqKernel k;
+    if (!eq_kernel_of(e, pass, first, &k)) continue;
+    const cudaError_t r = eq_launch(k, pass, first, last, a, true, e->stream);
+    if (r != cudaSuccess) return r;
+  }
+  return last ? fp32_flip_parity(e->d_lat, e->max_lat, e->stream) : cudaSuccess;
 }
 
 // Seeded initial state on the device, the generator of lb3d_b200/ic.py:
@@ -294,6 +361,30 @@ int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
   e->bytes = 2 * (long long)pop + (ncomp == 3 ? 24LL * capacity_sites : 0) + capacity_sites +
              capacity_sites * fp32_moment_bytes(ncomp) +
              (long long)max_lattices * sizeof(LatDesc);
+  // strategy 3's fields: without room for them fully relaxing members run
+  // strategy 2 like the others
+  {
+    const size_t n = (size_t)capacity_sites;
+    EqFields &X = e->X;
+    X.S = (unsigned)capacity_sites;
+    X.M = e->M;
+    // one block: Q, o1, o3 (float4), psi (ternary; a binary lattice's M holds
+    // psi), o2
+    const size_t b = ncomp == 3 ? 108 : 52;
+    const bool room = cudaMalloc(&e->eq_block, n * b) == cudaSuccess;
+    if (room) {
+      X.Q[0] = reinterpret_cast<float4 *>(e->eq_block);
+      X.o1 = X.Q[0] + (ncomp == 3 ? 4 : 2) * n;
+      X.o3 = ncomp == 3 ? X.o1 + n : nullptr;
+      X.psi = ncomp == 3 ? reinterpret_cast<float2 *>(X.o3 + n) : reinterpret_cast<float2 *>(e->M);
+      X.o2 = ncomp == 3 ? reinterpret_cast<float *>(X.psi + n) : reinterpret_cast<float *>(X.o1 + n);
+    }
+    X.Q[1] = X.Q[0];
+    if (room)
+      e->bytes += (long long)(n * b);
+    else
+      free_eq(e);
+  }
   e->members.resize(max_lattices);
   e->free_ranges[0] = capacity_sites;
   cudaStreamSynchronize(e->stream);
@@ -311,6 +402,7 @@ int lb3dc_ensemble_destroy(lb3dc_ensemble *e) {
     if (e->db[b]) cudaFree(e->db[b]);
   }
   if (e->rock) cudaFree(e->rock);
+  free_eq(e);
   if (e->M) cudaFree(e->M);
   if (e->J) cudaFree(e->J);
   if (e->d_lat) cudaFree(e->d_lat);
@@ -418,7 +510,7 @@ int lb3dc_ensemble_step(lb3dc_ensemble *e, int max_steps, int *steps_done) {
       drop_graph(e);
       cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeRelaxed);
       cudaError_t r = cudaSuccess;
-      for (int s = 0; s < chunk && r == cudaSuccess; ++s) r = launch_step(e);
+      for (int s = 0; s < chunk && r == cudaSuccess; ++s) r = launch_step(e, s == 0, s == chunk - 1);
       cudaStreamEndCapture(e->stream, &e->graph);
       if (r != cudaSuccess || !e->graph) return efail(e, LB3DC_ECUDA, "graph capture failed");
       if (cudaGraphInstantiate(&e->gexec, e->graph, 0) != cudaSuccess)
@@ -428,7 +520,7 @@ int lb3dc_ensemble_step(lb3dc_ensemble *e, int max_steps, int *steps_done) {
     if (cudaGraphLaunch(e->gexec, e->stream) != cudaSuccess) return efail(e, LB3DC_ECUDA, "graph launch failed");
   } else {
     for (int s = 0; s < chunk; ++s)
-      if (launch_step(e) != cudaSuccess) return efail(e, LB3DC_ECUDA, "launch failed");
+      if (launch_step(e, s == 0, s == chunk - 1) != cudaSuccess) return efail(e, LB3DC_ECUDA, "launch failed");
   }
   long long active_sites = 0;
   for (auto &m : e->members) {
@@ -436,7 +528,7 @@ int lb3dc_ensemble_step(lb3dc_ensemble *e, int max_steps, int *steps_done) {
     active_sites += m.n;
     m.remaining -= chunk;
     m.done_steps += chunk;
-    m.desc.parity ^= (chunk & 1);
+    m.desc.parity ^= e->eq ? 1 : (chunk & 1);
     if (m.remaining == 0) {
       m.finished = true;
       e->dirty = true;
@@ -529,13 +621,24 @@ int lb3dc_ensemble_retire_async(lb3dc_ensemble *e, int slot, double *n, double *
   const int cur = m.desc.parity;
   const size_t nb = (size_t)e->nc * 19 * N * sizeof(double), dbb = 3 * (size_t)N * sizeof(double);
   if (e->cstage_bytes < nb + dbb) {
-    // the staging is reused in stream order; grow it only when no copy is in flight
+    // the staging is reused in stream order; grow it only when no copy is in
+    // flight, and at once for the largest resident member (freeing it waits
+    // for the device)
+    long long largest = N;
+    for (const Member &o : e->members)
+      if (o.used) largest = std::max(largest, o.n);
+    const size_t most = ((size_t)e->nc * 19 + 3) * largest * sizeof(double);
     cudaStreamSynchronize(e->copy_stream);
     if (e->cstage) cudaFree(e->cstage);
     e->cstage = nullptr;
     e->cstage_bytes = 0;
-    if (cudaMalloc(&e->cstage, nb + dbb) != cudaSuccess) return efail(e, LB3DC_ENOMEM, "staging allocation failed");
-    e->cstage_bytes = nb + dbb;
+    size_t got = most;
+    if (cudaMalloc(&e->cstage, got) != cudaSuccess) {
+      cudaGetLastError();
+      got = nb + dbb;
+      if (cudaMalloc(&e->cstage, got) != cudaSuccess) return efail(e, LB3DC_ENOMEM, "staging allocation failed");
+    }
+    e->cstage_bytes = got;
   }
   // the member's last step is queued on the main stream before this point;
   // later steps do not touch it (it is no longer active)
