@@ -332,6 +332,23 @@ __global__ void k_recolour(DevParams P, double *__restrict__ g, const uint8_t *_
   }
 }
 
+// c . v of a lattice direction, the products and sums in axis order.  Terms of
+// a zero component are left out here and in the sums over directions below:
+// adding +-0 changes no finite value (the FP64 pipe bounds these kernels, and
+// the compiler may not drop a product with 0 by itself).
+__device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
+  double r = 0.0;
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < 3; ++k)
+    if (c[k]) {
+      const double t = v[k] * (double)c[k];
+      r = any ? r + t : t;
+      any = true;
+    }
+  return r;
+}
+
 // ---------------------------------------------------------------------------
 // Dipole relaxation, code/lb3d_collision.F90:296-403 (ternary, periodic).
 // Reads rho and da of the 18 neighbours; writes db in place (no neighbour
@@ -359,10 +376,12 @@ __global__ void __launch_bounds__(256) k_dipole(DevParams P, const double *__res
     double psi_b = 0.0 + rho[N + j];
     double pas[3] = {da[j], da[N + j], da[2 * N + j]};
     double hc_m = -(sgn * (psi_b - psi_r) * (double)gw(q));
-    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)};
-    for (int k = 0; k < 3; ++k) h_c[k] = h_c[k] + hc_m * c[k];
-    double hs_dot = 2.0 * ((c[0] * pas[0] + c[1] * pas[1]) + c[2] * pas[2]);
-    for (int k = 0; k < 3; ++k) h_s[k] = h_s[k] + (pas[k] - c[k] * hs_dot) * (double)gw(q);
+    const int c[3] = {cx(q), cy(q), cz(q)};
+    for (int k = 0; k < 3; ++k)
+      if (c[k]) h_c[k] = h_c[k] + hc_m * (double)c[k];
+    double hs_dot = 2.0 * cdot(c, pas);
+    for (int k = 0; k < 3; ++k)
+      h_s[k] = h_s[k] + (c[k] ? pas[k] - (double)c[k] * hs_dot : pas[k]) * (double)gw(q);
   }
   double h[3];
   for (int k = 0; k < 3; ++k) h[k] = h_c[k] + h_s[k];
@@ -399,7 +418,7 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
   double f_br[3] = {0, 0, 0}, f_rb[3] = {0, 0, 0}, f_wr[3] = {0, 0, 0}, f_wb[3] = {0, 0, 0};
 #pragma unroll
   for (int q = 0; q < 18; ++q) {
-    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)};
+    const int c[3] = {cx(q), cy(q), cz(q)};
     int xn = x + cx(q), yn = y + cy(q), zn = z + cz(q);
     double psi_r, psi_b;
     bool rk = false;
@@ -431,13 +450,15 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
     double green_b = psi_r * (double)gw(q);
     if (rk) {
       for (int k = 0; k < 3; ++k) {
-        f_wb[k] = f_wb[k] + green_r * c[k];
-        f_wr[k] = f_wr[k] + green_b * c[k];
+        if (c[k] == 0) continue;
+        f_wb[k] = f_wb[k] + green_r * (double)c[k];
+        f_wr[k] = f_wr[k] + green_b * (double)c[k];
       }
     } else {
       for (int k = 0; k < 3; ++k) {
-        f_rb[k] = f_rb[k] + green_r * c[k];
-        f_br[k] = f_br[k] + green_b * c[k];
+        if (c[k] == 0) continue;
+        f_rb[k] = f_rb[k] + green_r * (double)c[k];
+        f_br[k] = f_br[k] + green_b * (double)c[k];
       }
     }
   }
@@ -464,29 +485,33 @@ __device__ __forceinline__ void sc_force_ternary(const DevParams &P, int x, int 
 #pragma unroll
   for (int q = 0; q < 18; ++q) {
     long long j = sidx(wrap(x + cx(q), nx), wrap(y + cy(q), ny), wrap(z + cz(q), nz), nx, ny);
-    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)};
+    const int c[3] = {cx(q), cy(q), cz(q)};
     const double g = (double)gw(q);
     double psi_r = psi[j];
     double psi_b = psi[N + j];
     double green_r = psi_b * g;
     double green_b = psi_r * g;
     for (int k = 0; k < 3; ++k) {
-      f_rb[k] = f_rb[k] + green_r * c[k];
-      f_br[k] = f_br[k] + green_b * c[k];
+      if (c[k] == 0) continue;
+      f_rb[k] = f_rb[k] + green_r * (double)c[k];
+      f_br[k] = f_br[k] + green_b * (double)c[k];
     }
     double pss = psi[2 * N + j];
     double dd[3] = {db[j] * pss, db[N + j] * pss, db[2 * N + j] * pss};
-    double d_dotc = (dd[0] * c[0] + dd[1] * c[1]) + dd[2] * c[2];
-    for (int k = 0; k < 3; ++k) f_cs[k] = f_cs[k] + (dd[k] - (2.0 * d_dotc) * c[k]) * g;
-    double di_dotc = (dbx[0] * c[0] + dbx[1] * c[1]) + dbx[2] * c[2];
+    double d_dotc = cdot(c, dd);
+    for (int k = 0; k < 3; ++k)
+      f_cs[k] = f_cs[k] + (c[k] ? dd[k] - (2.0 * d_dotc) * (double)c[k] : dd[k]) * g;
+    double di_dotc = cdot(c, dbx);
     double greenc_s = (psi_b - psi_r) * g;
-    for (int k = 0; k < 3; ++k) f_sc[k] = f_sc[k] + greenc_s * (dbx[k] - (2.0 * di_dotc) * c[k]);
+    for (int k = 0; k < 3; ++k)
+      f_sc[k] = f_sc[k] + greenc_s * (c[k] ? dbx[k] - (2.0 * di_dotc) * (double)c[k] : dbx[k]);
     double di_dot_d = (dd[0] * dbx[0] + dd[1] * dbx[1]) + dd[2] * dbx[2];
     double green_ss = 8.0 * g;
-    for (int k = 0; k < 3; ++k)
-      f_ss[k] = f_ss[k] +
-                green_ss * (((di_dot_d - (2.0 * di_dotc) * d_dotc) * c[k] + dd[k] * di_dotc) +
-                            d_dotc * dbx[k]);
+    const double along = di_dot_d - (2.0 * di_dotc) * d_dotc;
+    for (int k = 0; k < 3; ++k) {
+      const double t = dd[k] * di_dotc;
+      f_ss[k] = f_ss[k] + green_ss * ((c[k] ? along * (double)c[k] + t : t) + d_dotc * dbx[k]);
+    }
   }
   double pb = psi[N + i], prr = psi[i], ps = psi[2 * N + i];
   for (int k = 0; k < 3; ++k) {
