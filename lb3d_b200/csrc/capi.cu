@@ -28,6 +28,7 @@ struct lb3dc_handle {
   // FP64 path
   double *f = nullptr, *g = nullptr, *rho = nullptr, *psi = nullptr, *mom = nullptr;
   double *da = nullptr, *db = nullptr;
+  double *post = nullptr;  // Lees-Edwards: post-stream boundary planes
   double *hlo = nullptr, *hhi = nullptr, *rlo = nullptr, *rhi = nullptr, *plo = nullptr,
          *phi = nullptr;
   // FP32 deviation path
@@ -223,7 +224,7 @@ long long footprint_bytes(const lb3dc_params &p) {
     b += 2 * nc * N * 8 + nc * 3 * N * 8;  // rho, psi, mom
     if (nc == 3) b += 6 * N * 8;        // da, db
     bool le = p.boundary_cond != 0 && (p.inv_fluid == 5 || p.inv_fluid == 6);
-    if (le) b += 2 * nc * 19 * np * 8 + 4 * nc * np * 8;
+    if (le) b += 4 * nc * 19 * np * 8 + 4 * nc * np * 8;
   } else {
     b += fp32_footprint(p);
   }
@@ -259,11 +260,10 @@ int need_loaded(lb3dc_handle *h) {
   return LB3DC_OK;
 }
 
-// The FP64 time loop streams inside the collision (fp64_step_pull) unless
-// something runs between the two: the Lees-Edwards stage-8 halo or an
-// invasion boundary on the post-stream populations.
+// The FP64 time loop streams inside the collision (fp64_step_pull) unless an
+// invasion boundary acts on the post-stream populations between the two.
 bool fp64_pull_ok(const lb3dc_handle *h) {
-  if (h->p.precision != LB3DC_FP64 || h->le || h->P.zouhe) return false;
+  if (h->p.precision != LB3DC_FP64 || h->P.zouhe) return false;
   const int k = h->p.inv_fluid;
   return !(h->p.boundary_cond != 0 && (k == 11 || k == 7 || k == 8));
 }
@@ -333,6 +333,7 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
     if (h->le) {
       rc = rc ? rc : dalloc(h, &h->hlo, nc * 19 * np);
       rc = rc ? rc : dalloc(h, &h->hhi, nc * 19 * np);
+      rc = rc ? rc : dalloc(h, &h->post, 2 * nc * 19 * np);
       rc = rc ? rc : dalloc(h, &h->rlo, nc * np);
       rc = rc ? rc : dalloc(h, &h->rhi, nc * np);
       rc = rc ? rc : dalloc(h, &h->plo, nc * np);
@@ -365,7 +366,7 @@ int lb3dc_destroy(lb3dc_handle *h) {
   if (h->io_pin) cudaFreeHost(h->io_pin);
   if (h->stream) cudaStreamSynchronize(h->stream);
   double *bufs[] = {h->f, h->g, h->rho, h->psi, h->mom, h->da, h->db, h->hlo, h->hhi,
-                    h->rlo, h->rhi, h->plo, h->phi, h->scratch};
+                    h->rlo, h->rhi, h->plo, h->phi, h->post, h->scratch};
   for (double *b : bufs)
     if (b) cudaFree(b);
   if (h->rock) cudaFree(h->rock);
@@ -536,7 +537,7 @@ int lb3dc_bc_apply(lb3dc_handle *h, int stage) {
       h->shear_u = h->shear_tmp * std::cos(h->p.shear_omega * (double)h->nt);
       le_neighbours(h);
       if (h->p.precision == LB3DC_FP64) {
-        CK(h, fp64_le_halo(h->P, le_step(h), h->f, h->hlo, h->hhi, nullptr, nullptr, nullptr,
+        CK(h, fp64_le_halo(h->P, le_step(h), h->f, false, h->hlo, h->hhi, nullptr, nullptr, nullptr,
                            nullptr, h->stream));
         h->timer.launches += 1;
       }
@@ -560,7 +561,7 @@ int lb3dc_bc_apply(lb3dc_handle *h, int stage) {
       h->timer.launches += 1;
     }
     if (h->le && h->p.precision == LB3DC_FP64) {
-      CK(h, fp64_le_halo(h->P, le_step(h), h->g, nullptr, nullptr, h->rlo, h->rhi, h->plo,
+      CK(h, fp64_le_halo(h->P, le_step(h), h->g, false, nullptr, nullptr, h->rlo, h->rhi, h->plo,
                          h->phi, h->stream));
       h->timer.launches += 1;
     }
@@ -578,7 +579,7 @@ int lb3dc_advection(lb3dc_handle *h) {
     CK(h, fp64_stream(h->P, h->f, h->g, h->rho, h->psi, h->mom, h->da, h->db, h->rock, h->hlo,
                       h->hhi, h->stream));
     h->timer.stop(h->stream);
-    h->timer.launches += h->P.nc;
+    h->timer.launches += fp64_stream_launches(h->P);
   } else {
     // The FP32 path streams inside its fused stream-collide kernel.
     h->pending_advection = true;
@@ -628,16 +629,22 @@ int lb3dc_time_loop(lb3dc_handle *h, int nsteps) {
     return LB3DC_OK;
   }
   if (fp64_pull_ok(h)) {
-    // stages 6 and 8 have nothing to do here; each step is the moments
-    // pass, the dipole relaxation and the pulling collision, f -> g, after
-    // which f and g trade places
+    // each step is the moments pass, the dipole relaxation and the pulling
+    // collision, f -> g, after which f and g trade places; stages 6 and 8 have
+    // work under Lees-Edwards only
     for (int s = 0; s < nsteps; ++s) {
-      h->nt += 1;
+      Fp64Le le;
+      if (h->le) {
+        if ((rc = lb3dc_bc_apply(h, 6))) return rc;
+        le = Fp64Le{le_step(h), h->hlo, h->hhi, h->post, h->rlo, h->rhi, h->plo, h->phi};
+      } else {
+        h->nt += 1;
+      }
       h->timer.start(h->stream);
       CK(h, fp64_step_pull(h->P, h->f, h->g, h->rho, h->psi, h->mom, h->da, h->db, h->rock,
-                           h->stream));
+                           h->stream, h->le ? &le : nullptr));
       h->timer.stop(h->stream);
-      h->timer.launches += h->P.nc + (h->p.ncomp == 3 ? 1 : 0) + 1;
+      h->timer.launches += fp64_stream_launches(h->P) + (h->p.ncomp == 3 ? 1 : 0) + (h->le ? 1 : 0) + 1;
       std::swap(h->f, h->g);
     }
     return LB3DC_OK;

@@ -41,58 +41,65 @@ __device__ __forceinline__ void site_xyz(long long i, int nx, int ny, int &x, in
   y = (int)(t - (long long)z * ny);
 }
 
-// src: populations [NC][19][nsites].  Writes the halo planes and, when
-// rho_out is given, their densities and psi (for the force stencil).
-template <int NC>
-__global__ void k_le_halo(DevParams P, LEStep S, const double *__restrict__ src,
+// src: populations [NC][19][nsites], or (COMPACT) the boundary planes
+// [2][NC][19][nz][ny] of x = nx - 1 and x = 0.  Writes the halo planes and,
+// when rlo is given, their densities and psi (for the force stencil).  Threads
+// [0, ny nz) build the bottom halo sites, the next ny nz the top ones, whose
+// clipping rule reads the adjusted bottom site: a top thread builds it only
+// when the rule applies.  A few thousand threads with a long FP64 chain each:
+// one side a thread in 64-thread blocks 16-17 us, both sides a thread in
+// 128-thread blocks 20 and 24 us (97x66x63 sites).
+template <int NC, bool COMPACT>
+__global__ void __launch_bounds__(64) k_le_halo(DevParams P, LEStep S, const double *__restrict__ src,
                           double *__restrict__ hlo, double *__restrict__ hhi,
                           double *__restrict__ rlo, double *__restrict__ rhi,
                           double *__restrict__ plo, double *__restrict__ phi) {
-  const int nx = P.nx, ny = P.ny, nz = P.nz;
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ny * nz) return;
+  const int nx = P.nx, ny = P.ny, nz = P.nz, NPi = ny * nz;
+  const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  if (u >= 2 * NPi) return;
+  const bool top = u >= NPi;
+  const int t = top ? u - NPi : u;
   const int y = t % ny, z = t / ny;
-  const long long N = P.nsites;
+  const long long N = P.nsites, NP = NPi;
   const double f = S.lefrac;
-  double hb[NC][19], ht[NC][19];
-  {
-    long long ia = sidx(nx - 1, y, ((z + S.eoff) % nz + nz) % nz, nx, ny);
-    long long ib = sidx(nx - 1, y, ((z + S.eoff + 1) % nz + nz) % nz, nx, ny);
+  auto at = [&](int c, int q, bool low, int zz) {
+    const int zw = (zz % nz + nz) % nz;
+    if (COMPACT) return src[((low ? 0 : NC * 19) + c * 19 + q) * NP + y + ny * zw];
+    return src[(c * 19 + q) * N + sidx(low ? nx - 1 : 0, y, zw, nx, ny)];
+  };
+  double hb[NC][19];
+  auto bottom = [&]() {
     for (int c = 0; c < NC; ++c)
       for (int q = 0; q < 19; ++q)
-        hb[c][q] = (1.0 - f) * src[(c * 19 + q) * N + ia] + f * src[(c * 19 + q) * N + ib];
+        hb[c][q] = (1.0 - f) * at(c, q, true, z + S.eoff) + f * at(c, q, true, z + S.eoff + 1);
     le_adjust<NC>(P, hb, hb, S.shear_u, -1.0);
-  }
-  {
-    long long ia = sidx(0, y, ((z - S.eoff - 1) % nz + nz) % nz, nx, ny);
-    long long ib = sidx(0, y, ((z - S.eoff) % nz + nz) % nz, nx, ny);
-    for (int c = 0; c < NC; ++c)
-      for (int q = 0; q < 19; ++q)
-        ht[c][q] = f * src[(c * 19 + q) * N + ia] + (1.0 - f) * src[(c * 19 + q) * N + ib];
-    le_adjust<NC>(P, ht, hb, S.shear_u, +1.0);
-  }
-  const long long NP = (long long)ny * nz;
-  if (hlo) {
-    for (int c = 0; c < NC; ++c)
-      for (int q = 0; q < 19; ++q) {
-        hlo[(c * 19 + q) * NP + t] = hb[c][q];
-        hhi[(c * 19 + q) * NP + t] = ht[c][q];
-      }
-  }
-  if (rlo) {
-    for (int c = 0; c < NC; ++c) {
-      double a = 0.0, b = 0.0;
+  };
+  auto put = [&](const double h[NC][19], double *hp, double *rp, double *pp) {
+    if (hp)
+      for (int c = 0; c < NC; ++c)
+        for (int q = 0; q < 19; ++q) hp[(c * 19 + q) * NP + t] = h[c][q];
+    if (rp)
+      for (int c = 0; c < NC; ++c) {
+        double a = 0.0;
 #pragma unroll
-      for (int q = 0; q < 19; ++q) {
-        a = a + hb[c][q] * (double)gw(q);
-        b = b + ht[c][q] * (double)gw(q);
+        for (int q = 0; q < 19; ++q) a = a + h[c][q] * (double)gw(q);
+        rp[c * NP + t] = a;
+        pp[c * NP + t] = get_psi(a);
       }
-      rlo[c * NP + t] = a;
-      rhi[c * NP + t] = b;
-      plo[c * NP + t] = get_psi(a);
-      phi[c * NP + t] = get_psi(b);
-    }
+  };
+  if (!top) {
+    bottom();
+    put(hb, hlo, rlo, plo);
+    return;
   }
+  double ht[NC][19], df[NC][19];
+  for (int c = 0; c < NC; ++c)
+    for (int q = 0; q < 19; ++q)
+      ht[c][q] = f * at(c, q, false, z - S.eoff - 1) + (1.0 - f) * at(c, q, false, z - S.eoff);
+  const bool neg = le_adjust_df<NC>(P, ht, S.shear_u, +1.0, df);
+  if (neg) bottom();
+  le_adjust_apply<NC>(ht, hb, df, neg);
+  put(ht, hhi, rhi, phi);
 }
 
 // ---------------------------------------------------------------------------
@@ -100,13 +107,14 @@ __global__ void k_le_halo(DevParams P, LEStep S, const double *__restrict__ src,
 // flux and the post-stream moments (code/lb3d_advection.F90:54-151,
 // code/lb3d_bc_bounce.F90:53-90, code/lb3d_analysis.F90:64-102).
 // ---------------------------------------------------------------------------
-// One launch per component c (components are independent here; the
-// advected dipole flux uses the surfactant only), which keeps one
-// component's 19 pulls live per thread; FLUX marks the surfactant launch,
-// which also accumulates the dipole flux.  STORE writes the post-stream
-// populations to fout and MOM the momenta: the moments pass of the pulling
-// step (k_collide with PULL) writes the moments only.
-template <int NC, bool LE, bool FLUX, bool ROCK, bool STORE = true, bool MOM = true>
+// A thread streams one component (components are independent here; the
+// advected dipole flux uses the surfactant only), c0 + blockIdx.y, which keeps
+// one component's 19 pulls live; FLUX compiles the dipole flux, accumulated
+// for the surfactant.  STORE writes the post-stream populations to fout: the
+// moments pass of the pulling step (k_collide with PULL) writes the moments
+// only, and under Lees-Edwards the populations of the x boundary planes
+// ([2][NC][19][nz][ny], x = nx - 1 and x = 0) to fout for the stage-8 halo.
+template <int NC, bool LE, bool FLUX, bool ROCK, bool STORE = true>
 __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__restrict__ fin,
                                                 double *__restrict__ fout, double *__restrict__ rho,
                                                 double *__restrict__ psi, double *__restrict__ mom,
@@ -114,7 +122,8 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
                                                 const double *__restrict__ db,
                                                 const uint8_t *__restrict__ rock,
                                                 const double *__restrict__ hlo,
-                                                const double *__restrict__ hhi, int c) {
+                                                const double *__restrict__ hhi, int c0) {
+  const int c = c0 + blockIdx.y;
   const long long N = P.nsites;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
@@ -143,14 +152,15 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
       upf[q] = !ROCK || rock[up[q]] == 0;
     }
   }
-  auto pulled = [&](int c, int q) -> double {
-    long long j = up[q];
-    if (LE && j < 0) {
-      long long h = -1 - j;
-      if (h < NP) return hlo[(c * 19 + q) * NP + h];
-      return hhi[(c * 19 + q) * NP + (h - NP)];
+  // address of the pulled population: selected, not loaded under a branch, so
+  // that the pulls overlap
+  auto pulled = [&](int q) -> const double * {
+    const double *src = fin + (c * 19 + q) * N + up[q];
+    if (LE && up[q] < 0) {
+      const long long h = -1 - (long long)up[q];
+      src = h < NP ? hlo + (c * 19 + q) * NP + h : hhi + (c * 19 + q) * NP + (h - NP);
     }
-    return fin[(c * 19 + q) * N + j];
+    return src;
   };
 
   double d0 = 0.0, d1 = 0.0, d2 = 0.0;
@@ -158,13 +168,25 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
     double n[19];
 #pragma unroll
     for (int q = 0; q < 18; ++q) {
-      if (fluid)
-        n[q] = upf[q] ? pulled(c, q) : fin[(c * 19 + bounce(q)) * N + i];
-      else
-        n[q] = fin[(c * 19 + q) * N + i];
+      if constexpr (!ROCK && !LE) {
+        n[q] = fin[(c * 19 + q) * N + up[q]];
+      } else {
+        const double *src = pulled(q);
+        if (!upf[q]) src = fin + (c * 19 + bounce(q)) * N + i;
+        if (!fluid) src = fin + (c * 19 + q) * N + i;
+        n[q] = *src;
+      }
     }
     n[REST] = fin[(c * 19 + REST) * N + i];
-    if (FLUX) {
+    if (LE && !STORE) {
+      const long long t = y + (long long)ny * z;
+#pragma unroll
+      for (int q = 0; q < 19; ++q) {
+        if (x == nx - 1) fout[(c * 19 + q) * NP + t] = n[q];
+        if (x == 0) fout[((NC + c) * 19 + q) * NP + t] = n[q];
+      }
+    }
+    if (FLUX && c == 2) {
       // advected dipole flux: bounce-back terms first (lb3d_bc_bounce_back_hw
       // runs before lb3d_advection_step), then the pulls, then the rest
       // population (code/lb3d_advection.F90:137-148).
@@ -205,20 +227,18 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
     }
     rho[c * N + i] = r;
     psi[c * N + i] = get_psi(r);
-    if (MOM) {
 #pragma unroll
-      for (int q = 0; q < 19; ++q) {
-        double ng = n[q] * (double)gw(q);
-        u0 = u0 + ng * (double)cx(q);
-        u1 = u1 + ng * (double)cy(q);
-        u2 = u2 + ng * (double)cz(q);
-      }
-      mom[(c * 3 + 0) * N + i] = u0;
-      mom[(c * 3 + 1) * N + i] = u1;
-      mom[(c * 3 + 2) * N + i] = u2;
+    for (int q = 0; q < 19; ++q) {
+      double ng = n[q] * (double)gw(q);
+      u0 = u0 + ng * (double)cx(q);
+      u1 = u1 + ng * (double)cy(q);
+      u2 = u2 + ng * (double)cz(q);
     }
+    mom[(c * 3 + 0) * N + i] = u0;
+    mom[(c * 3 + 1) * N + i] = u1;
+    mom[(c * 3 + 2) * N + i] = u2;
   }
-  if (FLUX) {
+  if (FLUX && c == 2) {
     da[i] = d0;
     da[N + i] = d1;
     da[2 * N + i] = d2;
@@ -404,7 +424,8 @@ __global__ void __launch_bounds__(256) k_dipole(DevParams P, const double *__res
 // rock), and rock neighbours reached through the y/z halo without their
 // rock colour (the Lees-Edwards y/z swaps do not copy it, :1079-1308).
 // ---------------------------------------------------------------------------
-template <bool LE>
+// ROCK false: no site is rock.
+template <bool LE, bool ROCK>
 __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y, int z, long long i,
                                                 const double *__restrict__ rho,
                                                 const double *__restrict__ psi,
@@ -429,7 +450,7 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
       psi_b = pp[NP + h];
     } else {
       long long j = sidx(wrap(xn, nx), wrap(yn, ny), wrap(zn, nz), nx, ny);
-      if (rock[j] != 0) {
+      if (ROCK && rock[j] != 0) {
         rk = true;
         bool through_halo = (yn < 0 || yn >= ny || zn < 0 || zn >= nz || xn < 0 || xn >= nx);
         double rcr = (LE && through_halo) ? 0.0 : P.rc_r;
@@ -526,7 +547,7 @@ __device__ __forceinline__ void sc_force_ternary(const DevParams &P, int x, int 
   }
 }
 
-template <int NC, bool LE>
+template <int NC, bool LE, bool ROCK>
 __device__ __forceinline__ void sc_forces(const DevParams &P, int x, int y, int z, long long i,
                                           const double *rho, const double *psi, const double *db,
                                           const uint8_t *rock, const double *plo,
@@ -534,14 +555,14 @@ __device__ __forceinline__ void sc_forces(const DevParams &P, int x, int y, int 
   for (int c = 0; c < NC; ++c) F[c][0] = F[c][1] = F[c][2] = 0.0;
   if (rock[i] != 0) return;
   if (NC == 2)
-    sc_force_binary<LE>(P, x, y, z, i, rho, psi, rock, plo, phi, F[0], F[1]);
+    sc_force_binary<LE, ROCK>(P, x, y, z, i, rho, psi, rock, plo, phi, F[0], F[1]);
   else
     sc_force_ternary(P, x, y, z, i, psi, db, F[0], F[1], F[NC - 1]);
 }
 
 // ---------------------------------------------------------------------------
-// Forces + BGK, code/lb3d_collision.F90:151-289.  With PULL (periodic
-// lattices without stage-8 boundaries) g is the pre-stream state and each
+// Forces + BGK, code/lb3d_collision.F90:151-289.  With PULL (lattices without
+// inflow boundaries) g is the pre-stream state and each
 // post-stream population is pulled from it as k_stream pulls it
 // (code/lb3d_advection.F90:109-151, bounce-back from a rock upstream site,
 // rock sites unmoved): the moments pass before (k_stream without STORE)
@@ -561,14 +582,16 @@ __global__ void __launch_bounds__(256, (PULL && ROCK && NC == 2) ? 3 : ((PULL ||
                                                  const double *__restrict__ db,
                                                  const uint8_t *__restrict__ rock,
                                                  const double *__restrict__ plo,
-                                                 const double *__restrict__ phi) {
+                                                 const double *__restrict__ phi,
+                                                 const double *__restrict__ hlo = nullptr,
+                                                 const double *__restrict__ hhi = nullptr) {
   const long long N = P.nsites;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= N) return;
   int x, y, z;
   site_xyz(i, P.nx, P.ny, x, y, z);
   double F[NC][3];
-  sc_forces<NC, LE>(P, x, y, z, i, rho, psi, db, rock, plo, phi, F);
+  sc_forces<NC, LE, ROCK>(P, x, y, z, i, rho, psi, db, rock, plo, phi, F);
   double r[NC];
   for (int c = 0; c < NC; ++c) r[c] = rho[c * N + i];
   if (applyforce(P, x + 1, y + 1, z + 1)) {
@@ -600,9 +623,21 @@ __global__ void __launch_bounds__(256, (PULL && ROCK && NC == 2) ? 3 : ((PULL ||
       if (q == REST || (ROCK && rock[i] != 0)) {
         nq = g[(c * 19 + q) * N + i];
       } else {
-        const long long j =
-            sidx(wrap(x - cx(q), P.nx), wrap(y - cy(q), P.ny), wrap(z - cz(q), P.nz), P.nx, P.ny);
-        nq = (ROCK && rock[j] != 0) ? g[(c * 19 + bounce(q)) * N + i] : g[(c * 19 + q) * N + j];
+        const int yu = wrap(y - cy(q), P.ny), zu = wrap(z - cz(q), P.nz), xu = x - cx(q);
+        const long long j = sidx(wrap(xu, P.nx), yu, zu, P.nx, P.ny);
+        // the address is selected, not the load: a branch around each load would
+        // keep the 19 pulls from overlapping (172 us against 81 for the sheared
+        // 97x66x63 lattice)
+        const double *src = g + (c * 19 + q) * N + j;
+        bool bounced = ROCK && rock[j] != 0;
+        if (LE) {
+          // across the sheared boundary: the stage-6 halo planes, never rock
+          const long long NP = (long long)P.ny * P.nz, t = (c * 19 + q) * NP + yu + (long long)P.ny * zu;
+          if (xu < 0) src = hlo + t, bounced = false;
+          if (xu >= P.nx) src = hhi + t, bounced = false;
+        }
+        if (ROCK && bounced) src = g + (c * 19 + bounce(q)) * N + i;
+        nq = *src;
       }
       double eq = r[c] * b[q];
       f[(c * 19 + q) * N + i] = nq - P.omega[c] * (nq - eq);
@@ -688,7 +723,7 @@ __global__ void k_dump(DevParams P, int field, const double *__restrict__ f,
     }
     case 5: {  // arr
       double F[NC][3];
-      sc_forces<NC, false>(P, x, y, z, i, rho, psi, db, rock, nullptr, nullptr, F);
+      sc_forces<NC, false, true>(P, x, y, z, i, rho, psi, db, rock, nullptr, nullptr, F);
       double den = 0.0;
       for (int c = 0; c < NC; ++c) {
         double t = sumg(c, 3) * P.amass[c];
@@ -762,16 +797,60 @@ static inline unsigned grid_for(long long n, int bs) { return (unsigned)((n + bs
 // ---------------------------------------------------------------------------
 using namespace fp64;
 
-cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, double *hlo,
+
+cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, bool compact, double *hlo,
                          double *hhi, double *rlo, double *rhi, double *plo, double *phi,
                          cudaStream_t st) {
-  int n = P.ny * P.nz;
-  if (P.nc == 2)
-    k_le_halo<2><<<grid_for(n, 128), 128, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
+  const unsigned g = grid_for(2LL * P.ny * P.nz, 64);
+  if (P.nc != 2) return cudaErrorInvalidValue;
+  if (compact)
+    k_le_halo<2, true><<<g, 64, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
   else
-    k_le_halo<3><<<grid_for(n, 128), 128, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
+    k_le_halo<2, false><<<g, 64, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
   return cudaGetLastError();
 }
+
+// Threads per block of the site kernels.  Small lattices take small blocks,
+// which spread their sites over more SMs (binary 64^3, a step: 60 us with 64,
+// 63 with 256; ternary 32^3: 29.7 with 64, 30.6 with 128, 31 with 256), the
+// smallest 128, whose neighbours share more of an L1 (ternary 16^3: 23.8
+// against 25.7 us).
+static int fp64_block(const DevParams &P) { return P.nsites > 300000 ? 256 : P.nsites > 16384 ? 64 : 128; }
+// Lattices bound by launches and latency stream all components in one launch
+// (ternary 32^3: 29.7 us a step against 33.5 with two).
+static bool fp64_small(const DevParams &P) { return P.nsites <= 65536; }
+
+// The stream kernel over all components: red and blue in one launch and the
+// surfactant, whose dipole flux takes twice the registers, in another (ternary
+// 128^3: 58 + 58 + 107 us as three launches); small lattices, bound by
+// launches and latency, all three in one.
+template <bool STORE>
+static cudaError_t launch_stream(const DevParams &P, const double *fin, double *fout, double *rho, double *psi,
+                                 double *mom, double *da, const double *db, const uint8_t *rock, const double *hlo,
+                                 const double *hhi, cudaStream_t st) {
+  const int bs = fp64_block(P);
+  const unsigned gr = grid_for(P.nsites, bs);
+#define LB3D_STREAM(NC_, LE_, FLUX_, ny_, c_)                                                        \
+  (P.any_rock ? k_stream<NC_, LE_, FLUX_, true, STORE><<<dim3(gr, ny_), bs, 0, st>>>(                 \
+                    P, fin, fout, rho, psi, mom, da, db, rock, hlo, hhi, c_)                          \
+              : k_stream<NC_, LE_, FLUX_, false, STORE><<<dim3(gr, ny_), bs, 0, st>>>(                \
+                    P, fin, fout, rho, psi, mom, da, db, rock, hlo, hhi, c_))
+  if (P.nc == 2) {
+    if (P.le)
+      LB3D_STREAM(2, true, false, 2, 0);
+    else
+      LB3D_STREAM(2, false, false, 2, 0);
+  } else if (fp64_small(P)) {
+    LB3D_STREAM(3, false, true, 3, 0);
+  } else {
+    LB3D_STREAM(3, false, false, 2, 0);
+    LB3D_STREAM(3, false, true, 1, 2);
+  }
+#undef LB3D_STREAM
+  return cudaGetLastError();
+}
+
+int fp64_stream_launches(const DevParams &P) { return P.nc == 2 || fp64_small(P) ? 1 : 2; }
 
 cudaError_t fp64_zouhe_flux(const DevParams &P, double *g, double *da, const double *db,
                             const uint8_t *rock, cudaStream_t st) {
@@ -801,88 +880,42 @@ cudaError_t fp64_stream(const DevParams &P, const double *fin, double *fout, dou
                         double *psi, double *mom, double *da, const double *db,
                         const uint8_t *rock, const double *hlo, const double *hhi,
                         cudaStream_t st) {
-  unsigned gr = grid_for(P.nsites, 256);
-#define LB3D_STREAM(NC_, LE_, FLUX_)                                                           \
-  (P.any_rock ? k_stream<NC_, LE_, FLUX_, true><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, da, \
-                                                                    db, rock, hlo, hhi, c)        \
-              : k_stream<NC_, LE_, FLUX_, false><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, da, \
-                                                                     db, rock, hlo, hhi, c))
-  for (int c = 0; c < P.nc; ++c) {
-    if (P.nc == 2) {
-      if (P.le)
-        LB3D_STREAM(2, true, false);
-      else
-        LB3D_STREAM(2, false, false);
-    } else if (c < 2) {
-      LB3D_STREAM(3, false, false);
-    } else {
-      LB3D_STREAM(3, false, true);
-    }
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-#undef LB3D_STREAM
-  return cudaSuccess;
+  return launch_stream<true>(P, fin, fout, rho, psi, mom, da, db, rock, hlo, hhi, st);
 }
 
 cudaError_t fp64_step_pull(const DevParams &P, const double *fin, double *fout, double *rho,
                            double *psi, double *mom, double *da, double *db, const uint8_t *rock,
-                           cudaStream_t st) {
-  if (P.le || P.zouhe) return cudaErrorInvalidValue;
-  unsigned gr = grid_for(P.nsites, 256);
+                           cudaStream_t st, const Fp64Le *le) {
+  if (P.zouhe || (P.le != 0) != (le != nullptr)) return cudaErrorInvalidValue;
+  const int bs = fp64_block(P);
+  const unsigned gr = grid_for(P.nsites, bs);
   const bool rk = P.any_rock != 0;
-  // moments pass: densities, psi and (surfactant) the advected dipole flux
-  for (int c = 0; c < P.nc; ++c) {
-#define LB3D_MOMENTS(NC_, FLUX_, ROCK_)                                                  \
-  k_stream<NC_, false, FLUX_, ROCK_, false, true><<<gr, 256, 0, st>>>(P, fin, nullptr, rho, psi, \
-                                                                      mom, da, db, rock, nullptr, \
-                                                                      nullptr, c)
-    if (P.nc == 2) {
-      if (rk)
-        LB3D_MOMENTS(2, false, true);
-      else
-        LB3D_MOMENTS(2, false, false);
-    } else if (c < 2) {
-      if (rk)
-        LB3D_MOMENTS(3, false, true);
-      else
-        LB3D_MOMENTS(3, false, false);
-    } else {
-      if (rk)
-        LB3D_MOMENTS(3, true, true);
-      else
-        LB3D_MOMENTS(3, true, false);
-    }
-#undef LB3D_MOMENTS
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if (P.nc == 3) {
-    k_dipole<<<grid_for(P.nsites, 256), 256, 0, st>>>(P, rho, da, db);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  if (P.nc == 2) {
-    if (rk)
-      k_collide<2, false, true, true><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, nullptr,
-                                                           nullptr);
-    else
-      k_collide<2, false, true, false><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, nullptr,
-                                                            nullptr);
-  } else {
-    if (rk)
-      k_collide<3, false, true, true><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, nullptr,
-                                                           nullptr);
-    else
-      k_collide<3, false, true, false><<<gr, 256, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, nullptr,
-                                                            nullptr);
-  }
+  // moments pass: densities, psi, momenta and (surfactant) the advected dipole flux
+  cudaError_t e = launch_stream<false>(P, fin, le ? le->post : nullptr, rho, psi, mom, da, db, rock,
+                                       le ? le->hlo : nullptr, le ? le->hhi : nullptr, st);
+  if (e == cudaSuccess && P.nc == 3) e = fp64_dipole(P, rho, da, db, st);
+  if (e == cudaSuccess && le)
+    e = fp64_le_halo(P, le->step, le->post, true, nullptr, nullptr, le->rlo, le->rhi, le->plo, le->phi, st);
+  if (e != cudaSuccess) return e;
+  const double *plo = le ? le->plo : nullptr, *phi = le ? le->phi : nullptr;
+  const double *hlo = le ? le->hlo : nullptr, *hhi = le ? le->hhi : nullptr;
+#define LB3D_PULL(NC_, LE_)                                                                                    \
+  (rk ? k_collide<NC_, LE_, true, true><<<gr, bs, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, plo, phi, hlo, hhi) \
+      : k_collide<NC_, LE_, true, false><<<gr, bs, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, plo, phi, hlo, hhi))
+  if (P.nc == 3)
+    LB3D_PULL(3, false);
+  else if (le)
+    LB3D_PULL(2, true);
+  else
+    LB3D_PULL(2, false);
+#undef LB3D_PULL
   return cudaGetLastError();
 }
 
 cudaError_t fp64_dipole(const DevParams &P, const double *rho, const double *da, double *db,
                         cudaStream_t st) {
-  k_dipole<<<grid_for(P.nsites, 256), 256, 0, st>>>(P, rho, da, db);
+  const int bs = fp64_block(P);
+  k_dipole<<<grid_for(P.nsites, bs), bs, 0, st>>>(P, rho, da, db);
   return cudaGetLastError();
 }
 
@@ -890,14 +923,15 @@ cudaError_t fp64_collide(const DevParams &P, const double *g, double *f, const d
                          const double *psi, const double *mom, const double *db,
                          const uint8_t *rock, const double *plo, const double *phi,
                          cudaStream_t st) {
-  unsigned gr = grid_for(P.nsites, 256);
+  const int bs = fp64_block(P);
+  const unsigned gr = grid_for(P.nsites, bs);
   if (P.nc == 2) {
     if (P.le)
-      k_collide<2, true><<<gr, 256, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
+      k_collide<2, true><<<gr, bs, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
     else
-      k_collide<2, false><<<gr, 256, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
+      k_collide<2, false><<<gr, bs, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
   } else {
-    k_collide<3, false><<<gr, 256, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
+    k_collide<3, false><<<gr, bs, 0, st>>>(P, g, f, rho, psi, mom, db, rock, plo, phi);
   }
   return cudaGetLastError();
 }

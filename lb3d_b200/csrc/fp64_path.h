@@ -6,7 +6,10 @@
 
 namespace lb3d {
 
-cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, double *hlo,
+// Lees-Edwards x-halo planes from the populations src (compact: from the
+// boundary planes [2][nc][19][nz][ny] of x = nx - 1 and x = 0), their
+// densities and psi when rlo is given; binary lattices.
+cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, bool compact, double *hlo,
                          double *hhi, double *rlo, double *rhi, double *plo, double *phi,
                          cudaStream_t st);
 // Zou-He flux boundaries on the z = 1 and z = nz planes (inv_fluid 12),
@@ -21,15 +24,25 @@ cudaError_t fp64_stream(const DevParams &P, const double *fin, double *fout, dou
                         double *psi, double *mom, double *da, const double *db,
                         const uint8_t *rock, const double *hlo, const double *hhi,
                         cudaStream_t st);
-// One time step with streaming fused into the collision (periodic lattices,
-// no Lees-Edwards planes, no stage-8 boundaries): moments pass (rho, psi,
-// momenta, dipole flux), dipole relaxation (ternary), pull + forces + BGK
-// from fin into fout.  Every buffer ends up as after fp64_stream +
-// fp64_dipole + fp64_collide, bit for bit, except that the post-stream
+// Kernels of fp64_stream, and of fp64_step_pull's moments pass.
+int fp64_stream_launches(const DevParams &P);
+// Lees-Edwards planes of a pulling step: the stage-6 halo (filled), the
+// step's offset, the post-stream boundary planes [2][nc][19][nz][ny] and the
+// stage-8 halo densities and psi (filled by the step).
+struct Fp64Le {
+  LEStep step;
+  const double *hlo, *hhi;
+  double *post, *rlo, *rhi, *plo, *phi;
+};
+// One time step with streaming fused into the collision (lattices without
+// inflow boundaries; le under Lees-Edwards): moments pass (rho, psi, momenta,
+// dipole flux), dipole relaxation (ternary), stage-8 halo (Lees-Edwards), pull
+// + forces + BGK from fin into fout.  Every buffer ends up as after fp64_stream
+// + fp64_dipole + fp64_collide, bit for bit, except that the post-stream
 // populations are never stored.
 cudaError_t fp64_step_pull(const DevParams &P, const double *fin, double *fout, double *rho,
                            double *psi, double *mom, double *da, double *db, const uint8_t *rock,
-                           cudaStream_t st);
+                           cudaStream_t st, const Fp64Le *le = nullptr);
 cudaError_t fp64_dipole(const DevParams &P, const double *rho, const double *da, double *db,
                         cudaStream_t st);
 cudaError_t fp64_collide(const DevParams &P, const double *g, double *f, const double *rho,

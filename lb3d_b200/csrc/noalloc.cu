@@ -13,6 +13,7 @@
 #include <cstdio>
 #include <mutex>
 #include <string>
+#include <utility>
 
 #include <cuda.h>
 
@@ -142,13 +143,18 @@ extern "C" int lb3dc_time_loop_fp64_noalloc(const lb3dc_params *p, double *f, do
   }
   lb3d::DevParams P = lb3d::dev_params_from(*p);
   P.any_rock = rock ? 1 : 0;  // a caller's mask may hold rock
+  // Every scratch field is written by the moments pass before the dipole and
+  // collide kernels read it, so nothing else needs clearing.  The pulling steps
+  // alternate between the caller's populations and the scratch ones; after an
+  // odd number of them the populations are copied back.
+  double *in = f, *out = g;
   for (int s = 0; s < nsteps; ++s) {
-    // Every scratch field is written by the stream kernel before the dipole
-    // and collide kernels read it, so nothing else needs clearing.
-    e = lb3d::fp64_stream(P, f, g, rho, psi, mom, da, db, rk, nullptr, nullptr, st);
-    if (e == cudaSuccess && nc == 3) e = lb3d::fp64_dipole(P, rho, da, db, st);
-    if (e == cudaSuccess)
-      e = lb3d::fp64_collide(P, g, f, rho, psi, mom, db, rk, nullptr, nullptr, st);
+    e = lb3d::fp64_step_pull(P, in, out, rho, psi, mom, da, db, rk, st);
+    if (e != cudaSuccess) return err(LB3DC_ECUDA, cudaGetErrorString(e));
+    std::swap(in, out);
+  }
+  if (in != f) {
+    e = cudaMemcpyAsync(f, in, (size_t)nc * 19 * n * 8, cudaMemcpyDeviceToDevice, st);
     if (e != cudaSuccess) return err(LB3DC_ECUDA, cudaGetErrorString(e));
   }
   return LB3DC_OK;
