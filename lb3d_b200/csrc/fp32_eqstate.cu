@@ -230,6 +230,8 @@ __device__ __forceinline__ float vmul(float a, float b) { return a * b; }
 __device__ __forceinline__ float2 vmul(float2 a, float2 b) { return mul2(a, b); }
 __device__ __forceinline__ float vfma(float a, float b, float c) { return fmaf(a, b, c); }
 __device__ __forceinline__ float2 vfma(float2 a, float2 b, float2 c) { return fma2(a, b, c); }
+__device__ __forceinline__ float vlane(float a, int) { return a; }
+__device__ __forceinline__ float vlane(float2 a, int k) { return k ? a.y : a.x; }
 __device__ __forceinline__ float vneg(float a) { return -a; }
 __device__ __forceinline__ float vsub(float a, float b) { return a - b; }
 // one instruction: b scaled by -1 is exact
@@ -373,10 +375,19 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
       }
       const V sg = vset(V(), lo ? 1.0f : -1.0f), sd = vset(V(), lo != row ? 1.0f : -1.0f);
       V up = vset(V(), 0.f);
+      // a sheared halo site's populations, read one plane ahead (their latency
+      // would hold up the whole CTA at the barrier)
+      float2 ahead[5];
+      auto read_sheared = [&](int z) {
+#pragma unroll
+        for (int k = 0; k < 5; ++k) ahead[k] = sheared(hq[k], z);
+      };
+      if constexpr (LE && !SURF)
+        if (side >= 0) read_sheared(zl == 0 ? nz - 1 : zl - 1);
 #pragma unroll 1
       for (int m = 0; m <= zc + 1; ++m) {
         if (part) {
-          const int z = zl == 0 ? nz - 1 : zl - 1;  // of plane m
+          const int z = zl;  // of plane m + 1
           V *mD = pD + (m % DS) * 4 * AN, *mZ = pZ + (m & 1) * 8 * AN, *mU = pU + ((m - 1) & 1) * 4 * AN;
           if (m > 0) mU[off[3]] = up;
           cp_async_wait<0>();
@@ -398,9 +409,10 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
           up = lo ? A : B;
           V down = lo ? B : A;
           if constexpr (LE && !SURF)
-            if (side >= 0)
-              z0v = sheared(hq[0], z), z1v = sheared(hq[1], z), z2v = sheared(hq[2], z), up = sheared(hq[3], z),
-              down = sheared(hq[4], z);
+            if (side >= 0) {
+              z0v = ahead[0], z1v = ahead[1], z2v = ahead[2], up = ahead[3], down = ahead[4];
+              if (m <= zc) read_sheared(z);
+            }
           mZ[off[0]] = z0v;
           mZ[off[1]] = z1v;
           mZ[off[2]] = z2v;
@@ -487,48 +499,59 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
           if (cz(d) == 1) return pU + ((own_site ? 1 - P : P) * 4 + dir_slot(d)) * AN + s;
           return pD + ((DS == 1 ? 0 : own_site ? 1 - P : P) * 4 + dir_slot(d)) * AN + s;
         };
-        // a site on the sheared boundary also leaves them for the stage-8 halo
-        // kernel (a rock site the populations it keeps)
-        float *lbp = nullptr;
-        if (LE && (vx == 0 || vx == nx - 1)) lbp = Lg.le_b[vx == 0 ? 3 : 2] + vy + ny * zo;
         V r = vset(V(), 0.f), j0 = r, j1 = r, j2 = r;
         float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+        // edge: the tile holds sites on the sheared boundary, which also leave
+        // their populations for the stage-8 halo kernel (a rock site those it
+        // keeps)
+        auto sum = [&](auto edge) {
+          float *lbp = nullptr;
+          if (decltype(edge)::value && (vx == 0 || vx == nx - 1)) lbp = Lg.le_b[vx == 0 ? 3 : 2] + vy + ny * zo;
 #pragma unroll
-        for (int d = 0; d < 19; ++d) {
-          V v;
-          const bool hit = ROCK && d < 18 && (mk >> d & 1u);
-          if (d == 18) {
-            v = rest1;
-          } else if (d == 4) {
-            v = hit ? d5p : u4q;
-          } else if (d == 5) {
-            v = hit ? u4p : d5;
-          } else {
-            const V *p = plane(d, false) - cx(d) - AW * cy(d);
-            if (hit) p = plane(bounce(d), true);
-            v = *p;
-          }
-          if constexpr (LE && !SURF) {
-            if (lbp) {
-              lbp[d * NP] = fluid ? v.x : rock_dev(d, rho0);
-              lbp[(19 + d) * NP] = fluid ? v.y : rock_dev(d, rho0);
+          for (int d = 0; d < 19; ++d) {
+            V v;
+            const bool hit = ROCK && d < 18 && (mk >> d & 1u);
+            if (d == 18) {
+              v = rest1;
+            } else if (d == 4) {
+              v = hit ? d5p : u4q;
+            } else if (d == 5) {
+              v = hit ? u4p : d5;
+            } else {
+              const V *p = plane(d, false) - cx(d) - AW * cy(d);
+              if (hit) p = plane(bounce(d), true);
+              v = *p;
+            }
+            if constexpr (decltype(edge)::value) {
+              if (lbp) {
+                lbp[d * NP] = fluid ? vlane(v, 0) : rock_dev(d, rho0);
+                lbp[(19 + d) * NP] = fluid ? vlane(v, 1) : rock_dev(d, rho0);
+              }
+            }
+            const float g = (float)gw(d);
+            r = vfma(vset(V(), g), v, r);
+            if (cx(d)) j0 = vfma(vset(V(), g * (float)cx(d)), v, j0);
+            if (cy(d)) j1 = vfma(vset(V(), g * (float)cy(d)), v, j1);
+            if (cz(d)) j2 = vfma(vset(V(), g * (float)cz(d)), v, j2);
+            if constexpr (SURF) {
+              // da = sum_q (n_s(x - c_q, q) g_q) db(x - c_q) + n_s(x, rest) db(x)
+              // planes m - 2, m - 1, m
+              const float4 *p = cz(d) == 1 ? dx + P * AN : cz(d) == 0 ? (P ? dm : dx + AN) : dm + P * AN;
+              const float4 bb = p[-cx(d) - AW * cy(d)];
+              const float ng = g * fmaf(wq(d), rho0, v);
+              a0 = fmaf(ng, bb.x, a0);
+              a1 = fmaf(ng, bb.y, a1);
+              a2 = fmaf(ng, bb.z, a2);
             }
           }
-          const float g = (float)gw(d);
-          r = vfma(vset(V(), g), v, r);
-          if (cx(d)) j0 = vfma(vset(V(), g * (float)cx(d)), v, j0);
-          if (cy(d)) j1 = vfma(vset(V(), g * (float)cy(d)), v, j1);
-          if (cz(d)) j2 = vfma(vset(V(), g * (float)cz(d)), v, j2);
-          if constexpr (SURF) {
-            // da = sum_q (n_s(x - c_q, q) g_q) db(x - c_q) + n_s(x, rest) db(x)
-            // planes m - 2, m - 1, m
-            const float4 *p = cz(d) == 1 ? dx + P * AN : cz(d) == 0 ? (P ? dm : dx + AN) : dm + P * AN;
-            const float4 bb = p[-cx(d) - AW * cy(d)];
-            const float ng = g * fmaf(wq(d), rho0, v);
-            a0 = fmaf(ng, bb.x, a0);
-            a1 = fmaf(ng, bb.y, a1);
-            a2 = fmaf(ng, bb.z, a2);
-          }
+        };
+        if constexpr (LE && !SURF) {
+          if (x0 == 0 || x0 + TX >= nx)
+            sum(std::true_type());
+          else
+            sum(std::false_type());
+        } else {
+          sum(std::false_type());
         }
         if constexpr (SURF) {
           const float am = Lg.amass[2] * Lg.omega[2];
@@ -798,11 +821,20 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
     const int x0 = T.x0, y0 = T.y0, z0 = T.z0, zc = T.zc;
     const int gx = x0 + tx, gy = y0 + ty;
     const bool act = gx < nx && gy < ny;
-    int rxy[RE];  // the in-plane offsets of this thread's ring entries
+    // the in-plane offsets of this thread's ring entries; the psi entries of
+    // sheared halo columns come from the stage-8 halo planes
+    int rxy[RE];
+    const float2 *rps[RE];
+    int rpl[RE];
 #pragma unroll
     for (int e = 0; e < RE; ++e) {
       const int s = tid + e * NT;
-      rxy[e] = s < AN ? wrapz(x0 - 1 + s % AW, nx) + nx * wrapz(y0 - 1 + s / AW, ny) : 0;
+      const int ry = wrapz(y0 - 1 + s / AW, ny);
+      rxy[e] = s < AN ? wrapz(x0 - 1 + s % AW, nx) + nx * ry : 0;
+      rps[e] = PS + rxy[e];
+      rpl[e] = pl;
+      const int vx = x0 - 1 + s % AW;
+      if (LE && s < AN && (vx == -1 || vx == nx)) rps[e] = Lg.le_p[vx < 0 ? 0 : 1] + ry, rpl[e] = ny;
     }
     const int own_xy = gx + nx * gy;
     auto load_ring = [&](int r) {  // plane z0 - 1 + r in slot r % RS
@@ -812,12 +844,7 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
         const int s = tid + e * NT;
         if (s >= AN) break;
         if (NC == 3) cp_async16(ringA + sl + s, DD + rxy[e] + pl * gz);
-        const float2 *src = PS + rxy[e] + pl * gz;
-        if (LE) {  // sheared halo columns: the stage-8 halo planes
-          const int vx = x0 - 1 + s % AW;
-          if (vx == -1 || vx == nx) src = Lg.le_p[vx < 0 ? 0 : 1] + wrapz(y0 - 1 + s / AW, ny) + ny * gz;
-        }
-        cp_async8(ringP + sl + s, src);
+        cp_async8(ringP + sl + s, rps[e] + (LE ? rpl[e] : pl) * gz);
       }
       if (act) {
         const int i = own_xy + pl * gz, o = (r % RS) * NT + tid;
@@ -972,9 +999,10 @@ using namespace f32;
 // Tile of the moments passes: 32 x 8, or 16 x 8 where that pads the lattice's
 // x side less.  At equal padding the wider tile is 3 % faster (ternary 128^3,
 // a step: 0.213 against 0.220 ms; binary 256x128x128: 0.162 against 0.164):
-// its halo is 0.33 of the tile's sites, the narrower one's 0.41.
-void eq_moments_tile(int nx, int *tx, int *ty) {
-  *tx = 1.03 * ((nx + 15) / 16 * 16) < (double)((nx + 31) / 32 * 32) ? 16 : 32;
+// its halo is 0.33 of the tile's sites, the narrower one's 0.41.  Sheared
+// lattices: 16 x 8, whose variant does not spill.
+void eq_moments_tile(int nx, bool le, int *tx, int *ty) {
+  *tx = le || 1.03 * ((nx + 15) / 16 * 16) < (double)((nx + 31) / 32 * 32) ? 16 : 32;
   *ty = 8;
 }
 
@@ -1001,9 +1029,10 @@ static bool eq_moments_fn(int pass, bool first, bool narrow, EqKernel *k) {
 template <int NC, bool ROCK, bool LE>
 static bool eq_fn(int pass, bool first, int tx, int ty, bool narrow, EqKernel *k) {
   if (pass == EQ_MOMENTS || pass == EQ_SURFACTANT) {
-    if (ty != 8 || (tx != 16 && tx != 32) || (pass == EQ_SURFACTANT && NC != 3)) return false;
-    return tx == 32 ? eq_moments_fn<NC, ROCK, LE, 32, 8>(pass, first, narrow, k)
-                    : eq_moments_fn<NC, ROCK, LE, 16, 8>(pass, first, narrow, k);
+    if (ty != 8 || (tx != 16 && (LE || tx != 32)) || (pass == EQ_SURFACTANT && NC != 3)) return false;
+    if constexpr (!LE)
+      if (tx == 32) return eq_moments_fn<NC, ROCK, LE, 32, 8>(pass, first, narrow, k);
+    return eq_moments_fn<NC, ROCK, LE, 16, 8>(pass, first, narrow, k);
   }
 #define LB3D_EQ_SHAPE(TX, TY)                                            \
   if (tx == TX && ty == TY) {                                            \

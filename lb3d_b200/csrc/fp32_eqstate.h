@@ -45,8 +45,8 @@ struct EqArgs {
 // pass exist for ternary lattices, and a first step (from populations) takes
 // all moments in EQ_MOMENTS.
 enum { EQ_MOMENTS, EQ_SURFACTANT, EQ_DIPOLE, EQ_COLLIDE, EQ_PASSES };
-// Tile of the moments passes for a lattice nx sites wide.
-void eq_moments_tile(int nx, int *tx, int *ty);
+// Tile of the moments passes for a lattice nx sites wide (le: Lees-Edwards).
+void eq_moments_tile(int nx, bool le, int *tx, int *ty);
 // The kernel of a pass for a lattice kind and tile; false if there is none.
 // narrow: 19 nc S < 2^32.
 bool eq_kernel(int pass, bool first, int nc, bool rock, bool le, int tx, int ty, bool narrow, EqKernel *k);

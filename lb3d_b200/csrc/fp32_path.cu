@@ -900,7 +900,7 @@ static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
 static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool first, int tx, int ty, EqKernel *k) {
   const bool rock = (s.lat.flags & LAT_ROCK) != 0;
   int ax = tx, ay = ty;
-  if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, &ax, &ay);
+  if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.le != 0, &ax, &ay);
   return eq_kernel(pass, first, P.nc, rock, s.le_h[0] != nullptr, ax, ay, 19ull * P.nc * s.S < (1ull << 32), k);
 }
 
@@ -969,18 +969,20 @@ static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
       continue;
     }
     int tx = sh.tx, ty = sh.ty, res = 0;
-    if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, &tx, &ty);
+    if (pass <= EQ_SURFACTANT) eq_moments_tile(P.nx, P.le != 0, &tx, &ty);
     if (fp32_prepare_kernel(kn.fn, kn.threads, kn.smem, &res) != cudaSuccess) return LB3DC_ECUDA;
-    const int nxy = ((L.nx + tx - 1) / tx) * ((L.ny + ty - 1) / ty);
+    const int nxt = (L.nx + tx - 1) / tx, nxy = nxt * ((L.ny + ty - 1) / ty);
     const int k = fp32_z_chunks(L.nz, nxy, res, 2);
     for (int c = 0; c < k; ++c) {
       const int z0 = (int)((long long)L.nz * c / k), z1 = (int)((long long)L.nz * (c + 1) / k);
-      for (int y0 = 0; y0 < L.ny; y0 += ty)
-        for (int x0 = 0; x0 < L.nx; x0 += tx) {
+      for (int yt = 0; yt * ty < L.ny; ++yt)
+        for (int xt = 0; xt < nxt; ++xt) {
           Tile t;
           t.lat = 0;
-          t.x0 = (short)x0;
-          t.y0 = (short)y0;
+          // sheared lattices: the tiles on the x boundary take longer; rotated
+          // by row and chunk they do not all fall to the same CTAs
+          t.x0 = (short)((P.le ? (xt + yt + c) % nxt : xt) * tx);
+          t.y0 = (short)(yt * ty);
           t.z0 = (short)z0;
           t.zc = (short)(z1 - z0);
           all.push_back(t);
