@@ -41,6 +41,31 @@ __device__ __forceinline__ void site_xyz(long long i, int nx, int ny, int &x, in
   y = (int)(t - (long long)z * ny);
 }
 
+// Site offsets of the -1, 0, +1 neighbours along each axis with the periodic
+// wrap applied once, as byte offsets of a double array: a kernel adds three of
+// them per neighbour and reads every field at that one 32-bit offset (a
+// lattice of 2^29 sites, where they would overflow, needs 570 GB).  Ternary
+// 128^3: dipole pass 113 -> 92 us (with four CTAs per SM), surfactant stream
+// 126 -> 106 us (with three), collide pass 453 -> 438 us; its pulls keep their
+// 64-bit addresses, with which the compiler does not hoist them into spills.
+struct Nb {
+  unsigned x[3], y[3], z[3];
+  __device__ __forceinline__ Nb(int px, int py, int pz, int nx, int ny, int nz) {
+    const unsigned row = 8u * nx, pl = row * ny;
+    x[0] = 8u * (px == 0 ? nx - 1 : px - 1), x[1] = 8u * px, x[2] = 8u * (px == nx - 1 ? 0 : px + 1);
+    y[0] = row * (py == 0 ? ny - 1 : py - 1), y[1] = row * py, y[2] = row * (py == ny - 1 ? 0 : py + 1);
+    z[0] = pl * (pz == 0 ? nz - 1 : pz - 1), z[1] = pl * pz, z[2] = pl * (pz == nz - 1 ? 0 : pz + 1);
+  }
+  // of the neighbour at +c_q (SGN 1) or the upstream site at -c_q (SGN -1)
+  template <int SGN>
+  __device__ __forceinline__ unsigned at(int q) const {
+    return x[1 + SGN * cx(q)] + y[1 + SGN * cy(q)] + z[1 + SGN * cz(q)];
+  }
+};
+__device__ __forceinline__ double ld(const double *__restrict__ p, unsigned byte) {
+  return __ldg(reinterpret_cast<const double *>(reinterpret_cast<const char *>(p) + byte));
+}
+
 // src: populations [NC][19][nsites], or (COMPACT) the boundary planes
 // [2][NC][19][nz][ny] of x = nx - 1 and x = 0.  Writes the halo planes and,
 // when rlo is given, their densities and psi (for the force stencil).  Threads
@@ -115,7 +140,7 @@ __global__ void __launch_bounds__(64) k_le_halo(DevParams P, LEStep S, const dou
 // only, and under Lees-Edwards the populations of the x boundary planes
 // ([2][NC][19][nz][ny], x = nx - 1 and x = 0) to fout for the stage-8 halo.
 template <int NC, bool LE, bool FLUX, bool ROCK, bool STORE = true>
-__global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__restrict__ fin,
+__global__ void __launch_bounds__(256, FLUX ? 3 : 2) k_stream(DevParams P, const double *__restrict__ fin,
                                                 double *__restrict__ fout, double *__restrict__ rho,
                                                 double *__restrict__ psi, double *__restrict__ mom,
                                                 double *__restrict__ da,
@@ -134,6 +159,7 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
   const bool fluid = !ROCK || rock[i] == 0;
   const long long NP = (long long)ny * nz;
 
+  const Nb nb(x, y, z, nx, ny, nz);
   // upstream site of each moving direction (32-bit: the FP64 path bounds a
   // lattice at 2^31 sites); negative values mark the LE halo planes
   int up[18];
@@ -169,7 +195,7 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
 #pragma unroll
     for (int q = 0; q < 18; ++q) {
       if constexpr (!ROCK && !LE) {
-        n[q] = fin[(c * 19 + q) * N + up[q]];
+        n[q] = ld(fin + (c * 19 + q) * N, nb.at<-1>(q));
       } else {
         const double *src = pulled(q);
         if (!upf[q]) src = fin + (c * 19 + bounce(q)) * N + i;
@@ -206,11 +232,11 @@ __global__ void __launch_bounds__(256, 2) k_stream(DevParams P, const double *__
 #pragma unroll
         for (int q = 0; q < 18; ++q) {
           if (upf[q]) {
-            long long j = up[q];
+            const unsigned j = nb.at<-1>(q);
             double ng = n[q] * (double)gw(q);
-            d0 = d0 + ng * db[j];
-            d1 = d1 + ng * db[N + j];
-            d2 = d2 + ng * db[2 * N + j];
+            d0 = d0 + ng * ld(db, j);
+            d1 = d1 + ng * ld(db + N, j);
+            d2 = d2 + ng * ld(db + 2 * N, j);
           }
         }
       }
@@ -374,7 +400,7 @@ __device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
 // Reads rho and da of the 18 neighbours; writes db in place (no neighbour
 // reads db in this pass).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_dipole(DevParams P, const double *__restrict__ rho,
+__global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *__restrict__ rho,
                                                 const double *__restrict__ da,
                                                 double *__restrict__ db) {
   const long long N = P.nsites;
@@ -383,6 +409,8 @@ __global__ void __launch_bounds__(256) k_dipole(DevParams P, const double *__res
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   int x, y, z;
   site_xyz(i, nx, ny, x, y, z);
+  const Nb nb(x, y, z, nx, ny, nz);
+  const double *rho_b = rho + N, *da1 = da + N, *da2 = da + 2 * N;
   double h_c[3] = {0.0, 0.0, 0.0};
   double h_s[3] = {da[i], da[N + i], da[2 * N + i]};
   double sN_tmp = fmaxf_(rho[2 * N + i], CLIP_RHO_S);
@@ -391,10 +419,10 @@ __global__ void __launch_bounds__(256) k_dipole(DevParams P, const double *__res
   const double sgn = (P.g_bs >= 0.0) ? 1.0 : -1.0;
 #pragma unroll
   for (int q = 0; q < 18; ++q) {
-    long long j = sidx(wrap(x + cx(q), nx), wrap(y + cy(q), ny), wrap(z + cz(q), nz), nx, ny);
-    double psi_r = 0.0 + rho[j];
-    double psi_b = 0.0 + rho[N + j];
-    double pas[3] = {da[j], da[N + j], da[2 * N + j]};
+    const unsigned j = nb.at<1>(q);
+    double psi_r = 0.0 + ld(rho, j);
+    double psi_b = 0.0 + ld(rho_b, j);
+    double pas[3] = {ld(da, j), ld(da1, j), ld(da2, j)};
     double hc_m = -(sgn * (psi_b - psi_r) * (double)gw(q));
     const int c[3] = {cx(q), cy(q), cz(q)};
     for (int k = 0; k < 3; ++k)
@@ -494,22 +522,22 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
   }
 }
 
-__device__ __forceinline__ void sc_force_ternary(const DevParams &P, int x, int y, int z, long long i,
+__device__ __forceinline__ void sc_force_ternary(const DevParams &P, const Nb &nb, long long i,
                                                  const double *__restrict__ psi,
                                                  const double *__restrict__ db, double *fr,
                                                  double *fb, double *fs) {
   const long long N = P.nsites;
-  const int nx = P.nx, ny = P.ny, nz = P.nz;
+  const double *psi_b_ = psi + N, *psi_s_ = psi + 2 * N, *db1 = db + N, *db2 = db + 2 * N;
   double f_br[3] = {0, 0, 0}, f_rb[3] = {0, 0, 0}, f_cs[3] = {0, 0, 0}, f_sc[3] = {0, 0, 0},
          f_ss[3] = {0, 0, 0};
   const double dbx[3] = {db[i], db[N + i], db[2 * N + i]};
 #pragma unroll
   for (int q = 0; q < 18; ++q) {
-    long long j = sidx(wrap(x + cx(q), nx), wrap(y + cy(q), ny), wrap(z + cz(q), nz), nx, ny);
+    const unsigned j = nb.at<1>(q);
     const int c[3] = {cx(q), cy(q), cz(q)};
     const double g = (double)gw(q);
-    double psi_r = psi[j];
-    double psi_b = psi[N + j];
+    double psi_r = ld(psi, j);
+    double psi_b = ld(psi_b_, j);
     double green_r = psi_b * g;
     double green_b = psi_r * g;
     for (int k = 0; k < 3; ++k) {
@@ -517,8 +545,8 @@ __device__ __forceinline__ void sc_force_ternary(const DevParams &P, int x, int 
       f_rb[k] = f_rb[k] + green_r * (double)c[k];
       f_br[k] = f_br[k] + green_b * (double)c[k];
     }
-    double pss = psi[2 * N + j];
-    double dd[3] = {db[j] * pss, db[N + j] * pss, db[2 * N + j] * pss};
+    double pss = ld(psi_s_, j);
+    double dd[3] = {ld(db, j) * pss, ld(db1, j) * pss, ld(db2, j) * pss};
     double d_dotc = cdot(c, dd);
     for (int k = 0; k < 3; ++k)
       f_cs[k] = f_cs[k] + (c[k] ? dd[k] - (2.0 * d_dotc) * (double)c[k] : dd[k]) * g;
@@ -557,7 +585,7 @@ __device__ __forceinline__ void sc_forces(const DevParams &P, int x, int y, int 
   if (NC == 2)
     sc_force_binary<LE, ROCK>(P, x, y, z, i, rho, psi, rock, plo, phi, F[0], F[1]);
   else
-    sc_force_ternary(P, x, y, z, i, psi, db, F[0], F[1], F[NC - 1]);
+    sc_force_ternary(P, Nb(x, y, z, P.nx, P.ny, P.nz), i, psi, db, F[0], F[1], F[NC - 1]);
 }
 
 // ---------------------------------------------------------------------------
