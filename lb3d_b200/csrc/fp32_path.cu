@@ -904,12 +904,21 @@ static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool 
   return eq_kernel(pass, first, P.nc, rock, s.le_h[0] != nullptr, ax, ay, 19ull * P.nc * s.S < (1ull << 32), k);
 }
 
+// Sheared lattices of at least this many sites run the halo kernels and the
+// moments of the tiles on the sheared boundary beside those of the others.
+static bool eq_forks(const DevParams &P) { return P.le && P.nsites >= (1LL << 20); }
+
 // One step of strategy 3: the moments pass (ternary: two of them after the
-// first step of a loop), the dipole pass (ternary) and the collide pass, each on its own tile list and resident grid; with le (a
-// binary Lees-Edwards lattice) the stage-6 halo kernel runs before the
-// moments pass and the stage-8 one before the collide pass.  Lattices with
-// rock launch plainly: the overlap of programmatic dependent launch measured
-// 0.8 % slower on the porous lattice, 0.9-1 % faster on the others.
+// first step of a loop), the dipole pass (ternary) and the collide pass, each on
+// its own tile list and resident grid; with le (a binary Lees-Edwards lattice)
+// the stage-6 halo kernel runs before the moments pass and the stage-8 one
+// before the collide pass.  The halo kernels, bound by FP64 latency at 12 % of
+// the issue slots, concern only the tiles on the sheared boundary (eq_edge of
+// the moments tiles, at the end of the list): a large lattice runs halo,
+// boundary tiles and halo on the copy stream while the other tiles run on st.
+// Lattices with rock launch plainly: the overlap of programmatic dependent
+// launch measured 0.8 % slower on the porous lattice, 0.9-1 % faster on the
+// others.
 static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rockp, bool first, bool last,
                            const LEStep *le, cudaStream_t st) {
   if (le && !s.le_h[0]) return cudaErrorInvalidValue;
@@ -922,18 +931,39 @@ static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rock
   a.mask = s.mask;
   a.X = EqFields{s.M, P.nc == 3 ? s.psi : reinterpret_cast<float2 *>(s.M), s.o1, s.o3, s.o2,
                  {reinterpret_cast<float4 *>(s.f[0]), reinterpret_cast<float4 *>(s.f[1])}, (unsigned)s.S};
-  for (int pass = 0; pass < EQ_PASSES; ++pass) {
+  const bool fork = le && eq_forks(P);
+  cudaError_t e = cudaSuccess;
+  for (int pass = 0; pass < EQ_PASSES && e == cudaSuccess; ++pass) {
     EqKernel k;
     if (!eq_kernel_of(P, s, pass, first, s.tx, s.ty, &k)) continue;
-    if (le && pass == EQ_MOMENTS) k_le_pre32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
-    if (le && pass == EQ_COLLIDE) k_le_post32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
     a.tiles = s.eq_tiles + s.eq_off[pass];
     a.ntiles = s.eq_ntiles[pass];
-    if ((e = eq_launch(k, pass, first, last, a, !rock, st)) != cudaSuccess) return e;
+    if (fork && pass == EQ_MOMENTS) {
+      // xev[0]: the previous step is done; xev[1]: the boundary's part is done
+      if ((e = cudaEventRecord(s.xev[0], st)) != cudaSuccess) break;
+      if ((e = cudaStreamWaitEvent(s.xs, s.xev[0], 0)) != cudaSuccess) break;
+      k_le_pre32<2><<<leg, 64, 0, s.xs>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+      EqArgs edge = a;
+      edge.tiles = a.tiles + (a.ntiles - s.eq_edge);
+      edge.ntiles = s.eq_edge;
+      a.ntiles -= s.eq_edge;
+      if ((e = cudaGetLastError()) == cudaSuccess) e = eq_launch(k, pass, first, last, edge, false, s.xs);
+      if (e != cudaSuccess) break;
+      k_le_post32<2><<<leg, 64, 0, s.xs>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+      if ((e = cudaGetLastError()) != cudaSuccess) break;
+      if ((e = cudaEventRecord(s.xev[1], s.xs)) != cudaSuccess) break;
+      if (a.ntiles) e = eq_launch(k, pass, first, last, a, false, st);
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(st, s.xev[1], 0);
+      continue;
+    }
+    if (le && !fork && pass == EQ_MOMENTS)
+      k_le_pre32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+    if (le && !fork && pass == EQ_COLLIDE)
+      k_le_post32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
+    if ((e = cudaGetLastError()) == cudaSuccess)
+      e = eq_launch(k, pass, first, last, a, !rock && !(fork && pass == EQ_COLLIDE), st);
   }
-  return cudaSuccess;
+  return e;
 }
 
 // The z chunking of one pass of strategy 3: nxy column tiles, `resident`
@@ -989,6 +1019,11 @@ static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
         }
     }
     s.eq_ntiles[pass] = (int)all.size() - s.eq_off[pass];
+    if (pass == EQ_MOMENTS && eq_forks(P)) {
+      auto inner = [&](const Tile &t) { return t.x0 != 0 && t.x0 + tx < L.nx; };
+      const auto end = std::stable_partition(all.begin() + s.eq_off[pass], all.end(), inner);
+      s.eq_edge = (int)(all.end() - end);
+    }
   }
   if (s.eq_tiles) cudaFree(s.eq_tiles);
   s.eq_tiles = nullptr;
