@@ -316,11 +316,17 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
   }
   const bool part = tid < AN;
   const int s = hx + AW * hy;
+  // The first tile, its descriptor and offsets are set up before the previous
+  // pass has finished: no pass of a loop writes them (the flip of the loop
+  // before completed before the loop's first pass could start).  A step of
+  // ternary 16^3 24.6 -> 15.2 us, 32^3 29.3 -> 19.5, 64^3 48.9 -> 39.8, 128^3
+  // 214 -> 202.
+  const Tile T0 = tiles[blockIdx.x];
+  if (tid == 0) sLat = lats[T0.lat];
   pdl_launch_next();
-  pdl_wait_previous();
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile T = tiles[t];
-    if (tid == 0) sLat = lats[T.lat];
+    const Tile T = t == blockIdx.x ? T0 : tiles[t];
+    if (tid == 0 && t != blockIdx.x) sLat = lats[T.lat];
     cta_barrier<NTH>();
     const LatDesc &Lg = sLat;
     const int nx = Lg.nx, ny = Lg.ny, nz = Lg.nz, pl = nx * ny;
@@ -357,6 +363,7 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
       const float *h = Lg.le_h[side] + wy + ny * z;
       return make_float2(h[d * NP], h[(19 + d) * NP]);
     };
+    pdl_wait_previous();  // from here on, data of earlier passes
     if (part) load(0);
     cp_async_commit();
     if (tid >= NT) {
@@ -587,11 +594,13 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
   __shared__ LatDesc sLat;
   const unsigned S = X.S;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  // the first tile early, as in the moments pass
+  const Tile T0 = tiles[blockIdx.x];
+  if (tid == 0) sLat = lats[T0.lat];
   pdl_launch_next();
-  pdl_wait_previous();
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile T = tiles[t];
-    if (tid == 0) sLat = lats[T.lat];
+    const Tile T = t == blockIdx.x ? T0 : tiles[t];
+    if (tid == 0 && t != blockIdx.x) sLat = lats[T.lat];
     __syncthreads();
     const LatDesc &Lg = sLat;
     const int nx = Lg.nx, ny = Lg.ny, nz = Lg.nz, pl = nx * ny;
@@ -617,6 +626,7 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
       for (int e = 0; e < RE; ++e)
         if (tid + e * NT < AN) cp_async16(slot + tid + e * NT, plane + rxy[e]);
     };
+    pdl_wait_previous();  // from here on, data of earlier passes
     load_ring(0);
     load_ring(1);
     load_ring(2);
@@ -802,11 +812,13 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
   __shared__ LatDesc sLat;
   const unsigned S = X.S;
   const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
+  // the first tile early, as in the moments pass
+  const Tile T0 = tiles[blockIdx.x];
+  if (tid == 0) sLat = lats[T0.lat];
   pdl_launch_next();
-  pdl_wait_previous();
   for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const Tile T = tiles[t];
-    if (tid == 0) sLat = lats[T.lat];
+    const Tile T = t == blockIdx.x ? T0 : tiles[t];
+    if (tid == 0 && t != blockIdx.x) sLat = lats[T.lat];
     __syncthreads();
     const LatDesc &Lg = sLat;
     const int nx = Lg.nx, ny = Lg.ny, nz = Lg.nz, pl = nx * ny;
@@ -858,6 +870,7 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
         }
       }
     };
+    pdl_wait_previous();  // from here on, data of earlier passes
     load_ring(0);
     load_ring(1);
     load_ring(2);
@@ -1062,11 +1075,12 @@ bool eq_kernel(int pass, bool first, int nc, bool rock, bool le, int tx, int ty,
 }
 
 cudaError_t eq_launch(const EqKernel &k, int pass, bool first, bool last, const EqArgs &a, bool pdl, cudaStream_t st) {
+  if (a.ntiles <= 0) return cudaSuccess;  // every CTA reads a tile
   int resident = 0;
   cudaError_t e = fp32_prepare_kernel(k.fn, k.threads, k.smem, &resident);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)std::max(1, std::min(a.ntiles, resident)));
+  cfg.gridDim = dim3((unsigned)std::min(a.ntiles, resident));
   cfg.blockDim = dim3((unsigned)k.threads);
   cfg.dynamicSmemBytes = k.smem;
   cfg.stream = st;
