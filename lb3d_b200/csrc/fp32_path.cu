@@ -1,4 +1,6 @@
-// fp32_path.cu -- FP32 deviation storage, one fused stream-collide pass.
+// fp32_path.cu -- FP32 deviation storage: the fused stream-collide pass, and the
+// host side of every FP32 strategy (fp32_split.cuh: strategies 1 and 2,
+// fp32_eqstate.cu: strategy 3).
 //
 // Populations are stored as FP32 deviations delta_{c,i} = n_{c,i} - w_i rho0
 // from the rest state (w_i = 1/36 moving, 1/3 rest), so the stored values
@@ -1346,6 +1348,8 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   // keep the launch shape chosen so far (set or autotuned); the kernel
   // variant may change with the rock flag
   int rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, s.split}, st);
+  if (rc == LB3DC_ENOMEM && s.split == 3)  // no room for the neighbour mask
+    rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, 2}, st);
   if (rc) return rc;
   (void)p;
   return cudaStreamSynchronize(st) == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;
