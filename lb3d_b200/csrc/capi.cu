@@ -642,7 +642,7 @@ int lb3dc_time_loop(lb3dc_handle *h, int nsteps) {
       }
       h->timer.start(h->stream);
       CK(h, fp64_step_pull(h->P, h->f, h->g, h->rho, h->psi, h->mom, h->da, h->db, h->rock,
-                           h->stream, h->le ? &le : nullptr));
+                           h->stream, h->le ? &le : nullptr, h->le || s > 0));
       h->timer.stop(h->stream);
       h->timer.launches += fp64_stream_launches(h->P) + (h->p.ncomp == 3 ? 1 : 0) + (h->le ? 1 : 0) + 1;
       std::swap(h->f, h->g);

@@ -123,6 +123,19 @@ LB3D_HDI bool in_accn_box(const DevParams &P, int x1, int y1, int z1) {
          (x1 <= P.g_accn_max_x) && (y1 >= P.g_accn_min_y) && (y1 <= P.g_accn_max_y);
 }
 
+#ifdef __CUDACC__
+// Programmatic dependent launch between the kernels of a step: each lets the
+// next one launch once all its CTAs are running, and waits for the previous
+// grid to complete, with its memory visible, before it reads or writes what
+// that grid touched.  Data that a grid still running may write is read with
+// plain loads, not through const __restrict__ pointers (read-only loads).
+// Without the launch attribute both are no-ops.
+__device__ __forceinline__ void pdl_launch_next() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+}
+__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+#endif
+
 }  // namespace lb3d
 
 #endif

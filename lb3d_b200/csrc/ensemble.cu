@@ -1,11 +1,12 @@
-// ensemble.cu -- many independent lattices advanced by one persistent
-// kernel over a packed site index (the batched FP32 deviation path).
+// ensemble.cu -- many independent lattices advanced by shared launches over a
+// packed site index (the batched FP32 deviation path).
 //
 // Every lattice occupies a contiguous range [base, base + N) of one packed
 // site space of capacity S; its populations live at f[(c*19+q)*S + base + i]
 // like a single lattice's.  A lattice table (LatDesc: size, parameters,
-// parity) and a tile list covering every active lattice drive the same fused
-// stream-collide kernel as the single-lattice path, so a lattice advances
+// parity) and a tile list covering every active lattice drive the same passes
+// as the single-lattice path (strategy 3 when every active lattice relaxes
+// fully, else strategy 2), so a lattice advances
 // exactly as it would alone (the per-site arithmetic does not depend on which
 // tiles or lattices share a launch).  Site ranges are handed out first-fit;
 // admission fails with LB3DC_ENOMEM when no range fits, which is how the

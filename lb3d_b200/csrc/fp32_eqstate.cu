@@ -42,16 +42,6 @@
 namespace lb3d {
 namespace f32 {
 
-// Programmatic dependent launch between the passes: each pass lets the next
-// one launch once all its CTAs are running, and waits for the previous grid
-// to complete, with its memory visible, before it reads anything that grid or
-// an earlier one wrote (with plain loads: the data changes during the kernel's
-// lifetime).  Without the launch attribute both are no-ops.
-__device__ __forceinline__ void pdl_launch_next() {
-  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
-}
-__device__ __forceinline__ void pdl_wait_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
-
 // Plane class of a direction and its index within the class: D (c_z = -1),
 // Z (c_z = 0), U (c_z = +1).  The two directions along z (4, 5) are pulled
 // by the thread that evaluated them and never leave its registers.

@@ -128,7 +128,7 @@ void fp32_tiles_for(const LatDesc &L, int lat_id, const FusedShape &sh, std::vec
 // Each pass runs as many CTAs as are resident at once for that kernel (at
 // most ntiles); max_grid > 0 caps that number.
 // With le (a binary single lattice whose LatDesc carries the halo planes,
-// strategy 2 only) the step also builds the sheared x-halos: the stage-6
+// strategy 2) the step also builds the sheared x-halos: the stage-6
 // populations before the moments pass and the stage-8 psi planes before the
 // collide pass.
 cudaError_t fp32_launch_fused(int nc, bool rock, bool body, const FusedShape &sh,

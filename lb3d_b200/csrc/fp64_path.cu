@@ -75,12 +75,14 @@ __device__ __forceinline__ double ld(const double *__restrict__ p, unsigned byte
 // one side a thread in 64-thread blocks 16-17 us, both sides a thread in
 // 128-thread blocks 20 and 24 us (97x66x63 sites).
 template <int NC, bool COMPACT>
-__global__ void __launch_bounds__(64) k_le_halo(DevParams P, LEStep S, const double *__restrict__ src,
+__global__ void __launch_bounds__(64) k_le_halo(DevParams P, LEStep S, const double *src,
                           double *__restrict__ hlo, double *__restrict__ hhi,
                           double *__restrict__ rlo, double *__restrict__ rhi,
                           double *__restrict__ plo, double *__restrict__ phi) {
   const int nx = P.nx, ny = P.ny, nz = P.nz, NPi = ny * nz;
   const int u = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait_previous();
+  pdl_launch_next();
   if (u >= 2 * NPi) return;
   const bool top = u >= NPi;
   const int t = top ? u - NPi : u;
@@ -140,14 +142,14 @@ __global__ void __launch_bounds__(64) k_le_halo(DevParams P, LEStep S, const dou
 // only, and under Lees-Edwards the populations of the x boundary planes
 // ([2][NC][19][nz][ny], x = nx - 1 and x = 0) to fout for the stage-8 halo.
 template <int NC, bool LE, bool FLUX, bool ROCK, bool STORE = true>
-__global__ void __launch_bounds__(256, FLUX ? 3 : 2) k_stream(DevParams P, const double *__restrict__ fin,
+__global__ void __launch_bounds__(256, FLUX ? 3 : 2) k_stream(DevParams P, const double *fin,
                                                 double *__restrict__ fout, double *__restrict__ rho,
                                                 double *__restrict__ psi, double *__restrict__ mom,
                                                 double *__restrict__ da,
-                                                const double *__restrict__ db,
+                                                const double *db,
                                                 const uint8_t *__restrict__ rock,
-                                                const double *__restrict__ hlo,
-                                                const double *__restrict__ hhi, int c0) {
+                                                const double *hlo,
+                                                const double *hhi, int c0) {
   const int c = c0 + blockIdx.y;
   const long long N = P.nsites;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -189,6 +191,8 @@ __global__ void __launch_bounds__(256, FLUX ? 3 : 2) k_stream(DevParams P, const
     return src;
   };
 
+  pdl_wait_previous();  // from here on, data of earlier kernels
+  pdl_launch_next();
   double d0 = 0.0, d1 = 0.0, d2 = 0.0;
   {
     double n[19];
@@ -380,8 +384,9 @@ __global__ void k_recolour(DevParams P, double *__restrict__ g, const uint8_t *_
 
 // c . v of a lattice direction, the products and sums in axis order.  Terms of
 // a zero component are left out here and in the sums over directions below:
-// adding +-0 changes no finite value (the FP64 pipe bounds these kernels, and
-// the compiler may not drop a product with 0 by itself).
+// adding +-0 changes no finite value, and the compiler may not drop a product
+// with 0 by itself.  60 % of the components are zero; ternary 128^3, a step:
+// 0.830 -> 0.792 ms.
 __device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
   double r = 0.0;
   bool any = false;
@@ -400,8 +405,8 @@ __device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
 // Reads rho and da of the 18 neighbours; writes db in place (no neighbour
 // reads db in this pass).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *__restrict__ rho,
-                                                const double *__restrict__ da,
+__global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *rho,
+                                                const double *da,
                                                 double *__restrict__ db) {
   const long long N = P.nsites;
   long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -411,6 +416,8 @@ __global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *__
   site_xyz(i, nx, ny, x, y, z);
   const Nb nb(x, y, z, nx, ny, nz);
   const double *rho_b = rho + N, *da1 = da + N, *da2 = da + 2 * N;
+  pdl_wait_previous();
+  pdl_launch_next();
   double h_c[3] = {0.0, 0.0, 0.0};
   double h_s[3] = {da[i], da[N + i], da[2 * N + i]};
   double sN_tmp = fmaxf_(rho[2 * N + i], CLIP_RHO_S);
@@ -604,13 +611,13 @@ __device__ __forceinline__ void sc_forces(const DevParams &P, int x, int y, int 
 template <int NC, bool LE, bool PULL = false, bool ROCK = true>
 __global__ void __launch_bounds__(256, (PULL && ROCK && NC == 2) ? 3 : ((PULL || NC == 3) ? 2 : 4)) k_collide(DevParams P, const double *__restrict__ g,
                                                  double *__restrict__ f,
-                                                 const double *__restrict__ rho,
-                                                 const double *__restrict__ psi,
-                                                 const double *__restrict__ mom,
-                                                 const double *__restrict__ db,
+                                                 const double *rho,
+                                                 const double *psi,
+                                                 const double *mom,
+                                                 const double *db,
                                                  const uint8_t *__restrict__ rock,
-                                                 const double *__restrict__ plo,
-                                                 const double *__restrict__ phi,
+                                                 const double *plo,
+                                                 const double *phi,
                                                  const double *__restrict__ hlo = nullptr,
                                                  const double *__restrict__ hhi = nullptr) {
   const long long N = P.nsites;
@@ -619,6 +626,8 @@ __global__ void __launch_bounds__(256, (PULL && ROCK && NC == 2) ? 3 : ((PULL ||
   int x, y, z;
   site_xyz(i, P.nx, P.ny, x, y, z);
   double F[NC][3];
+  pdl_wait_previous();
+  pdl_launch_next();
   sc_forces<NC, LE, ROCK>(P, x, y, z, i, rho, psi, db, rock, plo, phi, F);
   double r[NC];
   for (int c = 0; c < NC; ++c) r[c] = rho[c * N + i];
@@ -826,16 +835,36 @@ static inline unsigned grid_for(long long n, int bs) { return (unsigned)((n + bs
 using namespace fp64;
 
 
+// A kernel launch; pdl: the kernel may start while the one launched before it
+// on the stream, one of those below, drains.  Each kernel waits for the
+// previous grid first and lets the next one launch after that, so only
+// neighbours overlap: the populations that k_collide pulls were complete before
+// it could start and stay read-only loads (as plain loads, which may not pass
+// the stores before them, they took the step of ternary 128^3 from 0.76 to 1.35
+// ms); the fields of the kernel just before are plain loads.  A step, before ->
+// after: ternary 16^3 24.3 -> 19.8 us, 32^3 27.1 -> 26.0, binary 64^3 59.2 ->
+// 57.3, sheared 97x66x63 155 -> 144, ternary 128^3 758 -> 753.
+template <typename... K, typename... A>
+static cudaError_t launch(void (*k)(K...), dim3 grid, int block, cudaStream_t st, bool pdl, A... a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<K>(a)...);
+}
+
 cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, bool compact, double *hlo,
                          double *hhi, double *rlo, double *rhi, double *plo, double *phi,
-                         cudaStream_t st) {
+                         cudaStream_t st, bool pdl) {
   const unsigned g = grid_for(2LL * P.ny * P.nz, 64);
   if (P.nc != 2) return cudaErrorInvalidValue;
-  if (compact)
-    k_le_halo<2, true><<<g, 64, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
-  else
-    k_le_halo<2, false><<<g, 64, 0, st>>>(P, S, src, hlo, hhi, rlo, rhi, plo, phi);
-  return cudaGetLastError();
+  return launch(compact ? k_le_halo<2, true> : k_le_halo<2, false>, dim3(g), 64, st, pdl, P, S, src, hlo, hhi, rlo,
+                rhi, plo, phi);
 }
 
 // Threads per block of the site kernels.  Small lattices take small blocks,
@@ -855,27 +884,22 @@ static bool fp64_small(const DevParams &P) { return P.nsites <= 65536; }
 template <bool STORE>
 static cudaError_t launch_stream(const DevParams &P, const double *fin, double *fout, double *rho, double *psi,
                                  double *mom, double *da, const double *db, const uint8_t *rock, const double *hlo,
-                                 const double *hhi, cudaStream_t st) {
+                                 const double *hhi, cudaStream_t st, bool pdl = false, bool chain = false) {
   const int bs = fp64_block(P);
   const unsigned gr = grid_for(P.nsites, bs);
-#define LB3D_STREAM(NC_, LE_, FLUX_, ny_, c_)                                                        \
-  (P.any_rock ? k_stream<NC_, LE_, FLUX_, true, STORE><<<dim3(gr, ny_), bs, 0, st>>>(                 \
-                    P, fin, fout, rho, psi, mom, da, db, rock, hlo, hhi, c_)                          \
-              : k_stream<NC_, LE_, FLUX_, false, STORE><<<dim3(gr, ny_), bs, 0, st>>>(                \
-                    P, fin, fout, rho, psi, mom, da, db, rock, hlo, hhi, c_))
-  if (P.nc == 2) {
-    if (P.le)
-      LB3D_STREAM(2, true, false, 2, 0);
-    else
-      LB3D_STREAM(2, false, false, 2, 0);
-  } else if (fp64_small(P)) {
-    LB3D_STREAM(3, false, true, 3, 0);
-  } else {
-    LB3D_STREAM(3, false, false, 2, 0);
-    LB3D_STREAM(3, false, true, 1, 2);
-  }
-#undef LB3D_STREAM
-  return cudaGetLastError();
+  auto go = [&](auto rocky, auto plain, unsigned ny, int c0) {
+    const cudaError_t e = launch(P.any_rock ? rocky : plain, dim3(gr, ny), bs, st, pdl, P, fin, fout, rho, psi, mom,
+                                 da, db, rock, hlo, hhi, c0);
+    pdl = chain;
+    return e;
+  };
+  if (P.nc == 2)
+    return P.le ? go(k_stream<2, true, false, true, STORE>, k_stream<2, true, false, false, STORE>, 2, 0)
+                : go(k_stream<2, false, false, true, STORE>, k_stream<2, false, false, false, STORE>, 2, 0);
+  if (fp64_small(P)) return go(k_stream<3, false, true, true, STORE>, k_stream<3, false, true, false, STORE>, 3, 0);
+  const cudaError_t e = go(k_stream<3, false, false, true, STORE>, k_stream<3, false, false, false, STORE>, 2, 0);
+  return e != cudaSuccess ? e
+                          : go(k_stream<3, false, true, true, STORE>, k_stream<3, false, true, false, STORE>, 1, 2);
 }
 
 int fp64_stream_launches(const DevParams &P) { return P.nc == 2 || fp64_small(P) ? 1 : 2; }
@@ -913,38 +937,33 @@ cudaError_t fp64_stream(const DevParams &P, const double *fin, double *fout, dou
 
 cudaError_t fp64_step_pull(const DevParams &P, const double *fin, double *fout, double *rho,
                            double *psi, double *mom, double *da, double *db, const uint8_t *rock,
-                           cudaStream_t st, const Fp64Le *le) {
+                           cudaStream_t st, const Fp64Le *le, bool chained) {
   if (P.zouhe || (P.le != 0) != (le != nullptr)) return cudaErrorInvalidValue;
   const int bs = fp64_block(P);
   const unsigned gr = grid_for(P.nsites, bs);
   const bool rk = P.any_rock != 0;
   // moments pass: densities, psi, momenta and (surfactant) the advected dipole flux
   cudaError_t e = launch_stream<false>(P, fin, le ? le->post : nullptr, rho, psi, mom, da, db, rock,
-                                       le ? le->hlo : nullptr, le ? le->hhi : nullptr, st);
-  if (e == cudaSuccess && P.nc == 3) e = fp64_dipole(P, rho, da, db, st);
+                                       le ? le->hlo : nullptr, le ? le->hhi : nullptr, st, chained, true);
+  if (e == cudaSuccess && P.nc == 3) e = fp64_dipole(P, rho, da, db, st, true);
   if (e == cudaSuccess && le)
-    e = fp64_le_halo(P, le->step, le->post, true, nullptr, nullptr, le->rlo, le->rhi, le->plo, le->phi, st);
+    e = fp64_le_halo(P, le->step, le->post, true, nullptr, nullptr, le->rlo, le->rhi, le->plo, le->phi, st, true);
   if (e != cudaSuccess) return e;
   const double *plo = le ? le->plo : nullptr, *phi = le ? le->phi : nullptr;
   const double *hlo = le ? le->hlo : nullptr, *hhi = le ? le->hhi : nullptr;
-#define LB3D_PULL(NC_, LE_)                                                                                    \
-  (rk ? k_collide<NC_, LE_, true, true><<<gr, bs, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, plo, phi, hlo, hhi) \
-      : k_collide<NC_, LE_, true, false><<<gr, bs, 0, st>>>(P, fin, fout, rho, psi, mom, db, rock, plo, phi, hlo, hhi))
-  if (P.nc == 3)
-    LB3D_PULL(3, false);
-  else if (le)
-    LB3D_PULL(2, true);
-  else
-    LB3D_PULL(2, false);
-#undef LB3D_PULL
-  return cudaGetLastError();
+  auto go = [&](auto rocky, auto plain) {
+    return launch(rk ? rocky : plain, dim3(gr), bs, st, true, P, fin, fout, rho, psi, mom, db, rock, plo, phi, hlo,
+                  hhi);
+  };
+  if (P.nc == 3) return go(k_collide<3, false, true, true>, k_collide<3, false, true, false>);
+  if (le) return go(k_collide<2, true, true, true>, k_collide<2, true, true, false>);
+  return go(k_collide<2, false, true, true>, k_collide<2, false, true, false>);
 }
 
 cudaError_t fp64_dipole(const DevParams &P, const double *rho, const double *da, double *db,
-                        cudaStream_t st) {
+                        cudaStream_t st, bool pdl) {
   const int bs = fp64_block(P);
-  k_dipole<<<grid_for(P.nsites, bs), bs, 0, st>>>(P, rho, da, db);
-  return cudaGetLastError();
+  return launch(k_dipole, dim3(grid_for(P.nsites, bs)), bs, st, pdl, P, rho, da, db);
 }
 
 cudaError_t fp64_collide(const DevParams &P, const double *g, double *f, const double *rho,

@@ -11,7 +11,7 @@ namespace lb3d {
 // densities and psi when rlo is given; binary lattices.
 cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src, bool compact, double *hlo,
                          double *hhi, double *rlo, double *rhi, double *plo, double *phi,
-                         cudaStream_t st);
+                         cudaStream_t st, bool pdl = false);
 // Zou-He flux boundaries on the z = 1 and z = nz planes (inv_fluid 12),
 // applied to the post-stream populations g and the advected dipole flux da.
 cudaError_t fp64_zouhe_density(const DevParams &P, double *g, const uint8_t *rock, double fr,
@@ -39,12 +39,14 @@ struct Fp64Le {
 // dipole flux), dipole relaxation (ternary), stage-8 halo (Lees-Edwards), pull
 // + forces + BGK from fin into fout.  Every buffer ends up as after fp64_stream
 // + fp64_dipole + fp64_collide, bit for bit, except that the post-stream
-// populations are never stored.
+// populations are never stored.  The kernels of a step follow each other with
+// programmatic dependent launch; chained: the kernel launched before on the
+// stream is one of this step's kind, and the first one follows it so, too.
 cudaError_t fp64_step_pull(const DevParams &P, const double *fin, double *fout, double *rho,
                            double *psi, double *mom, double *da, double *db, const uint8_t *rock,
-                           cudaStream_t st, const Fp64Le *le = nullptr);
+                           cudaStream_t st, const Fp64Le *le = nullptr, bool chained = false);
 cudaError_t fp64_dipole(const DevParams &P, const double *rho, const double *da, double *db,
-                        cudaStream_t st);
+                        cudaStream_t st, bool pdl = false);
 cudaError_t fp64_collide(const DevParams &P, const double *g, double *f, const double *rho,
                          const double *psi, const double *mom, const double *db,
                          const uint8_t *rock, const double *plo, const double *phi,

@@ -149,7 +149,7 @@ extern "C" int lb3dc_time_loop_fp64_noalloc(const lb3dc_params *p, double *f, do
   // odd number of them the populations are copied back.
   double *in = f, *out = g;
   for (int s = 0; s < nsteps; ++s) {
-    e = lb3d::fp64_step_pull(P, in, out, rho, psi, mom, da, db, rk, st);
+    e = lb3d::fp64_step_pull(P, in, out, rho, psi, mom, da, db, rk, st, nullptr, s > 0);
     if (e != cudaSuccess) return err(LB3DC_ECUDA, cudaGetErrorString(e));
     std::swap(in, out);
   }
