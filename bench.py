@@ -38,11 +38,11 @@ BYTES_PER_SITE = {("f32", 3): 480, ("f32", 2): 304, ("f64", 3): 960, ("f64", 2):
 # DRAM bytes per site and step that ncu measured (dram__bytes_read.sum +
 # dram__bytes_write.sum summed over the step's passes) on the ternary 128^3
 # workload: strategy 2 (moments, dipole and staged collide passes; 32x4
-# tiles, 8-plane chunks) and strategy 3 (moments, dipole and TMA-fed collide
-# passes; 32x8 tiles).  Keyed by (tile x, tile y, strategy); for strategy 3
-# the tile shape moves only halo reloads that hit L2, so its figure stands
-# for every shape.
-NCU_TRAFFIC_PER_SITE = {(32, 4, 2): 772, (32, 8, 3): 561}
+# tiles, 8-plane chunks) and strategy 3 (two moments passes, dipole and
+# collide passes, a step within a loop; 16x8 tiles).  Keyed by (tile x, tile y,
+# strategy); for strategy 3 the tile shape moves only halo reloads that hit
+# L2, so its figure stands for every shape.
+NCU_TRAFFIC_PER_SITE = {(32, 4, 2): 772, (16, 8, 3): 258}
 
 
 def ncu_traffic(shape):
@@ -50,10 +50,10 @@ def ncu_traffic(shape):
     if key in NCU_TRAFFIC_PER_SITE:
         return NCU_TRAFFIC_PER_SITE[key]
     if shape[3] == 3:
-        return NCU_TRAFFIC_PER_SITE[(32, 8, 3)]
+        return NCU_TRAFFIC_PER_SITE[(16, 8, 3)]
     return None
 PHYS = dict(tau_d=1.0, g_br=0.08, g_bs=-0.006, g_ss=-0.0045, beta=10.0, d_0=1.0, bdist=2, restore=1)
-STRATEGIES = ["fused", "split", "split, staged collide", "moment field, TMA-fed collide"]
+STRATEGIES = ["fused", "split", "split, staged collide", "equilibrium arguments carried"]
 
 
 def measured_peak():

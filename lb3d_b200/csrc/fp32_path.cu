@@ -1056,9 +1056,9 @@ static void attach_le(Fp32State &s) {
 
 // Shape before any autotuning.  Fully relaxing lattices: strategy 3 with 16x8
 // tiles, the fastest or within 3 % of it on every lattice measured (ternary
-// 32^3, 64^3, 75x67x87, 128^3: 0.029, 0.049, 0.070, 0.213 ms a step against
-// 0.058, 0.082, 0.126, 0.383 for strategy 2; binary 256x128x128 0.161 against
-// 0.418, sheared 0.288 against 0.536, porous 192^3 0.268 against 0.911).
+// 32^3, 64^3, 75x67x87, 128^3: 0.019, 0.040, 0.062, 0.202 ms a step against
+// 0.058, 0.082, 0.126, 0.384 for strategy 2; binary 256x128x128 0.157 against
+// 0.432, sheared 0.214 against 0.565, porous 192^3 0.273 against 0.924).
 // Others: the split strategy with the staged collide pass, the fastest of 0 to
 // 2.
 static FusedShape default_shape(const DevParams &P) {
