@@ -32,7 +32,7 @@ extern "C" {
 #define LB3DC_EINVAL (-22)   /* bad argument or unsupported parameter set */
 #define LB3DC_ENOMEM (-12)   /* device or host allocation failed          */
 #define LB3DC_ECUDA (-5)     /* a CUDA runtime call failed                */
-#define LB3DC_ETIMEOUT (-110)/* a bounded device-side wait gave up        */
+#define LB3DC_ETIMEOUT (-110)/* kept for callers; no kernel reports it now */
 #define LB3DC_ENAN (-33)     /* non-finite populations detected           */
 #define LB3DC_ENOTSUP (-95)  /* valid request this build does not support */
 #define LB3DC_ESTATE (-71)   /* call out of order (e.g. no state loaded)  */
@@ -146,10 +146,10 @@ int lb3dc_advection(lb3dc_handle *h);
 int lb3dc_collision(lb3dc_handle *h);
 /* nsteps full time steps (stages 6..9 each); may fuse stages.  The FP64
  * path pulls the post-stream populations inside its collision kernel where
- * nothing acts on them between advection and collision (no Lees-Edwards
- * planes, no inflow boundaries): the results, rho, psi, the momenta and the
- * dipole flux included, are those of the stage-by-stage calls bit for
- * bit. */
+ * no inflow boundary acts on them between advection and collision: the
+ * results, rho, psi, the momenta and the dipole flux included, are those of
+ * the stage-by-stage calls bit for bit.  The FP32 path's strategy 3 (below)
+ * holds populations before and after the call, not between its steps. */
 int lb3dc_time_loop(lb3dc_handle *h, int nsteps);
 /* Waits for all work of h; reports deferred kernel errors. */
 int lb3dc_sync(lb3dc_handle *h);
@@ -163,15 +163,16 @@ int lb3dc_sync(lb3dc_handle *h);
  * (48 B / 32 B), a dipole pass (ternary) and a collide pass that reads them
  * with their halo, 2 = as 1, but the collide pass stages each site's pulled
  * populations in shared memory with asynchronous copies one plane ahead
- * and sums the own moments itself (no own-moment field), 3 = a moments
- * pass writing halo-padded moment fields, a dipole pass (ternary) and a
- * collide pass that receive those fields as TMA boxes with a one-site halo,
- * the collide pass writing the equilibrium: offered only when every
- * component relaxes fully (tau = 1) on a lattice at least 2 sites across in
- * x and y without inflow boundaries (LB3DC_ENOTSUP otherwise); each of its
- * passes chunks z to fill its own resident grid, so zc is not used.
- * Lees-Edwards lattices (binary) run strategies 2 and 3 only.  All strategies give the same result up to FP32
- * rounding; 0, 1, 2 and 3 agree bit for bit (up to the sign of zero). */
+ * and sums the own moments itself (no own-moment field), 3 = moments,
+ * dipole (ternary) and collide passes that carry the arguments of the
+ * equilibrium (4 numbers per component) between the steps of one
+ * lb3dc_time_loop instead of the populations: the default where it applies,
+ * offered only when every component relaxes fully (tau = 1) on a lattice at
+ * least 2 sites across in x and y without inflow boundaries (LB3DC_ENOTSUP
+ * otherwise); each of its passes chunks z to fill its own resident grid, so
+ * zc is not used.  Lees-Edwards lattices (binary) run strategies 2 and 3
+ * only.  All strategies give the same result up to FP32 rounding; 0, 1, 2
+ * and 3 agree bit for bit (up to the sign of zero). */
 int lb3dc_set_launch_shape(lb3dc_handle *h, int tx, int ty, int zc, int split);
 int lb3dc_get_launch_shape(const lb3dc_handle *h, int *tx, int *ty, int *zc, int *split);
 /* Times every supported shape and strategy on this lattice (on a saved copy
@@ -263,7 +264,7 @@ int lb3dc_io_wait(lb3dc_handle *h);
  * Parameter sweeps (many independent small lattices of uneven size) run as
  * one ensemble: every member occupies a contiguous range of one packed,
  * device-resident site space and all active members advance together in
- * the FP32 deviation path's fused kernel over one tile list, replayed from a
+ * the FP32 deviation path's passes over one tile list, replayed from a
  * CUDA graph while the active set is unchanged.  A member's results are the
  * same alone and in any mix.  No counterpart in the reference (which runs
  * one lattice per MPI job); the per-lattice arithmetic is that of the
@@ -271,7 +272,10 @@ int lb3dc_io_wait(lb3dc_handle *h);
  */
 typedef struct lb3dc_ensemble lb3dc_ensemble;
 /* capacity_sites bounds the sum of member sizes (19*capacity < 2^32);
- * device bytes: 2*19*ncomp*4 (+24 ternary) per site of capacity. */
+ * device bytes per site of capacity: 2*19*ncomp*4 (+24 ternary), the moment
+ * field (32 ternary, 8 binary) and, while the device has room for them, the
+ * fields of strategy 3 (108, 52); without those, members that relax fully
+ * run strategy 2 like the others. */
 int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
                           lb3dc_ensemble **out);
 int lb3dc_ensemble_destroy(lb3dc_ensemble *e);
