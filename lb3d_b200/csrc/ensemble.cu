@@ -223,7 +223,9 @@ cudaError_t launch_step(lb3dc_ensemble *e, bool first, bool last) {
   for (int pass = 0; pass < EQ_PASSES; ++pass) {
     EqKernel k;
     if (!eq_kernel_of(e, pass, first, &k)) continue;
-    const cudaError_t r = eq_launch(k, pass, first, last, a, true, e->stream);
+    // the first pass of a loop launches plainly: the flip of the loop before is
+    // complete before any pass reads the descriptors
+    const cudaError_t r = eq_launch(k, pass, first, last, a, !(first && pass == EQ_MOMENTS), e->stream);
     if (r != cudaSuccess) return r;
   }
   return last ? fp32_flip_parity(e->d_lat, e->max_lat, e->stream) : cudaSuccess;

@@ -307,9 +307,9 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
   const bool part = tid < AN;
   const int s = hx + AW * hy;
   // The first tile, its descriptor and offsets are set up before the previous
-  // pass has finished: no pass of a loop writes them (the flip of the loop
-  // before completed before the loop's first pass could start).  A step of
-  // ternary 16^3 24.6 -> 15.2 us, 32^3 29.3 -> 19.5, 64^3 48.9 -> 39.8, 128^3
+  // pass has finished: no pass of a loop writes them, and what did (the flip of
+  // the loop before, an upload) completed before the loop's first pass, which is
+  // launched plainly, could start.  A step of ternary 16^3 24.6 -> 15.2 us, 32^3 29.3 -> 19.5, 64^3 48.9 -> 39.8, 128^3
   // 214 -> 202.
   const Tile T0 = tiles[blockIdx.x];
   if (tid == 0) sLat = lats[T0.lat];

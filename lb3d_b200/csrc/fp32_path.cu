@@ -918,9 +918,12 @@ static bool eq_forks(const DevParams &P) { return P.le && P.nsites >= (1LL << 20
 // the issue slots, concern only the tiles on the sheared boundary (eq_edge of
 // the moments tiles, at the end of the list): a large lattice runs halo,
 // boundary tiles and halo on the copy stream while the other tiles run on st.
-// Lattices with rock launch plainly: the overlap of programmatic dependent
-// launch measured 0.8 % slower on the porous lattice, 0.9-1 % faster on the
-// others.
+// The first pass of a loop launches plainly: everything before it on the stream,
+// the parity flip of the loop before included, is complete and visible when it
+// starts, and so when any later pass does, which is what lets those read the
+// descriptor before their own wait.  Lattices with rock launch every pass
+// plainly: the overlap of programmatic dependent launch measured 0.8 % slower on
+// the porous lattice, 0.9-1 % faster on the others.
 static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rockp, bool first, bool last,
                            const LEStep *le, cudaStream_t st) {
   if (le && !s.le_h[0]) return cudaErrorInvalidValue;
@@ -963,7 +966,8 @@ static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rock
     if (le && !fork && pass == EQ_COLLIDE)
       k_le_post32<2><<<leg, 64, 0, st>>>(P, *le, s.d_lat, s.f[0], s.f[1], a.X.S);
     if ((e = cudaGetLastError()) == cudaSuccess)
-      e = eq_launch(k, pass, first, last, a, !rock && !(fork && pass == EQ_COLLIDE), st);
+      e = eq_launch(k, pass, first, last, a,
+                    !rock && !(first && pass == EQ_MOMENTS) && !(fork && pass == EQ_COLLIDE), st);
   }
   return e;
 }
