@@ -62,8 +62,10 @@ struct Nb {
     return x[1 + SGN * cx(q)] + y[1 + SGN * cy(q)] + z[1 + SGN * cz(q)];
   }
 };
-__device__ __forceinline__ double ld(const double *__restrict__ p, unsigned byte) {
-  return __ldg(reinterpret_cast<const double *>(reinterpret_cast<const char *>(p) + byte));
+// A plain load: with programmatic dependent launch most of what it reads is
+// written by the kernel just before, which may still run when this one starts.
+__device__ __forceinline__ double ld(const double *p, unsigned byte) {
+  return *reinterpret_cast<const double *>(reinterpret_cast<const char *>(p) + byte);
 }
 
 // src: populations [NC][19][nsites], or (COMPACT) the boundary planes
@@ -462,11 +464,9 @@ __global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *rh
 // ROCK false: no site is rock.
 template <bool LE, bool ROCK>
 __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y, int z, long long i,
-                                                const double *__restrict__ rho,
-                                                const double *__restrict__ psi,
+                                                const double *rho, const double *psi,
                                                 const uint8_t *__restrict__ rock,
-                                                const double *__restrict__ plo,
-                                                const double *__restrict__ phi, double *fr,
+                                                const double *plo, const double *phi, double *fr,
                                                 double *fb) {
   const long long N = P.nsites;
   const int nx = P.nx, ny = P.ny, nz = P.nz;
@@ -530,8 +530,7 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
 }
 
 __device__ __forceinline__ void sc_force_ternary(const DevParams &P, const Nb &nb, long long i,
-                                                 const double *__restrict__ psi,
-                                                 const double *__restrict__ db, double *fr,
+                                                 const double *psi, const double *db, double *fr,
                                                  double *fb, double *fs) {
   const long long N = P.nsites;
   const double *psi_b_ = psi + N, *psi_s_ = psi + 2 * N, *db1 = db + N, *db2 = db + 2 * N;
@@ -841,7 +840,7 @@ using namespace fp64;
 // neighbours overlap: the populations that k_collide pulls were complete before
 // it could start and stay read-only loads (as plain loads, which may not pass
 // the stores before them, they took the step of ternary 128^3 from 0.76 to 1.35
-// ms); the fields of the kernel just before are plain loads.  A step, before ->
+// ms); every field of an earlier kernel of the step is a plain load.  A step, before ->
 // after: ternary 16^3 24.3 -> 19.8 us, 32^3 27.1 -> 26.0, binary 64^3 59.2 ->
 // 57.3, sheared 97x66x63 155 -> 144, ternary 128^3 758 -> 753.
 template <typename... K, typename... A>

@@ -41,6 +41,50 @@ def test_fp32_loops_back_to_back(nc, dims):
     assert np.isfinite(a["n"]).all()
 
 
+FP64 = {"ternary 16^3": (3, (16, 16, 16), {}, False), "ternary 49x40x37": (3, (49, 40, 37), {}, False),
+        "binary": (2, (40, 17, 12), {}, False),
+        "binary rock": (2, (21, 18, 16), dict(g_wr=-0.1, rock_colour_r=1.0), True),
+        "sheared": (2, (33, 18, 17), dict(boundary_cond=-1, inv_fluid=5, shear_u=0.05), False),
+        "sheared rock": (2, (18, 17, 16), dict(boundary_cond=-1, inv_fluid=5, shear_u=0.05, g_wr=-0.1), True)}
+
+
+@pytest.mark.parametrize("kind", FP64)
+def test_fp64_loops_back_to_back(kind):
+    """Both ways a step is launched (all components in one stream launch up to
+    65536 sites, two above): every field of the download, the moments and the
+    dipole flux among them."""
+    nc, dims, kw, rock = FP64[kind]
+    p, st = _params(dims, nc, 0, **kw), uniform_mixture(*dims, nc, seed=3)
+    if rock:
+        st["rock"] = (np.random.default_rng(8).random(st["n"].shape[2:]) < 0.2).astype(np.float64)
+        st["n"] = st["n"] * (1 - st["rock"])
+    a, b = _loops(p, st, True), _loops(p, st, False)
+    for f in a:
+        assert np.array_equal(a[f], b[f]), f
+    assert np.isfinite(a["n"]).all()
+
+
+@pytest.mark.parametrize("nc,dims", [(3, (16, 16, 16)), (2, (33, 20, 18))])
+def test_no_alloc_calls_back_to_back(nc, dims):
+    """Calls of one to five steps on the caller's buffers, against the handle's
+    time loop waited for after every call."""
+    import torch
+
+    from .test_zz_no_alloc import _last_error, _noalloc
+    p, st = _params(dims, nc, 0), uniform_mixture(*dims, nc, seed=3)
+    ref = _loops(p, st, True)
+    n = torch.from_numpy(np.ascontiguousarray(st["n"])).cuda()
+    db = torch.from_numpy(np.ascontiguousarray(st["db"])).cuda() if nc == 3 else None
+    stream = torch.cuda.current_stream().cuda_stream
+    for steps in LOOPS:
+        rc = _noalloc(p, n.data_ptr(), db.data_ptr() if nc == 3 else None, None, steps, stream)
+        assert rc == 0, _last_error()
+    torch.cuda.synchronize()
+    assert np.array_equal(n.cpu().numpy(), ref["n"])
+    if nc == 3:
+        assert np.array_equal(db.cpu().numpy(), ref["db"])
+
+
 def test_ensemble_chunks_back_to_back():
     """Chunks of one to three steps (enqueued pass by pass) and of four and more
     (replayed from a graph)."""
