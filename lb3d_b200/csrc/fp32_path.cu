@@ -781,10 +781,10 @@ void fp32_tiles_for(const LatDesc &L, int lat_id, const FusedShape &sh, std::vec
       for (int x0 = 0; x0 < L.nx; x0 += sh.tx) {
         Tile t;
         t.lat = lat_id;
-        t.x0 = (short)x0;
-        t.y0 = (short)y0;
-        t.z0 = (short)z0;
-        t.zc = (short)std::min(zc, L.nz - z0);
+        t.x0 = x0;
+        t.y0 = y0;
+        t.z0 = z0;
+        t.zc = std::min(zc, L.nz - z0);
         out.push_back(t);
       }
 }
@@ -1017,10 +1017,10 @@ static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
           t.lat = 0;
           // sheared lattices: the tiles on the x boundary take longer; rotated
           // by row and chunk they do not all fall to the same CTAs
-          t.x0 = (short)((P.le ? (xt + yt + c) % nxt : xt) * tx);
-          t.y0 = (short)(yt * ty);
-          t.z0 = (short)z0;
-          t.zc = (short)(z1 - z0);
+          t.x0 = (P.le ? (xt + yt + c) % nxt : xt) * tx;
+          t.y0 = yt * ty;
+          t.z0 = z0;
+          t.zc = z1 - z0;
           all.push_back(t);
         }
     }

@@ -44,11 +44,12 @@ struct LatDesc {
 };
 constexpr int LAT_ROCK = 1, LAT_BODY = 2, LAT_ACTIVE = 4;
 
-// Tile: lattice id, xy origin and z range of one CTA work item.
+// Tile: lattice id, xy origin and z range of one CTA work item (a lattice's
+// side may be as long as its number of sites).
 struct Tile {
   int lat;
-  short x0, y0;
-  short z0, zc;
+  int x0, y0;
+  int z0, zc;
 };
 
 struct Fp32State {
