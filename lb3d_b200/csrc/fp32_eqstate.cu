@@ -656,7 +656,8 @@ __global__ void __launch_bounds__(TX *TY, 1024 / (TX * TY))
 // through five-slot rings as in the dipole pass, and the own entries with
 // them (prefetched in registers the 16-byte ones exposed their latency: 78
 // against 70 us at ternary 128^3).  to_pops: write the populations (the last
-// step of a loop) instead of the equilibrium's arguments.  Ternary 128^3: 70
+// step of a loop) instead of the equilibrium's arguments, EQ_POPS_AFTER_ARGS
+// where earlier steps of the loop wrote those.  Ternary 128^3: 70
 // us at 16 warps per SM and 62 % issue (the pass that wrote populations every
 // step: 154 us); binary 256x128x128: 66 us (172 us).
 // ---------------------------------------------------------------------------
@@ -779,6 +780,8 @@ __device__ __forceinline__ void force_binary_masked(const float2 *Pm, const floa
   }
 }
 
+constexpr int EQ_POPS = 1, EQ_POPS_AFTER_ARGS = 2;
+
 template <int NC, int TX, int TY>
 struct EqCollideGeom {
   static constexpr int NT = TX * TY, AW = TX + 2, AN = AW * (TY + 2), RS = 5;
@@ -878,14 +881,14 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
       const int gz = wrapz(z0 + k, nz);
       const int self = own_xy + pl * gz;
       if (ROCK && (mk >> 18 & 1u)) {
-        // a rock site's populations stay zero, in both buffers: the arguments
-        // of the loop's earlier steps were laid over one of them
-        if (to_pops) {
+        // a rock site's populations stay zero; the arguments between a loop's
+        // steps were laid over the first 8 planes of the buffer it read (all 38
+        // planes of both buffers rewritten in every loop: a one-step loop of the
+        // porous 128^3 lattice 430 us, this way 208)
+        if (to_pops == EQ_POPS_AFTER_ARGS) {
+          float *fi = (par ? f1 : f0) + base + self;
 #pragma unroll
-          for (int q = 0; q < 38; ++q) {
-            f0[base + (size_t)q * S + self] = rock_dev(q % 19, Lg.rho0);
-            f1[base + (size_t)q * S + self] = rock_dev(q % 19, Lg.rho0);
-          }
+          for (int q = 0; q < 8; ++q) fi[(size_t)q * S] = rock_dev(q, Lg.rho0);
         }
         continue;
       }
@@ -1079,7 +1082,7 @@ cudaError_t eq_launch(const EqKernel &k, int pass, bool first, bool last, const 
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = pdl ? 1 : 0;
-  int l = last ? 1 : 0;
+  int l = last ? (first ? EQ_POPS : EQ_POPS_AFTER_ARGS) : 0;
   void *p00[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.f0, (void *)&a.f1,
                  (void *)&a.db0, (void *)&a.db1, (void *)&a.rock, (void *)&a.X};
   void *p0[] = {(void *)&a.lats, (void *)&a.tiles, (void *)&a.ntiles, (void *)&a.mask, (void *)&a.X};

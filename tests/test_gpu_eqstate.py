@@ -91,6 +91,30 @@ def test_rock_populations_survive_a_change_of_strategy():
         assert np.array_equal(out[0][0], n) and out[0][1] == counts
 
 
+@pytest.mark.parametrize("kind", ["rock", "sheared rock"])
+def test_rock_populations_after_loops_of_one_step_and_more(kind):
+    """A loop of one step lays no arguments over the rock sites' populations, a
+    longer one over the first planes of the buffer it read: whichever buffer is
+    current afterwards holds them as uploaded."""
+    from lb3d_b200.lib import Lattice
+    nc, kw, rock, shear = KINDS[kind]
+    dims = (35, 9, 11)
+    p, st = _params(dims, nc, **kw), _state(dims, nc, rock, shear)
+    out = []
+    for split in (2, 3):
+        lat = Lattice(p, precision=1)
+        lat.upload_state(st)
+        lat.set_launch_shape(16, 8, 16, split)
+        got = []
+        for steps in (1, 3, 1, 1, 2, 1, 4, 2):
+            lat.time_loop(steps)
+            got.append((lat.download()["n"], lat.sanity()))
+        out.append(got)
+        lat.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a[0], b[0]) and a[1] == b[1]
+
+
 def test_ensemble_members_on_strategy_3():
     """Odd sizes, one member alone in a chunk of one step, and a member that
     does not relax fully joining (all run strategy 2 then)."""
