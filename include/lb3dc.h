@@ -280,7 +280,13 @@ int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
                           lb3dc_ensemble **out);
 int lb3dc_ensemble_destroy(lb3dc_ensemble *e);
 int lb3dc_ensemble_last_error(const lb3dc_ensemble *e, char *buf, int len);
+/* The strategy (split, as in lb3dc_set_launch_shape) and, for 0 to 2, its tile
+ * and z chunk.  3, the default, runs strategy 3, which sizes its own tiles,
+ * while every active member relaxes fully (tau = 1, at least 2 sites across in
+ * x and y) and otherwise strategy 2 with tx, ty and zc. */
 int lb3dc_ensemble_set_shape(lb3dc_ensemble *e, int tx, int ty, int zc, int split);
+/* tx, ty and zc as set; split: the strategy the members now active run. */
+int lb3dc_ensemble_get_shape(const lb3dc_ensemble *e, int *tx, int *ty, int *zc, int *split);
 /* Admits one periodic lattice (p->precision is ignored: members are FP32
  * deviation) that will run nsteps steps; n, db as in lb3dc_upload_state.
  * Returns LB3DC_ENOMEM when no slot or no contiguous site range is free:

@@ -51,7 +51,9 @@ struct lb3dc_ensemble {
   int max_lat = 0, tile_cap = 0, ntiles = 0, grid = 0;
   std::vector<Member> members;
   std::map<long long, long long> free_ranges;  // base -> length
-  FusedShape shape{32, 4, 8, 2};  // fastest measured on the parameter-sweep stream
+  // launch shape of the strategies 0 to 2, and whether strategy 3 runs where it applies
+  FusedShape shape{32, 4, 8, 2};
+  bool prefer_eq = true;
   float4 *M = nullptr, *J = nullptr;
   EqFields X{};     // strategy 3's fields (null pointers: no room for them)
   bool eq = false;  // the active members run strategy 3
@@ -135,12 +137,12 @@ void give_range(lb3dc_ensemble *e, long long base, long long n) {
   }
 }
 
-// Strategy 3 (fp32_eqstate.cu) advances the active members when all of them
-// relax fully; their tiles serve every pass.
+// Strategy 3 (fp32_eqstate.cu) advances the active members, unless the caller
+// chose another one, when all of them relax fully; their tiles serve every pass.
 constexpr int EQ_TX = 16, EQ_TY = 8;
 
 bool runs_eq(const lb3dc_ensemble *e) {
-  if (!e->X.o1 || e->shape.split != 2) return false;
+  if (!e->X.o1 || !e->prefer_eq) return false;
   for (const Member &m : e->members)
     if (m.used && m.remaining > 0 && !fp32_eq_eligible(dev_params_from(m.p))) return false;
   return true;
@@ -432,8 +434,8 @@ int lb3dc_ensemble_last_error(const lb3dc_ensemble *e, char *buf, int len) {
 
 int lb3dc_ensemble_set_shape(lb3dc_ensemble *e, int tx, int ty, int zc, int split) {
   if (!e) return LB3DC_EINVAL;
-  if (split < 0 || split > 2) return efail(e, LB3DC_EINVAL, "split must be 0, 1 or 2");
-  FusedShape sh{tx, ty, zc, split};
+  if (split < 0 || split > 3) return efail(e, LB3DC_EINVAL, "split must be 0, 1, 2 or 3");
+  FusedShape sh{tx, ty, zc, split == 3 ? 2 : split};
   if (fp32_fused_ctas_per_sm(e->nc, false, false, sh) < 1 || zc < 1)
     return efail(e, LB3DC_EINVAL, "unsupported launch shape");
   // the own-moment field is read by the plain split strategy only; it is
@@ -448,7 +450,17 @@ int lb3dc_ensemble_set_shape(lb3dc_ensemble *e, int tx, int ty, int zc, int spli
     e->bytes += e->S * fp32_own_bytes(e->nc);
   }
   e->shape = sh;
+  e->prefer_eq = split == 3;
   e->dirty = true;
+  return LB3DC_OK;
+}
+
+int lb3dc_ensemble_get_shape(const lb3dc_ensemble *e, int *tx, int *ty, int *zc, int *split) {
+  if (!e) return LB3DC_EINVAL;
+  if (tx) *tx = e->shape.tx;
+  if (ty) *ty = e->shape.ty;
+  if (zc) *zc = e->shape.zc;
+  if (split) *split = runs_eq(e) ? 3 : e->shape.split;
   return LB3DC_OK;
 }
 

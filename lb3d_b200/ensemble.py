@@ -2,7 +2,7 @@
 
 `Ensemble` wraps the lb3dc_ensemble_* C-ABI: members of uneven size share
 one packed, device-resident site space and advance together in one
-persistent fused kernel launch per step (replayed from a CUDA graph).
+launch of each pass per step (replayed from a CUDA graph).
 
 `Server` is the request loop for parameter-sweep solves: requests that have
 arrived are admitted in arrival order while their HBM footprint fits in the
@@ -38,6 +38,7 @@ def _bind():
         "lb3dc_ensemble_destroy": (I, [V]),
         "lb3dc_ensemble_last_error": (I, [V, ctypes.c_char_p, I]),
         "lb3dc_ensemble_set_shape": (I, [V, I, I, I, I]),
+        "lb3dc_ensemble_get_shape": (I, [V] + [ctypes.POINTER(I)] * 4),
         "lb3dc_ensemble_admit": (I, [V, P, _D, _D, I, ctypes.POINTER(I)]),
         "lb3dc_ensemble_admit_seeded": (I, [V, P, ctypes.c_ulonglong, _D, ctypes.c_double, I,
                                             ctypes.POINTER(I)]),
@@ -108,7 +109,7 @@ class PinnedPool:
 
 
 class Ensemble:
-    def __init__(self, ncomp=3, capacity_sites=1 << 24, max_lattices=1024, shape=(32, 4, 8, 2)):
+    def __init__(self, ncomp=3, capacity_sites=1 << 24, max_lattices=1024, shape=(32, 4, 8, 3)):
         L = _bind()
         h = ctypes.c_void_p()
         rc = L.lb3dc_ensemble_create(int(ncomp), int(capacity_sites), int(max_lattices), ctypes.byref(h))
@@ -124,6 +125,13 @@ class Ensemble:
         if shape:
             sh = tuple(shape) + ((1,) if len(shape) == 3 else ())
             self._ck(L.lb3dc_ensemble_set_shape(self.h, *map(int, sh)))
+
+    @property
+    def launch_shape(self):
+        """(tile x, tile y, z chunk, strategy the members now active run)"""
+        v = [ctypes.c_int() for _ in range(4)]
+        self._ck(_bind().lb3dc_ensemble_get_shape(self.h, *map(ctypes.byref, v)))
+        return tuple(x.value for x in v)
 
     def _err(self):
         buf = ctypes.create_string_buffer(512)

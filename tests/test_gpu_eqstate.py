@@ -135,6 +135,36 @@ def test_ensemble_members_on_strategy_3():
         assert np.array_equal(got["n"], ref["n"]) and np.array_equal(got["db"], ref["db"])
 
 
+@pytest.mark.parametrize("nc", [2, 3])
+@pytest.mark.parametrize("kw", [{}, dict(g_accn=2e-4, g_accn_x=-1e-4)], ids=["free", "body force"])
+def test_ensemble_strategy_is_the_one_asked_for(nc, kw):
+    """Binary and ternary members, without and with a body force, in chunks of
+    1 to 3 steps and in chunks replayed from a graph: strategy 3 by default while
+    all of them relax fully, 2 (or 0) where the caller says so, the same bits
+    either way; a member that does not relax fully takes all to strategy 2."""
+    from lb3d_b200.ensemble import Ensemble
+    members = [(17, 9, 5), (16, 33, 12), (7, 8, 31)]
+    got = {}
+    for shape in (None, (32, 4, 8, 3), (16, 8, 4, 2), (32, 4, 8, 0)):
+        ens = Ensemble(nc, capacity_sites=20000, max_lattices=8, **({} if shape is None else dict(shape=shape)))
+        want = 3 if shape is None else shape[3]
+        assert ens.launch_shape == (shape or (32, 4, 8))[:3] + (want,)
+        slots = [ens.admit(_params(d, nc, **kw), _state(d, nc), steps=21) for d in members]
+        for chunk in (1, 3, 5, 5, 5, 2):
+            assert ens.launch_shape[3] == want and ens.step(chunk) == chunk
+        got[shape] = [ens.retire(s, d[::-1]) for s, d in zip(slots, members)]
+        ens.admit(_params((9, 9, 9), nc, tau_r=1.2), _state((9, 9, 9), nc), steps=1)
+        assert ens.launch_shape[3] == (2 if want == 3 else want)
+        ens.close()
+    for shape, out in got.items():
+        for a, b in zip(got[(16, 8, 4, 2)], out):
+            assert np.array_equal(a["n"], b["n"]), shape
+            assert nc == 2 or np.array_equal(a["db"], b["db"]), shape
+    for a, d in zip(got[None], members):
+        ref = _run(_params(d, nc, **kw), _state(d, nc), (16, 8, 16, 2), (21,))[0]
+        assert np.array_equal(a["n"], ref["n"])
+
+
 @pytest.mark.parametrize("nc,rock", [(3, False), (2, True)])
 def test_download_planes(nc, rock):
     """Densities and momenta of a download are the FP64 sums, in direction order,
