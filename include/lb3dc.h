@@ -274,8 +274,9 @@ typedef struct lb3dc_ensemble lb3dc_ensemble;
 /* capacity_sites bounds the sum of member sizes (19*capacity < 2^32);
  * device bytes per site of capacity: 2*19*ncomp*4 (+24 ternary), the moment
  * field (32 ternary, 8 binary) and, while the device has room for them, the
- * fields of strategy 3 (108, 52); without those, members that relax fully
- * run strategy 2 like the others. */
+ * fields of strategy 3 (108, 52), given back when a later allocation of the
+ * ensemble (staging, tile lists) finds no room; without those, members that
+ * relax fully run strategy 2 like the others. */
 int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
                           lb3dc_ensemble **out);
 int lb3dc_ensemble_destroy(lb3dc_ensemble *e);

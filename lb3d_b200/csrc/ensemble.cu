@@ -81,17 +81,6 @@ int efail(lb3dc_ensemble *e, int code, const std::string &m) {
   return code;
 }
 
-// Device staging for a member's FP64 populations, grown on demand and kept.
-bool ensure_stage(lb3dc_ensemble *e, size_t bytes) {
-  if (e->stage_bytes >= bytes) return true;
-  if (e->stage) cudaFree(e->stage);
-  e->stage = nullptr;
-  e->stage_bytes = 0;
-  if (cudaMalloc(&e->stage, bytes) != cudaSuccess) return false;
-  e->stage_bytes = bytes;
-  return true;
-}
-
 void drop_graph(lb3dc_ensemble *e) {
   if (e->gexec) cudaGraphExecDestroy(e->gexec);
   if (e->graph) cudaGraphDestroy(e->graph);
@@ -100,11 +89,47 @@ void drop_graph(lb3dc_ensemble *e) {
   e->graph_steps = 0;
 }
 
+// Bytes of strategy 3's fields per site of capacity.
+size_t eq_bytes(const lb3dc_ensemble *e) { return e->nc == 3 ? 108 : 52; }
+
 void free_eq(lb3dc_ensemble *e) {
-  if (e->eq_block) cudaFree(e->eq_block);
+  if (e->eq_block) {
+    cudaFree(e->eq_block);
+    e->bytes -= (long long)((size_t)e->S * eq_bytes(e));
+  }
   e->eq_block = nullptr;
   e->X = EqFields{};
   cudaGetLastError();
+}
+
+// A device allocation that the ensemble cannot do without: where the device has
+// no room for it, strategy 3's fields make way (fully relaxing members run
+// strategy 2 from then on).
+bool alloc_device(lb3dc_ensemble *e, void **p, size_t bytes) {
+  *p = nullptr;
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  if (!e->eq_block) return false;
+  cudaStreamSynchronize(e->stream);
+  drop_graph(e);
+  free_eq(e);
+  e->dirty = true;
+  if (cudaMalloc(p, bytes) == cudaSuccess) return true;
+  cudaGetLastError();
+  *p = nullptr;
+  return false;
+}
+
+// Device staging for a member's FP64 populations, grown on demand and kept.
+bool ensure_stage(lb3dc_ensemble *e, size_t bytes) {
+  if (e->stage_bytes >= bytes) return true;
+  if (e->stage) cudaFree(e->stage);
+  e->stage = nullptr;
+  e->stage_bytes = 0;
+  if (!alloc_device(e, (void **)&e->stage, bytes)) return false;
+  e->stage_bytes = bytes;
+  return true;
 }
 
 bool take_range(lb3dc_ensemble *e, long long n, long long *base) {
@@ -187,9 +212,13 @@ int rebuild(lb3dc_ensemble *e) {
   }
   if ((int)tiles.size() > e->tile_cap) {
     if (e->d_tiles) cudaFree(e->d_tiles);
-    e->tile_cap = (int)tiles.size() * 2 + 64;
-    if (cudaMalloc(&e->d_tiles, (size_t)e->tile_cap * sizeof(Tile)) != cudaSuccess)
+    e->d_tiles = nullptr;
+    e->tile_cap = 0;
+    const int cap = (int)tiles.size() * 2 + 64;
+    if (!alloc_device(e, (void **)&e->d_tiles, (size_t)cap * sizeof(Tile)))
       return efail(e, LB3DC_ENOMEM, "tile list allocation failed");
+    e->tile_cap = cap;
+    if (e->eq && !e->eq_block) return rebuild(e);  // strategy 3's fields made way: other tiles
   }
   e->ntiles = (int)tiles.size();
   if (e->ntiles)
@@ -375,8 +404,7 @@ int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
     X.M = e->M;
     // one block: Q, o1, o3 (float4), psi (ternary; a binary lattice's M holds
     // psi), o2
-    const size_t b = ncomp == 3 ? 108 : 52;
-    const bool room = cudaMalloc(&e->eq_block, n * b) == cudaSuccess;
+    const bool room = cudaMalloc(&e->eq_block, n * eq_bytes(e)) == cudaSuccess;
     if (room) {
       X.Q[0] = reinterpret_cast<float4 *>(e->eq_block);
       X.o1 = X.Q[0] + (ncomp == 3 ? 4 : 2) * n;
@@ -385,10 +413,12 @@ int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
       X.o2 = ncomp == 3 ? reinterpret_cast<float *>(X.psi + n) : reinterpret_cast<float *>(X.o1 + n);
     }
     X.Q[1] = X.Q[0];
-    if (room)
-      e->bytes += (long long)(n * b);
-    else
+    if (room) {
+      e->bytes += (long long)(n * eq_bytes(e));
+    } else {
+      e->eq_block = nullptr;
       free_eq(e);
+    }
   }
   e->members.resize(max_lattices);
   e->free_ranges[0] = capacity_sites;
@@ -442,11 +472,8 @@ int lb3dc_ensemble_set_shape(lb3dc_ensemble *e, int tx, int ty, int zc, int spli
   // allocated the first time that strategy is chosen
   if (split == 1 && !e->J) {
     cudaSetDevice(e->device);
-    if (cudaMalloc(&e->J, (size_t)e->S * fp32_own_bytes(e->nc)) != cudaSuccess) {
-      e->J = nullptr;
-      cudaGetLastError();
+    if (!alloc_device(e, (void **)&e->J, (size_t)e->S * fp32_own_bytes(e->nc)))
       return efail(e, LB3DC_ENOMEM, "own-moment field allocation failed");
-    }
     e->bytes += e->S * fp32_own_bytes(e->nc);
   }
   e->shape = sh;
@@ -651,7 +678,7 @@ int lb3dc_ensemble_retire_async(lb3dc_ensemble *e, int slot, double *n, double *
     if (cudaMalloc(&e->cstage, got) != cudaSuccess) {
       cudaGetLastError();
       got = nb + dbb;
-      if (cudaMalloc(&e->cstage, got) != cudaSuccess) return efail(e, LB3DC_ENOMEM, "staging allocation failed");
+      if (!alloc_device(e, (void **)&e->cstage, got)) return efail(e, LB3DC_ENOMEM, "staging allocation failed");
     }
     e->cstage_bytes = got;
   }

@@ -1,0 +1,77 @@
+"""Work on a device that has almost no memory left: what strategy 3 takes beyond
+strategy 2 makes way for what a call cannot do without."""
+import contextlib
+
+import numpy as np
+import pytest
+
+from lb3d_b200.config import Params
+from lb3d_b200.ic import uniform_mixture
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+@contextlib.contextmanager
+def _only(left):
+    """Leaves about `left` bytes of device memory free."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held = []
+    while True:
+        free = torch.cuda.mem_get_info()[0]
+        size = (free - left) // (2 * MB) * (2 * MB)
+        if size < 32 * MB or len(held) == 8:
+            break
+        held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+    assert abs(torch.cuda.mem_get_info()[0] - left) < 48 * MB
+    try:
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+def _params(dims, nc=3):
+    return Params(nx=dims[0], ny=dims[1], nz=dims[2], ncomp=nc, tau_d=1.0, g_br=0.08, g_bs=-0.006, g_ss=-0.0045,
+                  beta=10.0, d_0=1.0, bdist=2, restore=1, precision=1).finalize()
+
+
+@pytest.mark.parametrize("first", ["admit", "retire", "retire_async"])
+def test_ensemble_gives_the_strategy_3_fields_back(first):
+    """A 72^3 member's staging takes 170 MB (179 MB with its dipoles); 100 MB are
+    left beside the fields of strategy 3 (216 MB)."""
+    from lb3d_b200.ensemble import Ensemble
+    from lb3d_b200.lib import lib
+    dims, small = (72, 72, 72), (16, 16, 16)
+    p, st = _params(dims), uniform_mixture(*dims, 3, seed=5)
+    out = []
+    for full in (False, True):
+        ens = Ensemble(3, capacity_sites=2_000_000, max_lattices=4)
+        before = lib().lb3dc_ensemble_bytes(ens.h)
+        seeded = first != "admit"
+        with contextlib.ExitStack() as stack:
+            if full:
+                stack.enter_context(_only(100 * MB))
+            slot = ens.admit(p, None if seeded else st, steps=6, seed=11)
+            assert slot is not None
+            ens.step(3), ens.step(3), ens.sync()
+            if first == "retire_async":
+                ens.retire_async(slot, dims)
+                while not ens.poll(slot):
+                    pass
+                got = ens.collect(slot)
+            else:
+                got = ens.retire(slot, dims)
+            assert ens.launch_shape[3] == (2 if full else 3)
+            assert lib().lb3dc_ensemble_bytes(ens.h) == before - (108 * 2_000_000 if full else 0)
+            # and it goes on
+            slot = ens.admit(_params(small), seed=3, steps=2)
+            ens.step(2)
+            more = ens.retire(slot, small)
+        out.append((got, more))
+        ens.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a["n"], b["n"]) and np.array_equal(a["db"], b["db"])
+
