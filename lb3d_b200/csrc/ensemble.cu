@@ -506,7 +506,12 @@ int lb3dc_ensemble_admit(lb3dc_ensemble *e, const lb3dc_params *p, const double 
   // FP64 populations to the device, converted there into deviations in the
   // parity-0 buffer's range
   const size_t nb = (size_t)e->nc * 19 * N * sizeof(double);
-  if (!ensure_stage(e, nb)) return efail(e, LB3DC_ENOMEM, "staging allocation failed");
+  if (!ensure_stage(e, nb)) {
+    // not admitted: the slot and its range are free again
+    give_range(e, base, N);
+    m = Member();
+    return efail(e, LB3DC_ENOMEM, "staging allocation failed");
+  }
   if (cudaMemcpyAsync(e->stage, n, nb, cudaMemcpyHostToDevice, e->stream) != cudaSuccess ||
       fp32_from_fp64(e->stage, e->f[0], e->S, base, N, e->nc, rho0, nullptr, e->stream) != cudaSuccess)
     return efail(e, LB3DC_ECUDA, "upload failed");

@@ -75,3 +75,21 @@ def test_ensemble_gives_the_strategy_3_fields_back(first):
     for a, b in zip(*out):
         assert np.array_equal(a["n"], b["n"]) and np.array_equal(a["db"], b["db"])
 
+
+
+def test_failed_admission_leaves_no_member():
+    """Strategy 3's fields (28 MB) do not make enough room for the staging
+    (114 MB): the request stays with the caller, and neither a slot
+    nor its sites are taken."""
+    from lb3d_b200.ensemble import Ensemble
+    dims = (64, 64, 64)
+    st = uniform_mixture(*dims, 3, seed=5)
+    ens = Ensemble(3, capacity_sites=270_000, max_lattices=2)
+    before = ens.stats()
+    with _only(40 * MB):
+        assert ens.admit(_params(dims), st, steps=2) is None
+        assert ens.stats() == before
+    slot = ens.admit(_params(dims), st, steps=2)
+    assert slot == 0 and ens.step(2) == 2
+    assert np.isfinite(ens.retire(slot, dims)["n"]).all()
+    ens.close()
