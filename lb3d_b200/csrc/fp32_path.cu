@@ -992,13 +992,36 @@ int fp32_z_chunks(int nz, int nxy, int resident, int halo) {
   return best;
 }
 
-static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st) {
-  const LatDesc &L = s.lat;
+// A tile list on the device; null when there is no room for it.
+static Tile *upload_tiles(const std::vector<Tile> &tiles, cudaStream_t st, int *rc) {
+  Tile *d = nullptr;
+  *rc = LB3DC_OK;
+  if (cudaMalloc(&d, tiles.size() * sizeof(Tile)) != cudaSuccess) {
+    cudaGetLastError();
+    *rc = LB3DC_ENOMEM;
+    return nullptr;
+  }
+  if (cudaMemcpyAsync(d, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, st) == cudaSuccess &&
+      cudaStreamSynchronize(st) == cudaSuccess)
+    return d;
+  cudaFree(d);
+  *rc = LB3DC_ECUDA;
+  return nullptr;
+}
+
+// The tile lists of strategy 3's passes, one after the other.
+struct EqTiles {
   std::vector<Tile> all;
+  int off[EQ_PASSES], ntiles[EQ_PASSES], edge = 0;
+};
+
+static int eq_build_tiles(const DevParams &P, const Fp32State &s, const FusedShape &sh, EqTiles &out) {
+  const LatDesc &L = s.lat;
+  std::vector<Tile> &all = out.all;
   // a chunk of any pass works on one plane beyond each of its ends
   for (int pass = 0; pass < EQ_PASSES; ++pass) {
-    s.eq_off[pass] = (int)all.size();
-    s.eq_ntiles[pass] = 0;
+    out.off[pass] = (int)all.size();
+    out.ntiles[pass] = 0;
     EqKernel kn;
     if (!eq_kernel_of(P, s, pass, false, sh.tx, sh.ty, &kn)) {
       if (pass == EQ_MOMENTS || pass == EQ_COLLIDE) return LB3DC_EINVAL;
@@ -1024,20 +1047,14 @@ static int eq_build_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh
           all.push_back(t);
         }
     }
-    s.eq_ntiles[pass] = (int)all.size() - s.eq_off[pass];
+    out.ntiles[pass] = (int)all.size() - out.off[pass];
     if (pass == EQ_MOMENTS && eq_forks(P)) {
       auto inner = [&](const Tile &t) { return t.x0 != 0 && t.x0 + tx < L.nx; };
-      const auto end = std::stable_partition(all.begin() + s.eq_off[pass], all.end(), inner);
-      s.eq_edge = (int)(all.end() - end);
+      const auto end = std::stable_partition(all.begin() + out.off[pass], all.end(), inner);
+      out.edge = (int)(all.end() - end);
     }
   }
-  if (s.eq_tiles) cudaFree(s.eq_tiles);
-  s.eq_tiles = nullptr;
-  if (cudaMalloc(&s.eq_tiles, all.size() * sizeof(Tile)) != cudaSuccess) return LB3DC_ENOMEM;
-  if (cudaMemcpyAsync(s.eq_tiles, all.data(), all.size() * sizeof(Tile), cudaMemcpyHostToDevice, st) !=
-      cudaSuccess)
-    return LB3DC_ECUDA;
-  return cudaStreamSynchronize(st) == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;
+  return LB3DC_OK;
 }
 
 // Lees-Edwards lattices: the compact pre-stream boundary planes from the
@@ -1087,25 +1104,35 @@ static int ensure_own(const DevParams &P, Fp32State &s) {
   return LB3DC_OK;
 }
 
+// Switches to a launch shape; where that fails the present one stays whole.
 static int rebuild_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st) {
-  if (sh.split == 1) {
-    int rc = ensure_own(P, s);
-    if (rc) return rc;
-  }
+  const bool rock = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
+  int rc = LB3DC_OK, per = 0;
+  if (sh.split != 3 && (per = fp32_fused_ctas_per_sm(P.nc, rock, body, sh)) < 1) return LB3DC_EINVAL;
+  if (sh.split == 1 && (rc = ensure_own(P, s))) return rc;
+  EqTiles eq;
+  Tile *d_eq = nullptr;
   if (sh.split == 3) {
     if (!fp32_eq_eligible(P)) return LB3DC_ENOTSUP;
-    int rc = ensure_eq(P, s, st);
-    if (rc == LB3DC_OK) rc = eq_build_tiles(P, s, sh, st);
-    if (rc != LB3DC_OK) return rc;
+    if ((rc = ensure_eq(P, s, st)) || (rc = eq_build_tiles(P, s, sh, eq))) return rc;
+    if (!(d_eq = upload_tiles(eq.all, st, &rc))) return rc;
   }
   std::vector<Tile> tiles;
   fp32_tiles_for(s.lat, 0, sh, tiles);
+  Tile *d = upload_tiles(tiles, st, &rc);
+  if (!d) {
+    if (d_eq) cudaFree(d_eq);
+    return rc;
+  }
+  if (d_eq) {
+    if (s.eq_tiles) cudaFree(s.eq_tiles);
+    s.eq_tiles = d_eq;
+    std::copy(eq.off, eq.off + EQ_PASSES, s.eq_off);
+    std::copy(eq.ntiles, eq.ntiles + EQ_PASSES, s.eq_ntiles);
+    s.eq_edge = eq.edge;
+  }
   if (s.d_tiles) cudaFree(s.d_tiles);
-  s.d_tiles = nullptr;
-  if (cudaMalloc(&s.d_tiles, tiles.size() * sizeof(Tile)) != cudaSuccess) return LB3DC_ENOMEM;
-  if (cudaMemcpyAsync(s.d_tiles, tiles.data(), tiles.size() * sizeof(Tile), cudaMemcpyHostToDevice,
-                      st) != cudaSuccess)
-    return LB3DC_ECUDA;
+  s.d_tiles = d;
   s.ntiles = (int)tiles.size();
   s.tx = sh.tx;
   s.ty = sh.ty;
@@ -1114,14 +1141,8 @@ static int rebuild_tiles(const DevParams &P, Fp32State &s, const FusedShape &sh,
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  bool rock = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
-  if (sh.split == 3) {
-    s.grid = s.ntiles;  // each pass sizes its own grid at launch
-    return LB3DC_OK;
-  }
-  int per = fp32_fused_ctas_per_sm(P.nc, rock, body, sh);
-  if (per < 1) return LB3DC_EINVAL;
-  s.grid = std::min(s.ntiles, per * nsm);
+  // strategy 3: each pass sizes its own grid at launch
+  s.grid = sh.split == 3 ? s.ntiles : std::min(s.ntiles, per * nsm);
   return LB3DC_OK;
 }
 
@@ -1352,8 +1373,10 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   // keep the launch shape chosen so far (set or autotuned); the kernel
   // variant may change with the rock flag
   int rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, s.split}, st);
-  if (rc == LB3DC_ENOMEM && s.split == 3)  // no room for the neighbour mask
+  if (rc == LB3DC_ENOMEM && s.split == 3) {  // no room for the neighbour mask
+    s.split = 2;                             // d_tiles serve it as they are
     rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, 2}, st);
+  }
   if (rc) return rc;
   (void)p;
   return cudaStreamSynchronize(st) == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;

@@ -93,3 +93,47 @@ def test_failed_admission_leaves_no_member():
     assert slot == 0 and ens.step(2) == 2
     assert np.isfinite(ens.retire(slot, dims)["n"]).all()
     ens.close()
+
+
+@contextlib.contextmanager
+def _nothing():
+    """Leaves no device memory free."""
+    import torch
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    held, size = [], torch.cuda.mem_get_info()[0] // (2 * MB) * (2 * MB)
+    while size >= 2 * MB:
+        try:
+            held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            size = size // (4 * MB) * (2 * MB)
+    try:
+        yield
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+
+
+@pytest.mark.parametrize("split", [2, 3])
+def test_a_launch_shape_without_room_leaves_the_present_one(split):
+    """Chunks of one plane make a tile list of 6 MB on this lattice."""
+    from lb3d_b200.lib import LB3DC_ENOMEM, Lattice, Lb3dError
+    dims = (2, 2, 300_000)
+    p, st = _params(dims, 2), uniform_mixture(*dims, 2, seed=5)
+    out = []
+    for full in (False, True):
+        lat = Lattice(p)
+        lat.upload_state(st)
+        lat.set_launch_shape(32, 4, 64, split)
+        lat.time_loop(2)
+        lat.sync()
+        with _nothing() if full else contextlib.nullcontext():
+            if full:
+                with pytest.raises(Lb3dError) as err:
+                    lat.set_launch_shape(16, 8, 1, split)
+                assert err.value.code == LB3DC_ENOMEM and lat.launch_shape == (32, 4, 64, split)
+            lat.time_loop(3)
+            lat.sync()
+        out.append(lat.download()["n"])
+        lat.close()
+    assert np.array_equal(*out)
