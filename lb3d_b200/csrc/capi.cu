@@ -277,6 +277,10 @@ int ensure_scratch(lb3dc_handle *h, long long bytes) {
   h->scratch = nullptr;
   h->scratch_bytes = 0;
   int rc = dalloc(h, (unsigned char **)&h->scratch, (size_t)bytes);
+  if (rc && h->p.precision == LB3DC_FP32_DEV && fp32_make_room(h->s32, h->stream)) {
+    cudaGetLastError();
+    rc = dalloc(h, (unsigned char **)&h->scratch, (size_t)bytes);
+  }
   if (rc) return rc;
   h->scratch_bytes = bytes;
   return 0;
@@ -342,7 +346,6 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
   } else if (!rc) {
     rc = fp32_alloc(h->P, *p, h->s32, h->stream);
     if (rc) fail(h, rc, "FP32 state allocation failed");
-    h->bytes += h->s32.bytes;
   }
   if (!rc) {
     e = cudaStreamSynchronize(h->stream);
@@ -386,7 +389,7 @@ int lb3dc_last_error(const lb3dc_handle *h, char *buf, int len) {
   return h ? h->errcode : g_create_code;
 }
 
-long long lb3dc_device_bytes(const lb3dc_handle *h) { return h ? h->bytes : 0; }
+long long lb3dc_device_bytes(const lb3dc_handle *h) { return h ? h->bytes + h->s32.bytes : 0; }
 
 int lb3dc_upload_state(lb3dc_handle *h, const double *n, const double *db, const double *rock,
                        double shear_sum, int nt) {

@@ -861,6 +861,38 @@ bool fp32_eq_eligible(const DevParams &P) {
   return P.nx >= 2 && P.ny >= 2;
 }
 
+static void free_eq(Fp32State &s) {
+  if (s.o1) s.bytes -= s.S * (s.lat.nc == 3 ? 44 : 20);
+  if (s.mask) s.bytes -= s.S * 4;
+  void *bufs[] = {s.o1, s.o2, s.o3, s.psi, s.mask, s.eq_tiles};
+  for (void *b : bufs)
+    if (b) cudaFree(b);
+  s.o1 = s.o3 = nullptr;
+  s.o2 = nullptr;
+  s.psi = nullptr;
+  s.mask = nullptr;
+  s.eq_tiles = nullptr;
+}
+
+bool fp32_make_room(Fp32State &s, cudaStream_t st) {
+  if (!s.o1) return false;
+  cudaStreamSynchronize(st);
+  free_eq(s);
+  if (s.split == 3) s.split = 2;  // d_tiles serve it as they are
+  return true;
+}
+
+// A device allocation of the handle; strategy 3's fields make way for it.
+static int alloc_device(Fp32State &s, void **p, size_t bytes, cudaStream_t st) {
+  for (int k = 0; k < 2; ++k) {
+    if (cudaMalloc(p, bytes) == cudaSuccess) return LB3DC_OK;
+    cudaGetLastError();
+    *p = nullptr;
+    if (k || !fp32_make_room(s, st)) break;
+  }
+  return LB3DC_ENOMEM;
+}
+
 // The fields of strategy 3, allocated the first time a lattice is switched to
 // it, and (with rock) the neighbour mask and the rock sites' psi entries.
 static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
@@ -872,13 +904,8 @@ static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
       ok = cudaMalloc(&s.o3, N * sizeof(float4)) == cudaSuccess && cudaMalloc(&s.psi, N * sizeof(float2)) == cudaSuccess;
     if (!ok) {
       cudaGetLastError();
-      if (s.o1) cudaFree(s.o1);
-      if (s.o2) cudaFree(s.o2);
-      if (s.o3) cudaFree(s.o3);
-      if (s.psi) cudaFree(s.psi);
-      s.o1 = s.o3 = nullptr;
-      s.o2 = nullptr;
-      s.psi = nullptr;
+      if (s.o1) s.bytes += s.S * (P.nc == 3 ? 44 : 20);  // free_eq takes them off
+      free_eq(s);
       return LB3DC_ENOMEM;
     }
     s.bytes += (long long)N * (P.nc == 3 ? 44 : 20);
@@ -1155,7 +1182,13 @@ int fp32_set_shape(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaS
   if (sh.split && !s.M) return LB3DC_EINVAL;
   if (sh.split < 0 || sh.split > 3) return LB3DC_EINVAL;
   if (sh.zc < 1) return LB3DC_EINVAL;
-  return rebuild_tiles(P, s, sh, st);
+  const FusedShape entry{s.tx, s.ty, s.zc, s.split};
+  int rc = rebuild_tiles(P, s, sh, st);
+  if (rc == LB3DC_ENOMEM && sh.split != 3 && fp32_make_room(s, st)) {
+    rc = rebuild_tiles(P, s, sh, st);
+    if (rc) rebuild_tiles(P, s, entry, st);
+  }
+  return rc;
 }
 
 std::vector<FusedShape> fp32_candidate_shapes(const DevParams &P) {
@@ -1188,7 +1221,9 @@ int fp32_autotune(const DevParams &P, Fp32State &s, const uint8_t *rock, double 
   const size_t pop = (size_t)P.nc * 19 * s.S * sizeof(float);
   const size_t dbs = P.nc == 3 ? 3 * (size_t)s.S * sizeof(float) : 0;
   float *save = nullptr;
-  if (cudaMalloc(&save, pop + dbs) != cudaSuccess) return LB3DC_ENOMEM;
+  const FusedShape entry{s.tx, s.ty, s.zc, s.split};
+  if (alloc_device(s, (void **)&save, pop + dbs, st)) return LB3DC_ENOMEM;
+  const bool made_way = s.split != entry.split;
   const int cur0 = s.lat.parity;
   cudaMemcpyAsync(save, s.f[cur0], pop, cudaMemcpyDeviceToDevice, st);
   if (dbs) cudaMemcpyAsync((char *)save + pop, s.db[cur0], dbs, cudaMemcpyDeviceToDevice, st);
@@ -1229,7 +1264,9 @@ int fp32_autotune(const DevParams &P, Fp32State &s, const uint8_t *rock, double 
   cudaFree(save);
   if (ntried) *ntried = n;
   s.timer = saved_timer;
-  int rc = rebuild_tiles(P, s, best, st);
+  // strategy 3, where it made way for the copy, was not timed: back to it
+  int rc = made_way ? rebuild_tiles(P, s, entry, st) : LB3DC_ENOMEM;
+  if (rc == LB3DC_ENOMEM) rc = rebuild_tiles(P, s, best, st);
   if (rc) return rc;
   return cudaStreamSynchronize(st) == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;
 }
@@ -1292,17 +1329,7 @@ void fp32_free(Fp32State &s) {
   if (s.d_tiles) cudaFree(s.d_tiles);
   if (s.M) cudaFree(s.M);
   if (s.J) cudaFree(s.J);
-  if (s.psi) cudaFree(s.psi);
-  if (s.o1) cudaFree(s.o1);
-  if (s.o2) cudaFree(s.o2);
-  if (s.o3) cudaFree(s.o3);
-  if (s.mask) cudaFree(s.mask);
-  if (s.eq_tiles) cudaFree(s.eq_tiles);
-  s.psi = nullptr;
-  s.o1 = s.o3 = nullptr;
-  s.o2 = nullptr;
-  s.mask = nullptr;
-  s.eq_tiles = nullptr;
+  free_eq(s);
   if (s.stage) cudaFree(s.stage);
   s.stage = nullptr;
   for (int i = 0; i < 4; ++i) {
@@ -1374,7 +1401,7 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   // variant may change with the rock flag
   int rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, s.split}, st);
   if (rc == LB3DC_ENOMEM && s.split == 3) {  // no room for the neighbour mask
-    s.split = 2;                             // d_tiles serve it as they are
+    fp32_make_room(s, st);
     rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, 2}, st);
   }
   if (rc) return rc;
@@ -1472,7 +1499,8 @@ int fp32_dump(const DevParams &P, Fp32State &s, int field, const uint8_t *rock, 
   const int nc = P.nc;
   double *n = nullptr, *rho = nullptr, *psi = nullptr, *mom = nullptr, *db = nullptr;
   size_t bytes = ((size_t)nc * 19 * N + 2 * (size_t)nc * N + 3 * (size_t)nc * N + 3 * (size_t)N) * 8;
-  if (cudaMalloc(&n, bytes) != cudaSuccess) return LB3DC_ENOMEM;
+  const FusedShape entry{s.tx, s.ty, s.zc, s.split};
+  if (alloc_device(s, (void **)&n, bytes, st)) return LB3DC_ENOMEM;
   rho = n + (size_t)nc * 19 * N;
   psi = rho + (size_t)nc * N;
   mom = psi + (size_t)nc * N;
@@ -1485,6 +1513,7 @@ int fp32_dump(const DevParams &P, Fp32State &s, int field, const uint8_t *rock, 
   if (e == cudaSuccess) e = fp64_dump(P, field, n, rho, psi, db, rock, out, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   cudaFree(n);
+  if (s.split != entry.split) rebuild_tiles(P, s, entry, st);  // strategy 3 again, where it had made way
   return e == cudaSuccess ? LB3DC_OK : LB3DC_ECUDA;
 }
 

@@ -113,6 +113,10 @@ int fp32_step(const DevParams &P, Fp32State &s, const uint8_t *rock, cudaStream_
 // every step, or with le_per_step one for each step.
 int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, cudaStream_t st,
              const LEStep *le = nullptr, bool le_per_step = false);
+// Gives strategy 3's fields back (it takes more than the others, and is the
+// default) so that another allocation finds room; the lattice runs strategy 2
+// from then on.  False when there is nothing to give.
+bool fp32_make_room(Fp32State &s, cudaStream_t st);
 int fp32_dump(const DevParams &P, Fp32State &s, int field, const uint8_t *rock, double *out,
               cudaStream_t st);
 cudaError_t fp32_reduce_conservation(const DevParams &P, Fp32State &s, const uint8_t *rock,
