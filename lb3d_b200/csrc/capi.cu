@@ -261,9 +261,10 @@ int need_loaded(lb3dc_handle *h) {
 }
 
 // The FP64 time loop streams inside the collision (fp64_step_pull) unless an
-// invasion boundary acts on the post-stream populations between the two.
+// invasion boundary acts on the post-stream populations between the two or a
+// sheared lattice found no room for its post-stream boundary planes.
 bool fp64_pull_ok(const lb3dc_handle *h) {
-  if (h->p.precision != LB3DC_FP64 || h->P.zouhe) return false;
+  if (h->p.precision != LB3DC_FP64 || h->P.zouhe || (h->le && !h->post)) return false;
   const int k = h->p.inv_fluid;
   return !(h->p.boundary_cond != 0 && (k == 11 || k == 7 || k == 8));
 }
@@ -337,11 +338,15 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
     if (h->le) {
       rc = rc ? rc : dalloc(h, &h->hlo, nc * 19 * np);
       rc = rc ? rc : dalloc(h, &h->hhi, nc * 19 * np);
-      rc = rc ? rc : dalloc(h, &h->post, 2 * nc * 19 * np);
       rc = rc ? rc : dalloc(h, &h->rlo, nc * np);
       rc = rc ? rc : dalloc(h, &h->rhi, nc * np);
       rc = rc ? rc : dalloc(h, &h->plo, nc * np);
       rc = rc ? rc : dalloc(h, &h->phi, nc * np);
+      // optional: without room for them the steps stream in a pass of their own
+      if (!rc && dalloc(h, &h->post, 2 * nc * 19 * np)) {
+        cudaGetLastError();
+        fail(h, LB3DC_OK, "");
+      }
     }
   } else if (!rc) {
     rc = fp32_alloc(h->P, *p, h->s32, h->stream);

@@ -177,3 +177,23 @@ def test_lattice_gives_the_strategy_3_fields_back(what, per_site):
         lat.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_sheared_fp64_lattice_without_room_for_its_boundary_planes():
+    """A thin sheared lattice whose post-stream boundary planes (152 MiB) do not
+    fit beside the rest (513 MiB): it steps all the same, to the same bits."""
+    from lb3d_b200.lib import Lattice
+    dims = (2, 512, 512)
+    p = _params(dims, 2, boundary_cond=-1, inv_fluid=5, shear_u=0.05)
+    st = uniform_mixture(*dims, 2, seed=5)
+    out = []
+    for full in (False, True):
+        with _only(590 * MB) if full else contextlib.nullcontext():
+            lat = Lattice(p, precision=0)
+        lat.upload_state(st)
+        lat.time_loop(3)
+        out.append((lat.download(), lat.device_bytes))
+        lat.close()
+    for f in out[0][0]:
+        assert np.array_equal(out[0][0][f], out[1][0][f]), f
+    assert out[0][1] - out[1][1] == 2 * 2 * 19 * 512 * 512 * 8
