@@ -387,8 +387,11 @@ __global__ void k_recolour(DevParams P, double *__restrict__ g, const uint8_t *_
 // c . v of a lattice direction, the products and sums in axis order.  Terms of
 // a zero component are left out here and in the sums over directions below:
 // adding +-0 changes no finite value, and the compiler may not drop a product
-// with 0 by itself.  60 % of the components are zero; ternary 128^3, a step:
-// 0.830 -> 0.792 ms.
+// with 0 by itself.  24 of the 54 components of the moving directions are zero;
+// ternary 128^3, a step: 0.830 -> 0.792 ms.  A product of 0 and a number that is
+// not finite, which such a term would have added as NaN, belongs to one that
+// leaves the sums below without a finite result, too: only then are they formed
+// again with every term.
 __device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
   double r = 0.0;
   bool any = false;
@@ -400,6 +403,27 @@ __device__ __forceinline__ double cdot(const int c[3], const double v[3]) {
       any = true;
     }
   return r;
+}
+
+__device__ __forceinline__ bool finite_sum(const double a[3]) { return isfinite((a[0] + a[1]) + a[2]); }
+
+// The field of k_dipole with the terms of zero components.
+__device__ __forceinline__ void dipole_field_all(const DevParams &P, int x, int y, int z, long long i,
+                                                 const double *rho, const double *da, double sgn, double h[3]) {
+  const long long N = P.nsites;
+  double h_c[3] = {0.0, 0.0, 0.0};
+  double h_s[3] = {da[i], da[N + i], da[2 * N + i]};
+#pragma unroll 1
+  for (int q = 0; q < 18; ++q) {
+    const long long j = sidx(wrap(x + cx(q), P.nx), wrap(y + cy(q), P.ny), wrap(z + cz(q), P.nz), P.nx, P.ny);
+    const double pas[3] = {da[j], da[N + j], da[2 * N + j]};
+    const double hc_m = -(sgn * ((0.0 + rho[N + j]) - (0.0 + rho[j])) * (double)gw(q));
+    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)};
+    for (int k = 0; k < 3; ++k) h_c[k] = h_c[k] + hc_m * c[k];
+    const double hs_dot = 2.0 * ((c[0] * pas[0] + c[1] * pas[1]) + c[2] * pas[2]);
+    for (int k = 0; k < 3; ++k) h_s[k] = h_s[k] + (pas[k] - c[k] * hs_dot) * (double)gw(q);
+  }
+  for (int k = 0; k < 3; ++k) h[k] = h_c[k] + h_s[k];
 }
 
 // ---------------------------------------------------------------------------
@@ -443,6 +467,10 @@ __global__ void __launch_bounds__(256, 4) k_dipole(DevParams P, const double *rh
   double h[3];
   for (int k = 0; k < 3; ++k) h[k] = h_c[k] + h_s[k];
   double h_m = P.beta * sqrt((h[0] * h[0] + h[1] * h[1]) + h[2] * h[2]);
+  if (!isfinite(h_m)) {
+    dipole_field_all(P, x, y, z, i, rho, da, sgn, h);
+    h_m = P.beta * sqrt((h[0] * h[0] + h[1] * h[1]) + h[2] * h[2]);
+  }
   double sd_eq[3];
   const double third = 1.0 / 3.0;
   for (int k = 0; k < 3; ++k) sd_eq[k] = (third * P.beta) * h[k];
@@ -472,12 +500,10 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
   const int nx = P.nx, ny = P.ny, nz = P.nz;
   const long long NP = (long long)ny * nz;
   double f_br[3] = {0, 0, 0}, f_rb[3] = {0, 0, 0}, f_wr[3] = {0, 0, 0}, f_wb[3] = {0, 0, 0};
-#pragma unroll
-  for (int q = 0; q < 18; ++q) {
-    const int c[3] = {cx(q), cy(q), cz(q)};
+  // psi of the neighbour in direction q; rk: it is rock
+  auto neighbour = [&](int q, double &psi_r, double &psi_b, bool &rk) {
     int xn = x + cx(q), yn = y + cy(q), zn = z + cz(q);
-    double psi_r, psi_b;
-    bool rk = false;
+    rk = false;
     if (LE && (xn < 0 || xn >= nx)) {
       long long h = wrap(yn, ny) + (long long)ny * wrap(zn, nz);
       const double *pp = (xn < 0) ? plo : phi;
@@ -502,6 +528,13 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
         psi_b = psi[N + j];
       }
     }
+  };
+#pragma unroll
+  for (int q = 0; q < 18; ++q) {
+    const int c[3] = {cx(q), cy(q), cz(q)};
+    double psi_r, psi_b;
+    bool rk;
+    neighbour(q, psi_r, psi_b, rk);
     double green_r = psi_b * (double)gw(q);
     double green_b = psi_r * (double)gw(q);
     if (rk) {
@@ -518,25 +551,81 @@ __device__ __forceinline__ void sc_force_binary(const DevParams &P, int x, int y
       }
     }
   }
-  double pb = psi[N + i], prr = psi[i];
-  for (int k = 0; k < 3; ++k) {
-    double br = -(P.g_br * f_br[k]);
-    double rb = -(P.g_br * f_rb[k]);
-    double wr = -(P.g_wr * f_wr[k]);
-    double wb = -(P.g_wb * f_wb[k]);
-    fb[k] = (br + ((wb / P.tau[1]) * P.tau_wb)) * pb;
-    fr[k] = (rb + ((wr / P.tau[0]) * P.tau_wr)) * prr;
+  const double pb = psi[N + i], prr = psi[i];
+  auto forces = [&]() {
+    for (int k = 0; k < 3; ++k) {
+      double br = -(P.g_br * f_br[k]);
+      double rb = -(P.g_br * f_rb[k]);
+      double wr = -(P.g_wr * f_wr[k]);
+      double wb = -(P.g_wb * f_wb[k]);
+      fb[k] = (br + ((wb / P.tau[1]) * P.tau_wb)) * pb;
+      fr[k] = (rb + ((wr / P.tau[0]) * P.tau_wr)) * prr;
+    }
+  };
+  forces();
+  if (finite_sum(fb) && finite_sum(fr)) return;
+  // with the terms of zero components
+  for (int k = 0; k < 3; ++k) f_br[k] = f_rb[k] = f_wr[k] = f_wb[k] = 0.0;
+#pragma unroll 1
+  for (int q = 0; q < 18; ++q) {
+    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)}, g = (double)gw(q);
+    double psi_r, psi_b;
+    bool rk;
+    neighbour(q, psi_r, psi_b, rk);
+    const double green_r = psi_b * g, green_b = psi_r * g;
+    for (int k = 0; k < 3; ++k) {
+      if (rk) {
+        f_wb[k] = f_wb[k] + green_r * c[k];
+        f_wr[k] = f_wr[k] + green_b * c[k];
+      } else {
+        f_rb[k] = f_rb[k] + green_r * c[k];
+        f_br[k] = f_br[k] + green_b * c[k];
+      }
+    }
+  }
+  forces();
+}
+
+// The sums over the directions of sc_force_ternary.
+struct TernarySums {
+  double br[3] = {0, 0, 0}, rb[3] = {0, 0, 0}, cs[3] = {0, 0, 0}, sc[3] = {0, 0, 0}, ss[3] = {0, 0, 0};
+};
+
+// With the terms of zero components.
+__device__ __forceinline__ void ternary_sums_all(const DevParams &P, int x, int y, int z, const double *psi,
+                                                 const double *db, const double dbx[3], TernarySums &f) {
+  const long long N = P.nsites;
+  f = TernarySums();
+#pragma unroll 1
+  for (int q = 0; q < 18; ++q) {
+    const long long j = sidx(wrap(x + cx(q), P.nx), wrap(y + cy(q), P.ny), wrap(z + cz(q), P.nz), P.nx, P.ny);
+    const double c[3] = {(double)cx(q), (double)cy(q), (double)cz(q)}, g = (double)gw(q);
+    const double psi_r = psi[j], psi_b = psi[N + j], pss = psi[2 * N + j];
+    const double green_r = psi_b * g, green_b = psi_r * g;
+    const double dd[3] = {db[j] * pss, db[N + j] * pss, db[2 * N + j] * pss};
+    const double d_dotc = (dd[0] * c[0] + dd[1] * c[1]) + dd[2] * c[2];
+    const double di_dotc = (dbx[0] * c[0] + dbx[1] * c[1]) + dbx[2] * c[2];
+    const double greenc_s = (psi_b - psi_r) * g, green_ss = 8.0 * g;
+    const double di_dot_d = (dd[0] * dbx[0] + dd[1] * dbx[1]) + dd[2] * dbx[2];
+    for (int k = 0; k < 3; ++k) {
+      f.rb[k] = f.rb[k] + green_r * c[k];
+      f.br[k] = f.br[k] + green_b * c[k];
+      f.cs[k] = f.cs[k] + (dd[k] - (2.0 * d_dotc) * c[k]) * g;
+      f.sc[k] = f.sc[k] + greenc_s * (dbx[k] - (2.0 * di_dotc) * c[k]);
+      f.ss[k] = f.ss[k] + green_ss * (((di_dot_d - (2.0 * di_dotc) * d_dotc) * c[k] + dd[k] * di_dotc) +
+                                      d_dotc * dbx[k]);
+    }
   }
 }
 
-__device__ __forceinline__ void sc_force_ternary(const DevParams &P, const Nb &nb, long long i,
+__device__ __forceinline__ void sc_force_ternary(const DevParams &P, int x, int y, int z, long long i,
                                                  const double *psi, const double *db, double *fr,
                                                  double *fb, double *fs) {
   const long long N = P.nsites;
   const double *psi_b_ = psi + N, *psi_s_ = psi + 2 * N, *db1 = db + N, *db2 = db + 2 * N;
-  double f_br[3] = {0, 0, 0}, f_rb[3] = {0, 0, 0}, f_cs[3] = {0, 0, 0}, f_sc[3] = {0, 0, 0},
-         f_ss[3] = {0, 0, 0};
+  TernarySums f;
   const double dbx[3] = {db[i], db[N + i], db[2 * N + i]};
+  const Nb nb(x, y, z, P.nx, P.ny, P.nz);
 #pragma unroll
   for (int q = 0; q < 18; ++q) {
     const unsigned j = nb.at<1>(q);
@@ -548,36 +637,43 @@ __device__ __forceinline__ void sc_force_ternary(const DevParams &P, const Nb &n
     double green_b = psi_r * g;
     for (int k = 0; k < 3; ++k) {
       if (c[k] == 0) continue;
-      f_rb[k] = f_rb[k] + green_r * (double)c[k];
-      f_br[k] = f_br[k] + green_b * (double)c[k];
+      f.rb[k] = f.rb[k] + green_r * (double)c[k];
+      f.br[k] = f.br[k] + green_b * (double)c[k];
     }
     double pss = ld(psi_s_, j);
     double dd[3] = {ld(db, j) * pss, ld(db1, j) * pss, ld(db2, j) * pss};
     double d_dotc = cdot(c, dd);
     for (int k = 0; k < 3; ++k)
-      f_cs[k] = f_cs[k] + (c[k] ? dd[k] - (2.0 * d_dotc) * (double)c[k] : dd[k]) * g;
+      f.cs[k] = f.cs[k] + (c[k] ? dd[k] - (2.0 * d_dotc) * (double)c[k] : dd[k]) * g;
     double di_dotc = cdot(c, dbx);
     double greenc_s = (psi_b - psi_r) * g;
     for (int k = 0; k < 3; ++k)
-      f_sc[k] = f_sc[k] + greenc_s * (c[k] ? dbx[k] - (2.0 * di_dotc) * (double)c[k] : dbx[k]);
+      f.sc[k] = f.sc[k] + greenc_s * (c[k] ? dbx[k] - (2.0 * di_dotc) * (double)c[k] : dbx[k]);
     double di_dot_d = (dd[0] * dbx[0] + dd[1] * dbx[1]) + dd[2] * dbx[2];
     double green_ss = 8.0 * g;
     const double along = di_dot_d - (2.0 * di_dotc) * d_dotc;
     for (int k = 0; k < 3; ++k) {
       const double t = dd[k] * di_dotc;
-      f_ss[k] = f_ss[k] + green_ss * ((c[k] ? along * (double)c[k] + t : t) + d_dotc * dbx[k]);
+      f.ss[k] = f.ss[k] + green_ss * ((c[k] ? along * (double)c[k] + t : t) + d_dotc * dbx[k]);
     }
   }
-  double pb = psi[N + i], prr = psi[i], ps = psi[2 * N + i];
-  for (int k = 0; k < 3; ++k) {
-    double br = -(P.g_br * f_br[k]);
-    double rb = -(P.g_br * f_rb[k]);
-    double sc = (2.0 * P.g_bs) * f_sc[k];
-    double cs = -((2.0 * P.g_bs) * f_cs[k]);
-    double ss = -(P.g_ss * f_ss[k]);
-    fb[k] = (br + cs) * pb;
-    fr[k] = (rb - cs) * prr;
-    fs[k] = (sc + ss) * ps;
+  const double pb = psi[N + i], prr = psi[i], ps = psi[2 * N + i];
+  auto forces = [&]() {
+    for (int k = 0; k < 3; ++k) {
+      double br = -(P.g_br * f.br[k]);
+      double rb = -(P.g_br * f.rb[k]);
+      double sc = (2.0 * P.g_bs) * f.sc[k];
+      double cs = -((2.0 * P.g_bs) * f.cs[k]);
+      double ss = -(P.g_ss * f.ss[k]);
+      fb[k] = (br + cs) * pb;
+      fr[k] = (rb - cs) * prr;
+      fs[k] = (sc + ss) * ps;
+    }
+  };
+  forces();
+  if (!(finite_sum(fb) && finite_sum(fr) && finite_sum(fs))) {
+    ternary_sums_all(P, x, y, z, psi, db, dbx, f);
+    forces();
   }
 }
 
@@ -591,7 +687,7 @@ __device__ __forceinline__ void sc_forces(const DevParams &P, int x, int y, int 
   if (NC == 2)
     sc_force_binary<LE, ROCK>(P, x, y, z, i, rho, psi, rock, plo, phi, F[0], F[1]);
   else
-    sc_force_ternary(P, Nb(x, y, z, P.nx, P.ny, P.nz), i, psi, db, F[0], F[1], F[NC - 1]);
+    sc_force_ternary(P, x, y, z, i, psi, db, F[0], F[1], F[NC - 1]);
 }
 
 // ---------------------------------------------------------------------------
