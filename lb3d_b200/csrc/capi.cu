@@ -311,6 +311,11 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
   std::string why;
   int rc = validate(p, why);
   if (rc != LB3DC_OK) return fail(nullptr, rc, "%s", why.c_str());
+  // the FP64 kernels hold a site's offset in bytes in 32 bits; such lattices take
+  // more than 370 GB, so no present device has had room for one
+  if (p->precision == LB3DC_FP64 && (long long)p->nx * p->ny * p->nz > (1LL << 29))
+    return fail(nullptr, LB3DC_ENOMEM, "FP64 lattices are limited to 2^29 sites (asked for %lld bytes)",
+                footprint_bytes(*p));
   lb3dc_handle *h = new lb3dc_handle();
   h->p = *p;
   h->P = make_dev_params(*p);

@@ -43,11 +43,12 @@ __device__ __forceinline__ void site_xyz(long long i, int nx, int ny, int &x, in
 
 // Site offsets of the -1, 0, +1 neighbours along each axis with the periodic
 // wrap applied once, as byte offsets of a double array: a kernel adds three of
-// them per neighbour and reads every field at that one 32-bit offset (a
-// lattice of 2^29 sites, where they would overflow, needs 570 GB).  Ternary
-// 128^3: dipole pass 113 -> 92 us (with four CTAs per SM), surfactant stream
-// 126 -> 106 us (with three), collide pass 453 -> 438 us; its pulls keep their
-// 64-bit addresses, with which the compiler does not hoist them into spills.
+// them per neighbour and reads every field at that one 32-bit offset (lattices
+// of more than 2^29 sites, where they would overflow, take 370 GB binary and 580
+// GB ternary; lb3dc_create refuses them).  Ternary 128^3: dipole pass 113 -> 92
+// us (with four CTAs per SM), surfactant stream 126 -> 106 us (with three),
+// collide pass 453 -> 438 us; its pulls keep their 64-bit addresses, with which
+// the compiler does not hoist them into spills.
 struct Nb {
   unsigned x[3], y[3], z[3];
   __device__ __forceinline__ Nb(int px, int py, int pz, int nx, int ny, int nz) {

@@ -165,3 +165,19 @@ def test_inflow_boundaries_refused_before_device(kw, text):
         buf = ctypes.create_string_buffer(256)
         L.lib().lb3dc_last_error(None, buf, 256)
         assert text in buf.value, buf.value
+
+
+def test_fp64_size_limit_checked_at_creation():
+    """The FP64 kernels' 32-bit byte offsets reach 2^29 sites; larger lattices,
+    which no device has had room for, are refused before any device work.  Their
+    footprint can still be asked for."""
+    import ctypes
+    from lb3d_b200.config import to_cparams
+    for nc in (2, 3):
+        p = Params(nx=1024, ny=1024, nz=513, ncomp=nc, bdist=2).finalize()
+        cp, h = to_cparams(p), ctypes.c_void_p()
+        assert L.lib().lb3dc_create(ctypes.byref(cp), ctypes.byref(h)) == L.LB3DC_ENOMEM
+        buf = ctypes.create_string_buffer(256)
+        L.lib().lb3dc_last_error(None, buf, 256)
+        assert b"limited to 2^29 sites" in buf.value
+        assert L.footprint(p) > 1024 * 1024 * 513 * (1081 if nc == 3 else 689) - 1
