@@ -1464,8 +1464,9 @@ int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, 
   const bool rk = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
   if (le && !s.le_h[0]) return LB3DC_ESTATE;
   // kernels per step: the pass(es) (ternary strategy 3: one more after its
-  // first step), two Lees-Edwards halo kernels, and the parity flip (strategy
-  // 3: one for the whole loop)
+  // first step; large sheared lattices: the moments pass in two parts), two
+  // Lees-Edwards halo kernels, and the parity flip (strategy 3: one for the
+  // whole loop)
   const int passes = sh.split ? (P.nc == 3 ? 3 : 2) : 1;
   for (int i = 0; i < nsteps; ++i) {
     const LEStep *l = le ? le + (le_per_step ? i : 0) : nullptr;
@@ -1478,7 +1479,8 @@ int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, 
                                             s.J, l, &P);
     if (s.timer) {
       s.timer->stop(st);
-      s.timer->launches += passes + (sh.split == 3 && P.nc == 3 && i > 0 ? 1 : 0) + (le ? 2 : 0) + (flip ? 1 : 0);
+      s.timer->launches += passes + (sh.split == 3 && P.nc == 3 && i > 0 ? 1 : 0) + (le ? 2 : 0) + (flip ? 1 : 0) +
+                           (sh.split == 3 && l && eq_forks(P) && s.eq_edge < s.eq_ntiles[EQ_MOMENTS] ? 1 : 0);
     }
     if (e != cudaSuccess) return LB3DC_ECUDA;
     if (!flip) continue;

@@ -91,6 +91,25 @@ def test_rock_populations_survive_a_change_of_strategy():
         assert np.array_equal(out[0][0], n) and out[0][1] == counts
 
 
+@pytest.mark.parametrize("dims,nc,per_step,first", [((32, 16, 12), 2, 4, 4), ((128, 96, 96), 2, 5, 5),
+                                                    ((32, 192, 192), 2, 4, 4), ((20, 18, 16), 3, 4, 3)])
+def test_kernel_stats_count_every_launch(dims, nc, per_step, first):
+    """Sheared: two halo kernels, moments (from 2^20 sites in two parts, where
+    tiles lie off the sheared boundary) and collide pass.  Ternary: moments,
+    after a loop's first step in two launches, dipole and collide pass.  One
+    parity flip a loop."""
+    from lb3d_b200.lib import Lattice
+    kw = dict(boundary_cond=-1, inv_fluid=5, shear_u=0.05) if nc == 2 else {}
+    lat = Lattice(_params(dims, nc, **kw), precision=1)
+    lat.upload_state(_state(dims, nc, shear=nc == 2))
+    assert lat.launch_shape[3] == 3
+    lat.set_profiling(True)
+    lat.time_loop(1)
+    lat.time_loop(5)
+    assert lat.kernel_stats()[2] == 2 * first + 4 * per_step + 2
+    lat.close()
+
+
 @pytest.mark.parametrize("kind", ["rock", "sheared rock"])
 def test_rock_populations_after_loops_of_one_step_and_more(kind):
     """A loop of one step lays no arguments over the rock sites' populations, a
