@@ -151,11 +151,8 @@ __device__ __forceinline__ void eq_store(float *out, unsigned S, float rho, floa
 }
 // eq_store for two components (lanes x, y) with bgk_update2's paired
 // arithmetic; lane x goes to outA, lane y to outB.
-// With bA (optional) the two components' values also go to bA[q * SB] and
-// bB[q * SB].
 __device__ __forceinline__ void eq_store2(float *outA, float *outB, unsigned S, float2 rho, float2 drho,
-                                          float2 vx, float2 vy, float2 vz, float2 omega,
-                                          float *bA = nullptr, float *bB = nullptr, unsigned SB = 0) {
+                                          float2 vx, float2 vy, float2 vz, float2 omega) {
   const float2 tx = mul2(f2(3.0f), vx), ty = mul2(f2(3.0f), vy), tz = mul2(f2(3.0f), vz);
   const float2 uke = mul2(f2(0.5f), fma2(tz, vz, fma2(ty, vy, mul2(tx, vx))));
   const float2 a = neg2(uke);
@@ -173,12 +170,6 @@ __device__ __forceinline__ void eq_store2(float *outA, float *outB, unsigned S, 
     __stcs(outB + (I) * S, p.y);                                              \
     __stcs(outA + (J) * S, m.x);                                              \
     __stcs(outB + (J) * S, m.y);                                              \
-    if (bA) {                                                                 \
-      bA[(I) * SB] = p.x;                                                     \
-      bB[(I) * SB] = p.y;                                                     \
-      bA[(J) * SB] = m.x;                                                     \
-      bB[(J) * SB] = m.y;                                                     \
-    }                                                                         \
   }
   LB3D_EQ2(tx, 0, 1)
   LB3D_EQ2(ty, 2, 3)
@@ -193,10 +184,6 @@ __device__ __forceinline__ void eq_store2(float *outA, float *outB, unsigned S, 
   const float2 oeq0 = fma2(mul2(mul2(omega, rho), f2(W0)), a, mul2(mul2(omega, drho), f2(W0)));
   __stcs(outA + 18 * S, oeq0.x);
   __stcs(outB + 18 * S, oeq0.y);
-  if (bA) {
-    bA[18 * SB] = oeq0.x;
-    bB[18 * SB] = oeq0.y;
-  }
 }
 
 // Own-site moments of one component's post-stream deviations d[q * ST]:
@@ -219,8 +206,8 @@ __device__ __forceinline__ void own_moments(const float *d, float &dr, float &j0
   j1 = a1;
   j2 = a2;
 }
-// own_moments2 of values already in registers (lane x, lane y).
-__device__ __forceinline__ void own_moments2_reg(const float2 v[19], float2 &dr, float2 &j0,
+// own_moments of two components (lanes x, y) with paired instructions.
+__device__ __forceinline__ void own_moments2(const float2 v[19], float2 &dr, float2 &j0,
                                                  float2 &j1, float2 &j2) {
   float2 r = f2(0.f), a0 = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
 #pragma unroll
@@ -236,26 +223,6 @@ __device__ __forceinline__ void own_moments2_reg(const float2 v[19], float2 &dr,
   j1 = a1;
   j2 = a2;
 }
-// own_moments of two components (lanes x, y) with paired instructions.
-template <int ST>
-__device__ __forceinline__ void own_moments2(const float *dA, const float *dB, float2 &dr,
-                                             float2 &j0, float2 &j1, float2 &j2) {
-  float2 r = f2(0.f), a0 = f2(0.f), a1 = f2(0.f), a2 = f2(0.f);
-#pragma unroll
-  for (int q = 0; q < 19; ++q) {
-    const float2 v = make_float2(dA[q * ST], dB[q * ST]);
-    const float g = (float)gw(q);
-    r = fma2(f2(g), v, r);
-    if (cx(q)) a0 = fma2(f2(g * (float)cx(q)), v, a0);
-    if (cy(q)) a1 = fma2(f2(g * (float)cy(q)), v, a1);
-    if (cz(q)) a2 = fma2(f2(g * (float)cz(q)), v, a2);
-  }
-  dr = r;
-  j0 = a0;
-  j1 = a1;
-  j2 = a2;
-}
-
 // Site offsets (32-bit, relative to the lattice base) of the -1, 0, +1
 // neighbours along each axis, with the periodic wrap applied once.
 struct Nbr {

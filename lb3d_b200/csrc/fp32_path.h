@@ -76,8 +76,9 @@ struct Fp32State {
   float2 *le_p[2] = {nullptr, nullptr};
   float *le_b[4] = {nullptr, nullptr, nullptr, nullptr};
   // strategy 3 (fp32_eqstate.h): its fields beside M, the neighbour mask of a
-  // lattice with rock, and its tile lists, one per pass, each chunking z so that the tiles fill the pass's resident grid:
-  // eq_ntiles[p] tiles at eq_tiles + eq_off[p]
+  // lattice with rock, and its tile lists, one per pass, each chunking z so that
+  // the tiles fill the pass's resident grid: eq_ntiles[p] tiles at eq_tiles +
+  // eq_off[p]
   float2 *psi = nullptr;  // ternary (a binary lattice's M holds psi)
   float4 *o1 = nullptr, *o3 = nullptr;
   float *o2 = nullptr;
@@ -155,10 +156,10 @@ cudaError_t fp32_planes_to_fp64(const float *src, double *dst, long long S, long
 // Bytes per site of the split strategy's moment fields.
 inline long long fp32_moment_bytes(int nc) { return nc == 3 ? 32 : 8; }
 inline long long fp32_own_bytes(int nc) { return nc == 3 ? 48 : 32; }
-// Flips the parity of every active lattice (one tiny kernel).
 // Raises the dynamic shared memory limit of a kernel and returns how many of its
 // CTAs are resident at once on the current device (kept per kernel and device).
 cudaError_t fp32_prepare_kernel(const void *fn, int nthreads, size_t smem, int *ctas_total);
+// Flips the parity of every active lattice (one tiny kernel).
 cudaError_t fp32_flip_parity(LatDesc *d_lat, int nlat, cudaStream_t st);
 size_t fp32_fused_smem(int nc, const FusedShape &sh);
 int fp32_set_shape(const DevParams &P, Fp32State &s, const FusedShape &sh, cudaStream_t st);

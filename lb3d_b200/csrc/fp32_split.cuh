@@ -440,7 +440,7 @@ __global__ void __launch_bounds__(TX *TY, Collide2Geom<NC, TX, TY>::MINB)
         float dr[NC], rho[NC], j[NC][3];
         {
           float2 r2, a0, a1, a2;
-          own_moments2_reg(d01, r2, a0, a1, a2);
+          own_moments2(d01, r2, a0, a1, a2);
           dr[0] = r2.x, dr[1] = r2.y;
           j[0][0] = a0.x, j[1][0] = a0.y;
           j[0][1] = a1.x, j[1][1] = a1.y;
