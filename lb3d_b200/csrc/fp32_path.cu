@@ -933,18 +933,21 @@ static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool 
   return eq_kernel(pass, first, P.nc, rock, s.le_h[0] != nullptr, ax, ay, 19ull * P.nc * s.S < (1ull << 32), k);
 }
 
-// Sheared lattices of at least this many sites run the halo kernels and the
-// moments of the tiles on the sheared boundary beside those of the others.
-static bool eq_forks(const DevParams &P) { return P.le && P.nsites >= (1LL << 20); }
-
 // One step of strategy 3: the moments pass (ternary: two of them after the
 // first step of a loop), the dipole pass (ternary) and the collide pass, each on
 // its own tile list and resident grid; with le (a binary Lees-Edwards lattice)
 // the stage-6 halo kernel runs before the moments pass and the stage-8 one
 // before the collide pass.  The halo kernels, bound by FP64 latency at 12 % of
 // the issue slots, concern only the tiles on the sheared boundary (eq_edge of
-// the moments tiles, at the end of the list): a large lattice runs halo,
-// boundary tiles and halo on the copy stream while the other tiles run on st.
+// the moments tiles, at the end of the list): a lattice whose moments tiles fill
+// more than one round of the resident CTAs runs halo, boundary tiles and halo on
+// the copy stream while the other tiles run on st.  Where they fill about two
+// rounds or more, a step takes 128^3 173 -> 158 us, 144x112x112 140 -> 131,
+// 160x100x100 135 -> 128, 256x128x128 226 -> 215, 200^3 446 -> 418, 96x512x16 78
+// -> 76 (200x96x48 86 -> 89); where all run in one round, the boundary tiles take
+// as long as the others and start a halo kernel later: 112^3 114 us unforked and
+// 124 forked, 192x128x128 202 and 217, 224x160x128 280 and 313, 512x64x64 155 and
+// 169, 64x192x192 180 and 184.
 // The first pass of a loop launches plainly: everything before it on the stream,
 // the parity flip of the loop before included, is complete and visible when it
 // starts, and so when any later pass does, which is what lets those read the
@@ -963,7 +966,7 @@ static cudaError_t eq_step(const DevParams &P, Fp32State &s, const uint8_t *rock
   a.mask = s.mask;
   a.X = EqFields{s.M, P.nc == 3 ? s.psi : reinterpret_cast<float2 *>(s.M), s.o1, s.o3, s.o2,
                  {reinterpret_cast<float4 *>(s.f[0]), reinterpret_cast<float4 *>(s.f[1])}, (unsigned)s.S};
-  const bool fork = le && eq_forks(P);
+  const bool fork = le && s.eq_edge > 0;
   cudaError_t e = cudaSuccess;
   for (int pass = 0; pass < EQ_PASSES && e == cudaSuccess; ++pass) {
     EqKernel k;
@@ -1075,10 +1078,11 @@ static int eq_build_tiles(const DevParams &P, const Fp32State &s, const FusedSha
         }
     }
     out.ntiles[pass] = (int)all.size() - out.off[pass];
-    if (pass == EQ_MOMENTS && eq_forks(P)) {
+    if (pass == EQ_MOMENTS && P.le && out.ntiles[pass] > res) {
       auto inner = [&](const Tile &t) { return t.x0 != 0 && t.x0 + tx < L.nx; };
       const auto end = std::stable_partition(all.begin() + out.off[pass], all.end(), inner);
-      out.edge = (int)(all.end() - end);
+      const auto start = all.begin() + out.off[pass];
+      out.edge = end > start ? (int)(all.end() - end) : 0;  // all on the boundary: nothing to run beside
     }
   }
   return LB3DC_OK;
@@ -1464,7 +1468,7 @@ int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, 
   const bool rk = (s.lat.flags & LAT_ROCK) != 0, body = (s.lat.flags & LAT_BODY) != 0;
   if (le && !s.le_h[0]) return LB3DC_ESTATE;
   // kernels per step: the pass(es) (ternary strategy 3: one more after its
-  // first step; large sheared lattices: the moments pass in two parts), two
+  // first step; forked sheared lattices: the moments pass in two parts), two
   // Lees-Edwards halo kernels, and the parity flip (strategy 3: one for the
   // whole loop)
   const int passes = sh.split ? (P.nc == 3 ? 3 : 2) : 1;
@@ -1480,7 +1484,7 @@ int fp32_run(const DevParams &P, Fp32State &s, const uint8_t *rock, int nsteps, 
     if (s.timer) {
       s.timer->stop(st);
       s.timer->launches += passes + (sh.split == 3 && P.nc == 3 && i > 0 ? 1 : 0) + (le ? 2 : 0) + (flip ? 1 : 0) +
-                           (sh.split == 3 && l && eq_forks(P) && s.eq_edge < s.eq_ntiles[EQ_MOMENTS] ? 1 : 0);
+                           (sh.split == 3 && l && s.eq_edge > 0 && s.eq_edge < s.eq_ntiles[EQ_MOMENTS] ? 1 : 0);
     }
     if (e != cudaSuccess) return LB3DC_ECUDA;
     if (!flip) continue;

@@ -86,7 +86,7 @@ struct Fp32State {
   const uint8_t *rock = nullptr;  // the handle's rock flags, as of the last upload
   Tile *eq_tiles = nullptr;
   int eq_ntiles[4] = {0, 0, 0, 0}, eq_off[4] = {0, 0, 0, 0};
-  int eq_edge = 0;  // sheared lattices: moments tiles on the boundary, last in their list
+  int eq_edge = 0;  // forked sheared lattices: moments tiles on the boundary, last in their list
 };
 
 // Launch configuration of the fused kernel.

@@ -70,6 +70,18 @@ def test_large_sheared_lattice_forks(rock):
     assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("rock", [False, True])
+@pytest.mark.parametrize("dims", [(128, 128, 128), (75, 509, 17), (48, 1024, 16)])
+def test_forked_sheared_lattices_equal_the_staged_split(dims, rock):
+    """More moments tiles than resident CTAs: the boundary tiles run beside the
+    others."""
+    kw = dict(boundary_cond=-1, inv_fluid=5, shear_u=0.2, shear_omega=0.31)
+    p, st = _params(dims, 2, **kw), _state(dims, 2, rock, True)
+    a, b = (_run(p, st, (16, 8, 16, s), (1, 4)) for s in (2, 3))
+    for x, y in zip(a, b):
+        assert np.array_equal(x["n"], y["n"])
+
+
 def test_rock_populations_survive_a_change_of_strategy():
     """A loop lays its arguments over the buffer it read first; rock sites hold
     their populations again afterwards, in both buffers."""
@@ -91,11 +103,13 @@ def test_rock_populations_survive_a_change_of_strategy():
         assert np.array_equal(out[0][0], n) and out[0][1] == counts
 
 
-@pytest.mark.parametrize("dims,nc,per_step,first", [((32, 16, 12), 2, 4, 4), ((128, 96, 96), 2, 5, 5),
-                                                    ((32, 192, 192), 2, 4, 4), ((20, 18, 16), 3, 4, 3)])
+@pytest.mark.parametrize("dims,nc,per_step,first", [((32, 16, 12), 2, 4, 4), ((192, 64, 64), 2, 4, 4),
+                                                    ((80, 512, 16), 2, 5, 5), ((32, 512, 80), 2, 4, 4),
+                                                    ((20, 18, 16), 3, 4, 3)])
 def test_kernel_stats_count_every_launch(dims, nc, per_step, first):
-    """Sheared: two halo kernels, moments (from 2^20 sites in two parts, where
-    tiles lie off the sheared boundary) and collide pass.  Ternary: moments,
+    """Sheared: two halo kernels, moments (in two parts where the tiles fill more
+    than one round of the resident CTAs and some lie off the sheared boundary)
+    and collide pass.  Ternary: moments,
     after a loop's first step in two launches, dipole and collide pass.  One
     parity flip a loop."""
     from lb3d_b200.lib import Lattice
