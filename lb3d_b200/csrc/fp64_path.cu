@@ -963,20 +963,28 @@ cudaError_t fp64_le_halo(const DevParams &P, const LEStep &S, const double *src,
                 rhi, plo, phi);
 }
 
-// Threads per block of the site kernels.  Small lattices take small blocks,
-// which spread their sites over more SMs (binary 64^3, a step: 60 us with 64,
-// 63 with 256; ternary 32^3: 29.7 with 64, 30.6 with 128, 31 with 256), the
-// smallest 128, whose neighbours share more of an L1 (ternary 16^3: 23.8
-// against 25.7 us).
-static int fp64_block(const DevParams &P) { return P.nsites > 300000 ? 256 : P.nsites > 16384 ? 64 : 128; }
-// Lattices bound by launches and latency stream all components in one launch
-// (ternary 32^3: 29.7 us a step against 33.5 with two).
-static bool fp64_small(const DevParams &P) { return P.nsites <= 65536; }
+// Threads per block of the site kernels, on both sides of each line (a step, 64
+// / 128 / 256 threads).  Small lattices take small blocks, which spread their
+// sites over more SMs, the smallest 128, whose neighbours share more of an L1:
+// ternary 16^3 15.6 / 15.1 / 16.4 us, 25^3 18.6 / 18.2 / 19.6, 32^3 21.1 / 22.2 /
+// 24.8, 64^3 110 / 109 / 110; binary 64^3 52.7 / 53.1 / 55.0.  Large ones: ternary
+// 68^3 136 / 134 / 134, 96^3 355 / 348 / 345, 128^3 821 / 797 / 795; binary with
+// rock 80^3 240 / 235 / 234, 128^3 988 / 976 / 919; binary 72^3 76 / 77 / 78, 128^3
+// 411 / 405 / 410, sheared 97x66x63 154 / 155 / 162, 128^3 607 / 598 / 616.
+static int fp64_block(const DevParams &P) {
+  if (P.nsites > 300000) return P.nc == 3 || P.any_rock ? 256 : 128;
+  return P.nsites > 16384 ? 64 : 128;
+}
+// Up to here all components stream in one launch: its saved launch is worth more
+// than the occupancy that red and blue lose to the surfactant's registers (a step
+// with one and with two: ternary 16^3 15.1 and 16.3 us, 40^3 28.3 and 32.6, 44^3
+// 39.1 and 41.9, 64^3 109.0 and 109.9, 96^3 347 and 349; 112^3 552 and 551, 128^3
+// 798 and 794, 160x128x128 1010 and 1002).
+static bool fp64_small(const DevParams &P) { return P.nsites <= 1000000; }
 
 // The stream kernel over all components: red and blue in one launch and the
-// surfactant, whose dipole flux takes twice the registers, in another (ternary
-// 128^3: 58 + 58 + 107 us as three launches); small lattices, bound by
-// launches and latency, all three in one.
+// surfactant, whose dipole flux takes more registers, in another (ternary 128^3:
+// 58 + 58 + 107 us as three launches); small lattices all three in one.
 template <bool STORE>
 static cudaError_t launch_stream(const DevParams &P, const double *fin, double *fout, double *rho, double *psi,
                                  double *mom, double *da, const double *db, const uint8_t *rock, const double *hlo,

@@ -41,7 +41,7 @@ def test_fp32_loops_back_to_back(nc, dims):
     assert np.isfinite(a["n"]).all()
 
 
-FP64 = {"ternary 16^3": (3, (16, 16, 16), {}, False), "ternary 49x40x37": (3, (49, 40, 37), {}, False),
+FP64 = {"ternary 16^3": (3, (16, 16, 16), {}, False), "ternary 104x100x98": (3, (104, 100, 98), {}, False),
         "binary": (2, (40, 17, 12), {}, False),
         "binary rock": (2, (21, 18, 16), dict(g_wr=-0.1, rock_colour_r=1.0), True),
         "sheared": (2, (33, 18, 17), dict(boundary_cond=-1, inv_fluid=5, shear_u=0.05), False),
@@ -51,7 +51,7 @@ FP64 = {"ternary 16^3": (3, (16, 16, 16), {}, False), "ternary 49x40x37": (3, (4
 @pytest.mark.parametrize("kind", FP64)
 def test_fp64_loops_back_to_back(kind):
     """Both ways a step is launched (all components in one stream launch up to
-    65536 sites, two above): every field of the download, the moments and the
+    a million sites, two above): every field of the download, the moments and the
     dipole flux among them."""
     nc, dims, kw, rock = FP64[kind]
     p, st = _params(dims, nc, 0, **kw), uniform_mixture(*dims, nc, seed=3)
