@@ -333,20 +333,21 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
   if (!rc && p->precision == LB3DC_FP64) {
     rc = rc ? rc : dalloc(h, &h->f, nc * 19 * N);
     rc = rc ? rc : dalloc(h, &h->g, nc * 19 * N);
-    rc = rc ? rc : dalloc(h, &h->rho, nc * N);
-    rc = rc ? rc : dalloc(h, &h->psi, nc * N);
-    rc = rc ? rc : dalloc(h, &h->mom, nc * 3 * N);
+    rc = rc ? rc : dalloc(h, &h->rho, nc * 5 * N);  // one block
+    h->psi = h->rho + nc * N;
+    h->mom = h->psi + nc * N;
     if (nc == 3) {
       rc = rc ? rc : dalloc(h, &h->da, 3 * N);
       rc = rc ? rc : dalloc(h, &h->db, 3 * N);
     }
     if (h->le) {
-      rc = rc ? rc : dalloc(h, &h->hlo, nc * 19 * np);
-      rc = rc ? rc : dalloc(h, &h->hhi, nc * 19 * np);
-      rc = rc ? rc : dalloc(h, &h->rlo, nc * np);
-      rc = rc ? rc : dalloc(h, &h->rhi, nc * np);
-      rc = rc ? rc : dalloc(h, &h->plo, nc * np);
-      rc = rc ? rc : dalloc(h, &h->phi, nc * np);
+      // one block
+      rc = rc ? rc : dalloc(h, &h->hlo, nc * (2 * 19 + 4) * np);
+      h->hhi = h->hlo + nc * 19 * np;
+      h->rlo = h->hhi + nc * 19 * np;
+      h->rhi = h->rlo + nc * np;
+      h->plo = h->rhi + nc * np;
+      h->phi = h->plo + nc * np;
       // optional: without room for them the steps stream in a pass of their own
       if (!rc && dalloc(h, &h->post, 2 * nc * 19 * np)) {
         cudaGetLastError();
@@ -378,8 +379,7 @@ int lb3dc_destroy(lb3dc_handle *h) {
   cudaSetDevice(h->device);
   if (h->io_pin) cudaFreeHost(h->io_pin);
   if (h->stream) cudaStreamSynchronize(h->stream);
-  double *bufs[] = {h->f, h->g, h->rho, h->psi, h->mom, h->da, h->db, h->hlo, h->hhi,
-                    h->rlo, h->rhi, h->plo, h->phi, h->post, h->scratch};
+  double *bufs[] = {h->f, h->g, h->rho, h->da, h->db, h->hlo, h->post, h->scratch};
   for (double *b : bufs)
     if (b) cudaFree(b);
   if (h->rock) cudaFree(h->rock);

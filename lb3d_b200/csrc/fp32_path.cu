@@ -838,6 +838,9 @@ LatDesc fp32_make_desc(const DevParams &P, double rho0, long long base, bool roc
 // ---------------------------------------------------------------------------
 // single-lattice handle
 // ---------------------------------------------------------------------------
+// Bytes of strategy 3's fields per site beside the neighbour mask.
+static long long eq_bytes(int nc) { return nc == 3 ? 44 : 20; }
+
 long long fp32_footprint(const lb3dc_params &p) {
   const long long N = (long long)p.nx * p.ny * p.nz;
   const bool le = p.boundary_cond != 0 && (p.inv_fluid == 5 || p.inv_fluid == 6);
@@ -845,7 +848,7 @@ long long fp32_footprint(const lb3dc_params &p) {
   // the fields of strategy 3 when every component relaxes fully (with the
   // neighbour mask of a binary lattice with rock)
   const bool full = p.tau_r == 1.0 && p.tau_b == 1.0 && (p.ncomp == 2 || p.tau_s == 1.0);
-  const long long mf = full ? N * (p.ncomp == 3 ? 44 : 24) : 0;
+  const long long mf = full ? N * (eq_bytes(p.ncomp) + (p.ncomp == 2 ? 4 : 0)) : 0;
   return 2LL * p.ncomp * 19 * N * 4 + (p.ncomp == 3 ? 6LL * N * 4 : 0) +
          N * fp32_moment_bytes(p.ncomp) + mf +
          (le ? 2 * np * (p.ncomp * 19 * 4 + 8) + 4 * np * p.ncomp * 19 * 4 : 0) + N * 16 + 4096;
@@ -862,9 +865,9 @@ bool fp32_eq_eligible(const DevParams &P) {
 }
 
 static void free_eq(Fp32State &s) {
-  if (s.o1) s.bytes -= s.S * (s.lat.nc == 3 ? 44 : 20);
+  if (s.o1) s.bytes -= s.S * eq_bytes(s.lat.nc);
   if (s.mask) s.bytes -= s.S * 4;
-  void *bufs[] = {s.o1, s.o2, s.o3, s.psi, s.mask, s.eq_tiles};
+  void *bufs[] = {s.o1, s.mask, s.eq_tiles};
   for (void *b : bufs)
     if (b) cudaFree(b);
   s.o1 = s.o3 = nullptr;
@@ -898,17 +901,20 @@ static int alloc_device(Fp32State &s, void **p, size_t bytes, cudaStream_t st) {
 static int ensure_eq(const DevParams &P, Fp32State &s, cudaStream_t st) {
   const size_t N = (size_t)P.nsites;
   if (!s.o1) {
-    bool ok = cudaMalloc(&s.o1, N * sizeof(float4)) == cudaSuccess;
-    if (ok) ok = cudaMalloc(&s.o2, N * sizeof(float)) == cudaSuccess;
-    if (ok && P.nc == 3)
-      ok = cudaMalloc(&s.o3, N * sizeof(float4)) == cudaSuccess && cudaMalloc(&s.psi, N * sizeof(float2)) == cudaSuccess;
-    if (!ok) {
+    // one block: o1, o3 (float4), psi (ternary), o2
+    if (cudaMalloc(&s.o1, N * eq_bytes(P.nc)) != cudaSuccess) {
       cudaGetLastError();
-      if (s.o1) s.bytes += s.S * (P.nc == 3 ? 44 : 20);  // free_eq takes them off
-      free_eq(s);
+      s.o1 = nullptr;
       return LB3DC_ENOMEM;
     }
-    s.bytes += (long long)N * (P.nc == 3 ? 44 : 20);
+    if (P.nc == 3) {
+      s.o3 = s.o1 + N;
+      s.psi = reinterpret_cast<float2 *>(s.o3 + N);
+      s.o2 = reinterpret_cast<float *>(s.psi + N);
+    } else {
+      s.o2 = reinterpret_cast<float *>(s.o1 + N);
+    }
+    s.bytes += (long long)N * eq_bytes(P.nc);
   }
   if (s.lat.flags & LAT_ROCK) {
     if (!s.mask) {
@@ -1283,33 +1289,32 @@ int fp32_alloc(const DevParams &P, const lb3dc_params &p, Fp32State &s, cudaStre
     if (cudaMalloc(&s.f[b], pop) != cudaSuccess) return LB3DC_ENOMEM;
     s.bytes += pop;
     cudaMemsetAsync(s.f[b], 0, pop, st);
-    if (P.nc == 3) {
-      if (cudaMalloc(&s.db[b], 3 * N * sizeof(float)) != cudaSuccess) return LB3DC_ENOMEM;
-      s.bytes += 3 * N * sizeof(float);
-      cudaMemsetAsync(s.db[b], 0, 3 * N * sizeof(float), st);
-    }
   }
-  if (cudaMalloc(&s.M, (size_t)N * fp32_moment_bytes(P.nc)) != cudaSuccess) return LB3DC_ENOMEM;
-  s.bytes += N * fp32_moment_bytes(P.nc);
+  if (P.nc == 3) {
+    if (cudaMalloc(&s.db[0], 6 * N * sizeof(float)) != cudaSuccess) return LB3DC_ENOMEM;
+    s.db[1] = s.db[0] + 3 * N;
+    s.bytes += 6 * N * sizeof(float);
+    cudaMemsetAsync(s.db[0], 0, 6 * N * sizeof(float), st);
+  }
+  // one block: M and the staging planes
+  const size_t mb = (size_t)N * fp32_moment_bytes(P.nc), sb = 2 * (size_t)N * sizeof(double);
+  if (cudaMalloc(&s.M, mb + sb) != cudaSuccess) return LB3DC_ENOMEM;
+  s.stage = reinterpret_cast<double *>(reinterpret_cast<unsigned char *>(s.M) + mb);
+  s.bytes += (long long)(mb + sb);
   if (cudaMalloc(&s.d_lat, sizeof(LatDesc)) != cudaSuccess) return LB3DC_ENOMEM;
-  if (cudaMalloc(&s.stage, 2 * (size_t)N * sizeof(double)) != cudaSuccess) return LB3DC_ENOMEM;
-  s.bytes += 2 * N * (long long)sizeof(double);
   if (cudaStreamCreateWithFlags(&s.xs, cudaStreamNonBlocking) != cudaSuccess) return LB3DC_ECUDA;
   for (int i = 0; i < 4; ++i)
     if (cudaEventCreateWithFlags(&s.xev[i], cudaEventDisableTiming) != cudaSuccess) return LB3DC_ECUDA;
   if (P.le) {
-    const size_t np = (size_t)P.ny * P.nz;
-    for (int b = 0; b < 2; ++b) {
-      if (cudaMalloc(&s.le_h[b], (size_t)P.nc * 19 * np * sizeof(float)) != cudaSuccess ||
-          cudaMalloc(&s.le_p[b], np * sizeof(float2)) != cudaSuccess)
-        return LB3DC_ENOMEM;
-      s.bytes += (long long)(P.nc * 19 * np * sizeof(float) + np * sizeof(float2));
-    }
-    for (int b = 0; b < 4; ++b) {
-      if (cudaMalloc(&s.le_b[b], (size_t)P.nc * 19 * np * sizeof(float)) != cudaSuccess)
-        return LB3DC_ENOMEM;
-      s.bytes += (long long)(P.nc * 19 * np * sizeof(float));
-    }
+    // one block: the psi planes and the 2 + 4 population planes
+    const size_t np = (size_t)P.ny * P.nz, plane = (size_t)P.nc * 19 * np;
+    const size_t bytes = 2 * np * sizeof(float2) + 6 * plane * sizeof(float);
+    if (cudaMalloc(&s.le_p[0], bytes) != cudaSuccess) return LB3DC_ENOMEM;
+    s.le_p[1] = s.le_p[0] + np;
+    float *f = reinterpret_cast<float *>(s.le_p[1] + np);
+    for (int b = 0; b < 2; ++b) s.le_h[b] = f + b * plane;
+    for (int b = 0; b < 4; ++b) s.le_b[b] = f + (2 + b) * plane;
+    s.bytes += (long long)bytes;
   }
   s.lat = fp32_make_desc(P, p.rho0 > 0 ? p.rho0 : 0.7, 0, false);
   attach_le(s);
@@ -1326,15 +1331,15 @@ int fp32_alloc(const DevParams &P, const lb3dc_params &p, Fp32State &s, cudaStre
 void fp32_free(Fp32State &s) {
   for (int b = 0; b < 2; ++b) {
     if (s.f[b]) cudaFree(s.f[b]);
-    if (s.db[b]) cudaFree(s.db[b]);
-    s.f[b] = s.db[b] = nullptr;
+    s.f[b] = nullptr;
   }
+  if (s.db[0]) cudaFree(s.db[0]);
+  s.db[0] = s.db[1] = nullptr;
   if (s.d_lat) cudaFree(s.d_lat);
   if (s.d_tiles) cudaFree(s.d_tiles);
   if (s.M) cudaFree(s.M);
   if (s.J) cudaFree(s.J);
   free_eq(s);
-  if (s.stage) cudaFree(s.stage);
   s.stage = nullptr;
   for (int i = 0; i < 4; ++i) {
     if (s.xev[i]) cudaEventDestroy(s.xev[i]);
@@ -1342,16 +1347,9 @@ void fp32_free(Fp32State &s) {
   }
   if (s.xs) cudaStreamDestroy(s.xs);
   s.xs = nullptr;
-  for (int b = 0; b < 2; ++b) {
-    if (s.le_h[b]) cudaFree(s.le_h[b]);
-    if (s.le_p[b]) cudaFree(s.le_p[b]);
-    s.le_h[b] = nullptr;
-    s.le_p[b] = nullptr;
-  }
-  for (int b = 0; b < 4; ++b) {
-    if (s.le_b[b]) cudaFree(s.le_b[b]);
-    s.le_b[b] = nullptr;
-  }
+  if (s.le_p[0]) cudaFree(s.le_p[0]);
+  for (int b = 0; b < 2; ++b) s.le_h[b] = nullptr, s.le_p[b] = nullptr;
+  for (int b = 0; b < 4; ++b) s.le_b[b] = nullptr;
   s.d_lat = nullptr;
   s.d_tiles = nullptr;
   s.M = nullptr;
@@ -1365,6 +1363,7 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   // the caller has uploaded the rock flags (rockp, device) and set any_rock
   const bool any = P.any_rock != 0;
   if (any && P.nc == 3) return LB3DC_EINVAL;
+  const int flags = s.lat.flags;
   s.lat = fp32_make_desc(P, rho0, 0, any);
   attach_le(s);
   s.lat.parity = 0;
@@ -1401,9 +1400,12 @@ int fp32_upload(const DevParams &P, const lb3dc_params &p, Fp32State &s, const d
   if (cudaMemcpyAsync(s.d_lat, &s.lat, sizeof(LatDesc), cudaMemcpyHostToDevice, st) != cudaSuccess)
     return LB3DC_ECUDA;
   if (s.le_b[0] && le_gather(P, s, st) != cudaSuccess) return LB3DC_ECUDA;
-  // keep the launch shape chosen so far (set or autotuned); the kernel
-  // variant may change with the rock flag
-  int rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, s.split}, st);
+  // keep the launch shape chosen so far (set or autotuned); the kernel variant,
+  // and with it the tile lists, may change with the rock flag, the neighbour
+  // mask with every upload
+  int rc = s.lat.flags != flags ? rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, s.split}, st)
+           : s.split == 3       ? ensure_eq(P, s, st)
+                                : LB3DC_OK;
   if (rc == LB3DC_ENOMEM && s.split == 3) {  // no room for the neighbour mask
     fp32_make_room(s, st);
     rc = rebuild_tiles(P, s, FusedShape{s.tx, s.ty, s.zc, 2}, st);

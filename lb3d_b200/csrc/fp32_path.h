@@ -80,7 +80,7 @@ struct Fp32State {
   // the tiles fill the pass's resident grid: eq_ntiles[p] tiles at eq_tiles +
   // eq_off[p]
   float2 *psi = nullptr;  // ternary (a binary lattice's M holds psi)
-  float4 *o1 = nullptr, *o3 = nullptr;
+  float4 *o1 = nullptr, *o3 = nullptr;  // o1: the block that holds o3, psi and o2 too
   float *o2 = nullptr;
   uint32_t *mask = nullptr;
   const uint8_t *rock = nullptr;  // the handle's rock flags, as of the last upload
