@@ -42,7 +42,7 @@ BYTES_PER_SITE = {("f32", 3): 480, ("f32", 2): 304, ("f64", 3): 960, ("f64", 2):
 # collide passes, a step within a loop; 16x8 tiles).  Keyed by (tile x, tile y,
 # strategy); for strategy 3 the tile shape moves only halo reloads that hit
 # L2, so its figure stands for every shape.
-NCU_TRAFFIC_PER_SITE = {(32, 4, 2): 772, (16, 8, 3): 258}
+NCU_TRAFFIC_PER_SITE = {(32, 4, 2): 772, (16, 8, 3): 259}
 
 
 def step_bytes(prec, nc, strategy, steps):
