@@ -316,6 +316,11 @@ int lb3dc_create(const lb3dc_params *p, lb3dc_handle **out) {
   if (p->precision == LB3DC_FP64 && (long long)p->nx * p->ny * p->nz > (1LL << 29))
     return fail(nullptr, LB3DC_ENOMEM, "FP64 lattices are limited to 2^29 sites (asked for %lld bytes)",
                 footprint_bytes(*p));
+  // the FP32 kernels' offsets within the sheared planes are 32-bit; lattices at
+  // least two sites across stay below
+  if (p->precision == LB3DC_FP32_DEV && p->boundary_cond != 0 && (p->inv_fluid == 5 || p->inv_fluid == 6) &&
+      38LL * p->ny * p->nz >= (1LL << 32))
+    return fail(nullptr, LB3DC_EINVAL, "FP32 sheared lattices are limited to 38*ny*nz < 2^32");
   lb3dc_handle *h = new lb3dc_handle();
   h->p = *p;
   h->P = make_dev_params(*p);

@@ -279,6 +279,9 @@ __device__ __forceinline__ void pull_comp(const float *__restrict__ F, unsigned 
 // feeding code/lb3d_advection.F90:109-151): across x = 0 (c_x = +1) and
 // x = nx - 1 (c_x = -1) the upstream site lies in the sheared halo planes
 // Lg.le_h[0] / Lg.le_h[1], [nc][19][nz][ny], at the wrapped (y - c_y, z - c_z).
+// Offsets within a set of planes, [nc][19][nz][ny], are unsigned 32-bit: at most
+// 38 ny nz, and a lattice of at least two sites across stays below.
+static_assert(38ull * (((1ull << 32) - 1) / 19 / 2) < (1ull << 32), "19 sites < 2^32, two sites across");
 struct LeYZ {
   int y[3], z[3];  // wrap(gy + k - 1) and ny * wrap(gz + k - 1)
 };
@@ -295,7 +298,7 @@ __device__ __forceinline__ void make_leyz(LeYZ &w, int gy, int gz, int ny, int n
 // and a pull from a rock site inside the lattice bounces back.
 template <int Q, bool ROCK = false>
 __device__ __forceinline__ const float *le_src(const float *fc, unsigned S, int c, const Nbr &n, int gx,
-                                               int nx, const LeYZ &w, const LatDesc &Lg, int NP,
+                                               int nx, const LeYZ &w, const LatDesc &Lg, unsigned NP,
                                                int self = 0, const uint8_t *__restrict__ rk = nullptr) {
   if (cx(Q) == 1 && gx == 0) return Lg.le_h[0] + (c * 19 + Q) * NP + w.y[1 - cy(Q)] + w.z[1 - cz(Q)];
   if (cx(Q) == -1 && gx == nx - 1)
@@ -307,7 +310,7 @@ __device__ __forceinline__ const float *le_src(const float *fc, unsigned S, int 
 template <bool NARROW = false, bool ROCK = false>
 __device__ __forceinline__ void pull_comp_le(const float *__restrict__ F, unsigned S, int c, const Nbr &n,
                                              int self, int gx, int nx, const LeYZ &w,
-                                             const LatDesc &Lg, int NP, float d[19],
+                                             const LatDesc &Lg, unsigned NP, float d[19],
                                              const uint8_t *__restrict__ rk = nullptr) {
   const float *fc = NARROW ? F + (unsigned)(c * 19) * S : F + (size_t)(c * 19) * S;
   d[18] = __ldg(fc + 18 * S + self);
@@ -324,8 +327,8 @@ __device__ __forceinline__ void pull_comp_le(const float *__restrict__ F, unsign
 // le_b[3]); sites elsewhere write nothing.
 __device__ __forceinline__ void le_store_boundary(const LatDesc &Lg, int set, int c, int gx, int gy,
                                                   int gz, const float d[19]) {
-  const int nx = Lg.nx, NP = Lg.ny * Lg.nz;
-  const int o = (c * 19) * NP + gy + Lg.ny * gz;
+  const int nx = Lg.nx;
+  const unsigned NP = Lg.ny * Lg.nz, o = (c * 19) * NP + gy + Lg.ny * gz;
   if (gx == nx - 1) {
     float *b = Lg.le_b[set] + o;
 #pragma unroll

@@ -348,7 +348,7 @@ __global__ void __launch_bounds__(EqGeom<V, TX, TY, ROCK>::NTH, EqGeom<V, TX, TY
       }
     };
     // the populations of the stage-6 halo plane at a sheared halo site
-    const int NP = ny * nz;
+    const unsigned NP = ny * nz;
     auto sheared = [&](int d, int z) {
       const float *h = Lg.le_h[side] + wy + ny * z;
       return make_float2(h[d * NP], h[(19 + d) * NP]);
@@ -953,9 +953,9 @@ __global__ void __launch_bounds__(TX *TY, EqCollideGeom<NC, TX, TY>::MINB)
       const float2 vx2 = make_float2(vx[0], vx[1]), vy2 = make_float2(vy[0], vy[1]), vz2 = make_float2(vz[0], vz[1]);
       if (LE && (gx == 0 || gx == nx - 1)) {
         // the next step's pre-stream boundary plane of its stage-6 halo kernel
-        const int NP = ny * nz;
+        const unsigned NP = ny * nz;
         float *b = Lg.le_b[gx == nx - 1 ? 0 : 1] + gy + ny * gz;
-        eq_store2(b, b + 19 * NP, (unsigned)NP, rho2, dr2, vx2, vy2, vz2, one);
+        eq_store2(b, b + 19 * NP, NP, rho2, dr2, vx2, vy2, vz2, one);
       }
       if (to_pops) {
         float *fo = (par ? f0 : f1) + base + self;

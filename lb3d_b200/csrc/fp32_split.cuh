@@ -285,7 +285,7 @@ __device__ __forceinline__ void pull_async(const float *__restrict__ F, unsigned
 template <int NT, bool ROCK = false>
 __device__ __forceinline__ void pull_async_le(const float *__restrict__ F, unsigned S, int c, const Nbr &n,
                                               int self, int gx, int nx, const LeYZ &w,
-                                              const LatDesc &Lg, int NP, float *stage,
+                                              const LatDesc &Lg, unsigned NP, float *stage,
                                               const uint8_t *__restrict__ rk = nullptr) {
   const float *fc = F + (size_t)(c * 19) * S;
   cp_async4(stage + 18 * NT, fc + 18 * S + self);
@@ -573,8 +573,8 @@ __global__ void k_le_pre32(DevParams P, LEStep L, const LatDesc *__restrict__ la
     for (int c = 0; c < NC; ++c)
       for (int q = 0; q < 19; ++q) {
         const double w = __dmul_rn(wq64(q), rho0);
-        hb[c][q] = (1.0 - f) * ((double)B[(c * 19 + q) * NP + ia] + w) +
-                   f * ((double)B[(c * 19 + q) * NP + ib] + w);
+        hb[c][q] = (1.0 - f) * ((double)B[(c * 19 + q) * (unsigned)NP + ia] + w) +
+                   f * ((double)B[(c * 19 + q) * (unsigned)NP + ib] + w);
       }
     le_adjust<NC>(P, hb, hb, L.shear_u, -1.0);
   };
@@ -582,7 +582,7 @@ __global__ void k_le_pre32(DevParams P, LEStep L, const LatDesc *__restrict__ la
     bottom();
     for (int c = 0; c < NC; ++c)
       for (int q = 0; q < 19; ++q)
-        Lg.le_h[0][(c * 19 + q) * NP + u] = (float)(hb[c][q] - __dmul_rn(wq64(q), rho0));
+        Lg.le_h[0][(c * 19 + q) * (unsigned)NP + u] = (float)(hb[c][q] - __dmul_rn(wq64(q), rho0));
     return;
   }
   double ht[NC][19], df[NC][19];
@@ -592,8 +592,8 @@ __global__ void k_le_pre32(DevParams P, LEStep L, const LatDesc *__restrict__ la
     for (int c = 0; c < NC; ++c)
       for (int q = 0; q < 19; ++q) {
         const double w = __dmul_rn(wq64(q), rho0);
-        ht[c][q] = f * ((double)B[(c * 19 + q) * NP + ia] + w) +
-                   (1.0 - f) * ((double)B[(c * 19 + q) * NP + ib] + w);
+        ht[c][q] = f * ((double)B[(c * 19 + q) * (unsigned)NP + ia] + w) +
+                   (1.0 - f) * ((double)B[(c * 19 + q) * (unsigned)NP + ib] + w);
       }
   }
   // the top site's clipping rule reads the adjusted bottom site, which this
@@ -603,7 +603,7 @@ __global__ void k_le_pre32(DevParams P, LEStep L, const LatDesc *__restrict__ la
   le_adjust_apply<NC>(ht, hb, df, neg);
   for (int c = 0; c < NC; ++c)
     for (int q = 0; q < 19; ++q)
-      Lg.le_h[1][(c * 19 + q) * NP + u] = (float)(ht[c][q] - __dmul_rn(wq64(q), rho0));
+      Lg.le_h[1][(c * 19 + q) * (unsigned)NP + u] = (float)(ht[c][q] - __dmul_rn(wq64(q), rho0));
 }
 
 template <int NC>
@@ -624,7 +624,7 @@ __global__ void k_le_post32(DevParams P, LEStep L, const LatDesc *__restrict__ l
   // 0: the moments pass left them in the compact boundary planes, pulled as
   // it pulls every site (across x from the stage-6 halo planes)
   auto post = [&](int c, int q, int x, int yy, int zz) -> double {
-    const float v = Lg.le_b[x == 0 ? 3 : 2][(c * 19 + q) * NP + yy + ny * zz];
+    const float v = Lg.le_b[x == 0 ? 3 : 2][(c * 19 + q) * (unsigned)NP + yy + ny * zz];
     return (double)v + __dmul_rn(wq64(q), rho0);
   };
   double hb[NC][19];

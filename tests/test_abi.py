@@ -181,3 +181,20 @@ def test_fp64_size_limit_checked_at_creation():
         L.lib().lb3dc_last_error(None, buf, 256)
         assert b"limited to 2^29 sites" in buf.value
         assert L.footprint(p) > 1024 * 1024 * 513 * (1081 if nc == 3 else 689) - 1
+
+
+def test_fp32_sheared_plane_limit_checked_at_creation():
+    """Offsets within a sheared lattice's planes (38 ny nz populations) are 32-bit
+    in the FP32 kernels: every lattice two sites across that the path takes fits,
+    a larger one that is one site across is refused before any device work."""
+    import ctypes
+    from lb3d_b200.config import to_cparams
+    most = ((1 << 32) - 1) // 19
+    assert 38 * (most // 2) < 1 << 32
+    cp, h = to_cparams(Params(nx=1, ny=10700, nz=10700, ncomp=2, bdist=2, boundary_cond=-1, inv_fluid=5,
+                              shear_u=0.01, precision=1).finalize()), ctypes.c_void_p()
+    assert 10700 * 10700 < most and 38 * 10700 * 10700 >= 1 << 32
+    assert L.lib().lb3dc_create(ctypes.byref(cp), ctypes.byref(h)) == L.LB3DC_EINVAL
+    buf = ctypes.create_string_buffer(256)
+    L.lib().lb3dc_last_error(None, buf, 256)
+    assert b"38*ny*nz" in buf.value
