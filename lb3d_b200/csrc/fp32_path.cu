@@ -948,12 +948,12 @@ static bool eq_kernel_of(const DevParams &P, const Fp32State &s, int pass, bool 
 // the moments tiles, at the end of the list): a lattice whose moments tiles fill
 // more than one round of the resident CTAs runs halo, boundary tiles and halo on
 // the copy stream while the other tiles run on st.  Where they fill about two
-// rounds or more, a step takes 128^3 173 -> 158 us, 144x112x112 140 -> 131,
-// 160x100x100 135 -> 128, 256x128x128 226 -> 215, 200^3 446 -> 418, 96x512x16 78
-// -> 76 (200x96x48 86 -> 89); where all run in one round, the boundary tiles take
-// as long as the others and start a halo kernel later: 112^3 114 us unforked and
-// 124 forked, 192x128x128 202 and 217, 224x160x128 280 and 313, 512x64x64 155 and
-// 169, 64x192x192 180 and 184.
+// rounds or more, a step takes 128^3 162 -> 155 us, 144x112x112 131 -> 126,
+// 160x100x100 128 -> 123, 256x128x128 221 -> 211, 200^3 431 -> 407 (96x512x16 74
+// and 74, 200x96x48 79 -> 81); where all run in one round, the boundary tiles take
+// as long as the others and start a halo kernel later: 112^3 107 us unforked and
+// 118 forked, 192x128x128 188 and 201, 224x160x128 261 and 292, 512x64x64 145 and
+// 157, 64x192x192 170 and 172.
 // The first pass of a loop launches plainly: everything before it on the stream,
 // the parity flip of the loop before included, is complete and visible when it
 // starts, and so when any later pass does, which is what lets those read the
@@ -1116,7 +1116,7 @@ static void attach_le(Fp32State &s) {
 // tiles, the fastest or within 3 % of it on every lattice measured (ternary
 // 32^3, 64^3, 75x67x87, 128^3: 0.019, 0.040, 0.062, 0.202 ms a step against
 // 0.058, 0.082, 0.126, 0.384 for strategy 2; binary 256x128x128 0.157 against
-// 0.432, sheared 0.214 against 0.565, porous 192^3 0.273 against 0.924).
+// 0.432, sheared 0.211 against 0.564, porous 192^3 0.273 against 0.924).
 // Others: the split strategy with the staged collide pass, the fastest of 0 to
 // 2.
 static FusedShape default_shape(const DevParams &P) {
