@@ -379,12 +379,18 @@ int lb3dc_ensemble_create(int ncomp, long long capacity_sites, int max_lattices,
   }
   const size_t pop = (size_t)ncomp * 19 * capacity_sites * sizeof(float);
   bool ok = true;
-  for (int b = 0; b < 2; ++b) {
-    ok = ok && cudaMalloc(&e->f[b], pop) == cudaSuccess;
-    if (ncomp == 3) ok = ok && cudaMalloc(&e->db[b], 3 * (size_t)capacity_sites * 4) == cudaSuccess;
+  for (int b = 0; b < 2; ++b) ok = ok && cudaMalloc(&e->f[b], pop) == cudaSuccess;
+  // one block: M, the dipoles (ternary) and the rock flags
+  const size_t cap = (size_t)capacity_sites, mb = cap * fp32_moment_bytes(ncomp), dbb = ncomp == 3 ? 24 * cap : 0;
+  ok = ok && cudaMalloc(&e->M, mb + dbb + cap) == cudaSuccess;
+  if (ok) {
+    unsigned char *block = reinterpret_cast<unsigned char *>(e->M);
+    if (ncomp == 3) {
+      e->db[0] = reinterpret_cast<float *>(block + mb);
+      e->db[1] = e->db[0] + 3 * cap;
+    }
+    e->rock = block + mb + dbb;
   }
-  ok = ok && cudaMalloc(&e->rock, (size_t)capacity_sites) == cudaSuccess;
-  ok = ok && cudaMalloc(&e->M, (size_t)capacity_sites * fp32_moment_bytes(ncomp)) == cudaSuccess;
   ok = ok && cudaMalloc(&e->d_lat, (size_t)max_lattices * sizeof(LatDesc)) == cudaSuccess;
   if (!ok) {
     lb3dc_ensemble_destroy(e);
@@ -432,11 +438,8 @@ int lb3dc_ensemble_destroy(lb3dc_ensemble *e) {
   cudaSetDevice(e->device);
   if (e->stream) cudaStreamSynchronize(e->stream);
   drop_graph(e);
-  for (int b = 0; b < 2; ++b) {
+  for (int b = 0; b < 2; ++b)
     if (e->f[b]) cudaFree(e->f[b]);
-    if (e->db[b]) cudaFree(e->db[b]);
-  }
-  if (e->rock) cudaFree(e->rock);
   free_eq(e);
   if (e->M) cudaFree(e->M);
   if (e->J) cudaFree(e->J);
